@@ -1,22 +1,27 @@
 // compact.cu — stable active-particle compaction (compaction.wgsl:65-217,
 // host src/gpu/compaction.rs:447-505).
 //
-// Three kernels over tiles of TILE = 2048 slots (256 threads x 8 slots):
+// Over tiles of TILE = 2048 slots (256 threads x 8 slots):
 //   1. count:   each warp ballots the active bit of 32 slots at a time and
 //               sums popcounts; one count per tile;
-//   2. scan:    one block turns tile counts into exclusive offsets and the
-//               total (the active count);
-//   3. scatter: each active slot goes to offset(tile) + its rank among the
-//               active slots before it in the tile (ballot + popc), so the
-//               original order is kept; every slot >= active count receives
-//               its own old contents with the active bit cleared.
+//   2. index:   a tile's offset is the sum of the counts below it, and each
+//               active slot's rank in the tile comes from ballots and a
+//               prefix over the tile's warps, so the original order is kept;
+//   3. move:    every field is gathered through the indices; every slot >=
+//               active count receives its own old contents with the active
+//               bit cleared (move_fields.cu).
 // All FPG_FIELD_COUNT arrays move into a second structure-of-arrays block
 // that is then swapped with the particle handle's (no copy back).
+//
+// HBM binds: 184 B of fields, 8 B of indices and 8 B of flags per slot.
+// 5 M slots with 30 % dead: 175 us of kernels (360 us with a scatter whose
+// stores followed their loads one field at a time).
 #include <cuda_runtime.h>
 
 #include <cstring>
 
 #include "fpg_internal.h"
+#include "move_fields.h"
 
 namespace fpg {
 
@@ -27,8 +32,6 @@ void particles_assign_fields(void* block, size_t capacity, void** field);
 constexpr int CT_THREADS = 256;
 constexpr int CT_ITEMS = 8;
 constexpr int CT_TILE = CT_THREADS * CT_ITEMS;
-
-struct Fields { uint32_t* f[FPG_FIELD_COUNT]; };
 
 // Per-tile active count.  Slot order inside a tile: item-major chunks of 256
 // (chunk c covers slots tile*TILE + c*256 .. +255), warp w of the chunk
@@ -53,10 +56,8 @@ __global__ void __launch_bounds__(CT_THREADS) compact_count_kernel(const uint32_
     }
 }
 
-// Exclusive scan of tile counts in one block of 1024 threads; writes the
-// total to *active.
-__global__ void __launch_bounds__(1024) compact_scan_kernel(uint32_t* __restrict__ tile_counts, uint32_t n_tiles,
-                                                            uint32_t* __restrict__ active) {
+// Exclusive scan of the tile counts in one block of 1024 threads.
+__global__ void __launch_bounds__(1024) compact_scan_kernel(uint32_t* __restrict__ tile_counts, uint32_t n_tiles) {
     __shared__ uint32_t s[1024];
     const uint32_t per = (n_tiles + 1023u) / 1024u;
     const uint32_t begin = threadIdx.x * per;
@@ -77,54 +78,73 @@ __global__ void __launch_bounds__(1024) compact_scan_kernel(uint32_t* __restrict
         tile_counts[i] = run;
         run += v;
     }
-    if (threadIdx.x == 1023u) *active = s[1023];
 }
 
-__global__ void __launch_bounds__(CT_THREADS) compact_scatter_kernel(Fields src, Fields dst, uint32_t n,
-                                                                     const uint32_t* __restrict__ tile_offsets,
-                                                                     const uint32_t* __restrict__ active_ptr,
-                                                                     uint32_t* __restrict__ indices) {
-    __shared__ uint32_t s_warp[CT_ITEMS][CT_THREADS / 32];
+// The sum of one value per thread, on every thread.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31u) == 0u) s_warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < CT_THREADS / 32; ++w) t += s_warp[w];
+    return t;
+}
+
+// The original slot of each active particle, in slot order, and their number
+// (to the device and to page-locked host memory).  `tiles` holds the tile
+// counts, or with `scanned` their exclusive scan.  A CTA that gets the counts
+// sums the ones below it itself: 20 KB from L2 per CTA at 10 M slots, about
+// a microsecond beside the scan kernel's launch and its single block's
+// 3.7 us; the sums grow with the square of the tiles, so above kSelfSumTiles
+// (16.8 M slots, 32 KB a CTA) the scan kernel runs.
+constexpr uint32_t kSelfSumTiles = 8192;
+
+__global__ void __launch_bounds__(CT_THREADS) compact_index_kernel(const uint32_t* __restrict__ flags, uint32_t n,
+                                                                   const uint32_t* __restrict__ tiles, int scanned,
+                                                                   uint32_t* __restrict__ indices,
+                                                                   uint32_t* __restrict__ active_dev,
+                                                                   uint32_t* __restrict__ active_host) {
+    constexpr int kWarps = CT_THREADS / 32;
+    __shared__ uint32_t s_below[kWarps];
+    __shared__ uint32_t s_pre[CT_ITEMS * kWarps];       // counts, then exclusive prefix, in slot order
     const uint32_t tile = blockIdx.x;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    uint32_t below = 0;
+    if (!scanned)
+        for (uint32_t t = threadIdx.x; t < tile; t += CT_THREADS) below += tiles[t];
     unsigned ballots[CT_ITEMS];
 #pragma unroll
     for (int c = 0; c < CT_ITEMS; ++c) {
         const uint32_t slot = tile * CT_TILE + c * CT_THREADS + threadIdx.x;
-        const bool act = slot < n && (src.f[FPG_FIELD_FLAGS][slot] & 1u);
-        ballots[c] = __ballot_sync(0xffffffffu, act);
-        if (lane == 0) s_warp[c][warp] = __popc(ballots[c]);
+        ballots[c] = __ballot_sync(0xffffffffu, slot < n && (flags[slot] & 1u));
+        if (lane == 0) s_pre[c * kWarps + warp] = __popc(ballots[c]);
+    }
+    const uint32_t base = scanned ? tiles[tile] : block_sum(below, s_below);
+    __syncthreads();
+    if (warp == 0) {
+        // exclusive prefix of the 64 (chunk, warp) counts, two per lane
+        static_assert(CT_ITEMS * kWarps == 64, "two counts per lane");
+        const uint32_t a = s_pre[2u * lane], b = s_pre[2u * lane + 1u];
+        uint32_t v = a + b;
+#pragma unroll
+        for (unsigned d = 1; d < 32u; d <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) v += x;
+        }
+        s_pre[2u * lane] = v - a - b;
+        s_pre[2u * lane + 1u] = v - b;
+        if (lane == 31u && tile == gridDim.x - 1u) {
+            *active_dev = base + v;
+            *active_host = base + v;
+        }
     }
     __syncthreads();
-    // exclusive prefix over (chunk, warp) in slot order, computed per thread
-    const uint32_t active = *active_ptr;
-    uint32_t base = tile_offsets[tile];
 #pragma unroll
-    for (int c = 0; c < CT_ITEMS; ++c) {
-        uint32_t before = base;
-        for (unsigned w = 0; w < warp; ++w) before += s_warp[c][w];
-        uint32_t chunk_total = 0;
-        for (unsigned w = 0; w < CT_THREADS / 32; ++w) chunk_total += s_warp[c][w];
-        const uint32_t slot = tile * CT_TILE + c * CT_THREADS + threadIdx.x;
-        if (slot < n) {
-            if (ballots[c] & (1u << lane)) {
-                const uint32_t d = before + __popc(ballots[c] & lt_mask);
-#pragma unroll
-                for (int f = 0; f < FPG_FIELD_COUNT; ++f) dst.f[f][d] = src.f[f][slot];
-                if (indices) indices[d] = slot;
-            }
-            if (slot >= active) {
-#pragma unroll
-                for (int f = 0; f < FPG_FIELD_COUNT; ++f) {
-                    uint32_t v = src.f[f][slot];
-                    if (f == FPG_FIELD_FLAGS) v &= ~1u;
-                    dst.f[f][slot] = v;
-                }
-            }
-        }
-        base += chunk_total;
-    }
+    for (int c = 0; c < CT_ITEMS; ++c)
+        if (ballots[c] & (1u << lane))
+            indices[base + s_pre[c * kWarps + warp] + __popc(ballots[c] & ((1u << lane) - 1u))] =
+                tile * CT_TILE + c * CT_THREADS + threadIdx.x;
 }
 
 }  // namespace fpg
@@ -156,6 +176,7 @@ extern "C" fpg_status fpg_compaction_destroy(fpg_compaction* c) {
     if (!c) return FPG_OK;
     cudaFree(c->block);
     cudaFree(c->tile_counts);
+   
     cudaFree(c->active_count_dev);
     cudaFreeHost(c->active_count_host);
     delete c;
@@ -172,21 +193,21 @@ extern "C" fpg_status fpg_compact(fpg_ctx* ctx, fpg_particles* P, fpg_compaction
         return FPG_OK;
     }
     cudaStream_t s = ctx->pick(stream);
-    Fields src, dst;
-    void* dst_fields[FPG_FIELD_COUNT];
-    particles_assign_fields(c->block, c->capacity, dst_fields);
-    for (int f = 0; f < FPG_FIELD_COUNT; ++f) {
-        src.f[f] = static_cast<uint32_t*>(P->field[f]);
-        dst.f[f] = static_cast<uint32_t*>(dst_fields[f]);
-    }
+    void* dst[FPG_FIELD_COUNT];
+    particles_assign_fields(c->block, c->capacity, dst);
+    const uint32_t* flags = static_cast<const uint32_t*>(P->field[FPG_FIELD_FLAGS]);
+    // without a buffer of the caller's the indices lie where the move writes last
+    uint32_t* indices = indices_dev ? indices_dev : static_cast<uint32_t*>(dst[FPG_FIELD_COUNT - 1]);
     const uint32_t tiles = (uint32_t)c->n_tiles;
-    compact_count_kernel<<<tiles, CT_THREADS, 0, s>>>(src.f[FPG_FIELD_FLAGS], n, c->tile_counts);
-    compact_scan_kernel<<<1, 1024, 0, s>>>(c->tile_counts, tiles, c->active_count_dev);
-    compact_scatter_kernel<<<tiles, CT_THREADS, 0, s>>>(src, dst, n, c->tile_counts, c->active_count_dev,
-                                                         indices_dev);
-    ctx->count(3);
+    const bool scan = tiles > kSelfSumTiles;
+    compact_count_kernel<<<tiles, CT_THREADS, 0, s>>>(flags, n, c->tile_counts);
+    if (scan) compact_scan_kernel<<<1, 1024, 0, s>>>(c->tile_counts, tiles);
+    compact_index_kernel<<<tiles, CT_THREADS, 0, s>>>(flags, n, c->tile_counts, scan ? 1 : 0, indices,
+                                                      c->active_count_dev, c->active_count_host);
+    ctx->count(scan ? 3 : 2);
     FPG_CHECK_LAUNCH();
-    FPG_CUDA(cudaMemcpyAsync(c->active_count_host, c->active_count_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    const fpg_status st = move_fields(ctx, P->field, dst, indices, 0, c->active_count_dev, n, true, s);
+    if (st != FPG_OK) return st;
     FPG_CUDA(cudaStreamSynchronize(s));
     particles_swap_block(P, &c->block);
     const uint32_t act = *c->active_count_host;

@@ -120,7 +120,7 @@ struct fpg_compaction {
     fpg_ctx* ctx = nullptr;
     size_t capacity = 0;
     void* block = nullptr;                  // second structure-of-arrays (swapped in)
-    uint32_t* tile_counts = nullptr;        // per-tile active counts, then offsets
+    uint32_t* tile_counts = nullptr;        // per-tile active counts (their exclusive scan above 8192 tiles)
     uint32_t* active_count_dev = nullptr;
     uint32_t* active_count_host = nullptr;  // pinned
     size_t n_tiles = 0;

@@ -21,6 +21,7 @@
 #include <cub/cub.cuh>
 
 #include "fpg_internal.h"
+#include "move_fields.h"
 #include "physics.cuh"
 
 struct fpg_sorter {
@@ -92,18 +93,6 @@ __global__ void __launch_bounds__(256) cell_key_kernel(KeyArgs a, uint32_t* __re
     }
     keys[p] = key;
     vals[p] = p;
-}
-
-struct SortFields { uint32_t* f[FPG_FIELD_COUNT]; };
-
-// dst[f][i] = src[f][perm[i]] for i < n, dst[f][i] = src[f][i] above.
-__global__ void __launch_bounds__(256) permute_kernel(SortFields src, SortFields dst, const uint32_t* __restrict__ perm,
-                                                      uint32_t n, uint32_t capacity) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= capacity) return;
-    const uint32_t s = i < n ? perm[i] : i;
-#pragma unroll
-    for (int f = 0; f < FPG_FIELD_COUNT; ++f) dst.f[f][i] = src.f[f][s];
 }
 
 // Bits needed for keys 0..cells (cells itself is the inactive key).
@@ -183,17 +172,10 @@ extern "C" fpg_status fpg_sort_by_cell(fpg_ctx* ctx, fpg_particles* P, const fpg
     FPG_CUDA(cub::DeviceRadixSort::SortPairs(s->temp, tb, kb, vb, (int)n, 0, bits, st));
     ctx->count(1 + (bits + 7) / 8);  // histogram + one pass per 8-bit digit
     const uint32_t* perm = vb.Current();
-    SortFields src, dst;
-    void* dst_fields[FPG_FIELD_COUNT];
-    particles_assign_fields(s->block, s->capacity, dst_fields);
-    for (int f = 0; f < FPG_FIELD_COUNT; ++f) {
-        src.f[f] = static_cast<uint32_t*>(P->field[f]);
-        dst.f[f] = static_cast<uint32_t*>(dst_fields[f]);
-    }
-    const uint32_t cap = (uint32_t)P->capacity;
-    permute_kernel<<<(cap + 255) / 256, 256, 0, st>>>(src, dst, perm, n, cap);
-    ctx->count();
-    FPG_CHECK_LAUNCH();
+    void* dst[FPG_FIELD_COUNT];
+    particles_assign_fields(s->block, s->capacity, dst);
+    const fpg_status moved = move_fields(ctx, P->field, dst, perm, n, nullptr, (uint32_t)P->capacity, false, st);
+    if (moved != FPG_OK) return moved;
     if (perm_dev) FPG_CUDA(cudaMemcpyAsync(perm_dev, perm, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     particles_swap_block(P, &s->block);
     return FPG_OK;
