@@ -23,6 +23,7 @@
 #include "fpg_internal.h"
 #include "move_fields.h"
 #include "physics.cuh"
+#include "step_core.cuh"
 
 struct fpg_sorter {
     fpg_ctx* ctx = nullptr;
@@ -43,9 +44,8 @@ void particles_assign_fields(void* block, size_t capacity, void** field);
 struct KeyArgs {
     const int32_t* cell_x; const int32_t* cell_y; const float* pos_x; const float* pos_y; const float* pos_z;
     const uint32_t* flags;
-    const float* heights;
+    Levels lv;
     uint32_t n, nx, ny, nz;
-    int has_heights, monotonic;
 };
 
 // Same lower-corner arithmetic as the fused step (axis_bracket and
@@ -54,45 +54,49 @@ __device__ __forceinline__ uint32_t lower_index(float coord, uint32_t n) {
     return (uint32_t)floorf(clampf(coord, 0.0f, (float)(n - 1u)));
 }
 
-__device__ __forceinline__ float level_of_height(const float* h, uint32_t nz, int has, int mono, float z) {
-    if (!has) return z;
-    const float h0 = h[0];
-    if (z <= h0) return h0 > 0.0f ? z / h0 : 0.0f;
-    uint32_t k;
-    if (mono) {
-        uint32_t lo = 1u, hi = nz;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (z <= h[mid]) hi = mid; else lo = mid + 1u;
-        }
-        k = lo;
-    } else {
-        k = nz;
-        for (uint32_t i = 1u; i < nz; ++i) if (z <= h[i]) { k = i; break; }
-    }
-    if (k >= nz) return (float)(nz - 1u);
-    const float hprev = h[k - 1u];
-    const float denom = h[k] - hprev;
-    if (denom > 0.0f) return (float)(k - 1u) + (z - hprev) / denom;
-    return (float)(k - 1u);
+// lower_index(meters_to_level(z)): the level (k - 1) + (z - h[k-1]) / (h[k] -
+// h[k-1]) has lower corner k - 1 unless the quotient rounds up to 1, so the
+// IEEE division runs only for the last hundredth of a layer (k <= 256: a
+// float sum below k - 0.0099 cannot round to k).
+__device__ __forceinline__ uint32_t lower_level(const Levels& lv, float z) {
+    if (!lv.has) return lower_index(z, lv.nz);
+    const float h0 = lv.h[0];
+    if (z <= h0) return lower_index(h0 > 0.0f ? z / h0 : 0.0f, lv.nz);
+    const uint32_t k = level_index(lv, z);
+    if (k >= lv.nz) return lv.nz - 1u;
+    const float hprev = lv.h[k - 1u];
+    const float denom = lv.h[k] - hprev, above = z - hprev;
+    if (!(denom > 0.0f) || above < 0.99f * denom) return k - 1u;
+    return lower_index((float)(k - 1u) + above / denom, lv.nz);
 }
 
+__device__ __forceinline__ uint32_t cell_key(const KeyArgs& a, uint32_t flags, int32_t cx, int32_t cy, float px,
+                                             float py, float z) {
+    if (!(flags & FLAG_ACTIVE)) return a.nx * a.ny * a.nz;
+    const uint32_t ix = lower_index((float)cx + px, a.nx), iy = lower_index((float)cy + py, a.ny);
+    return (ix * a.ny + iy) * a.nz + lower_level(a.lv, z);
+}
+
+// Two adjacent slots per thread with 8-byte accesses, every load issued
+// before the flags are looked at, the level found by the met's bucket table
+// through L1.  32 B a slot, HBM-bound.
 __global__ void __launch_bounds__(256) cell_key_kernel(KeyArgs a, uint32_t* __restrict__ keys,
                                                        uint32_t* __restrict__ vals) {
-    extern __shared__ float s_h[];
-    for (uint32_t i = threadIdx.x; i < a.nz; i += blockDim.x) s_h[i] = a.heights[i];
-    __syncthreads();
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n) return;
-    uint32_t key = a.nx * a.ny * a.nz;
-    if (a.flags[p] & FLAG_ACTIVE) {
-        const uint32_t ix = lower_index((float)a.cell_x[p] + a.pos_x[p], a.nx);
-        const uint32_t iy = lower_index((float)a.cell_y[p] + a.pos_y[p], a.ny);
-        const uint32_t iz = lower_index(level_of_height(s_h, a.nz, a.has_heights, a.monotonic, a.pos_z[p]), a.nz);
-        key = (ix * a.ny + iy) * a.nz + iz;
+    const uint32_t p = 2u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (p + 1u < a.n) {
+        const uint2 f = __ldg(reinterpret_cast<const uint2*>(a.flags + p));
+        const int2 cx = __ldg(reinterpret_cast<const int2*>(a.cell_x + p));
+        const int2 cy = __ldg(reinterpret_cast<const int2*>(a.cell_y + p));
+        const float2 px = __ldg(reinterpret_cast<const float2*>(a.pos_x + p));
+        const float2 py = __ldg(reinterpret_cast<const float2*>(a.pos_y + p));
+        const float2 z = __ldg(reinterpret_cast<const float2*>(a.pos_z + p));
+        *reinterpret_cast<uint2*>(keys + p) = make_uint2(cell_key(a, f.x, cx.x, cy.x, px.x, py.x, z.x),
+                                                         cell_key(a, f.y, cx.y, cy.y, px.y, py.y, z.y));
+        *reinterpret_cast<uint2*>(vals + p) = make_uint2(p, p + 1u);
+    } else if (p < a.n) {
+        keys[p] = cell_key(a, a.flags[p], a.cell_x[p], a.cell_y[p], a.pos_x[p], a.pos_y[p], a.pos_z[p]);
+        vals[p] = p;
     }
-    keys[p] = key;
-    vals[p] = p;
 }
 
 // Bits needed for keys 0..cells (cells itself is the inactive key).
@@ -158,12 +162,11 @@ extern "C" fpg_status fpg_sort_by_cell(fpg_ctx* ctx, fpg_particles* P, const fpg
     a.pos_y = (const float*)P->field[FPG_FIELD_POS_Y];
     a.pos_z = (const float*)P->field[FPG_FIELD_POS_Z];
     a.flags = (const uint32_t*)P->field[FPG_FIELD_FLAGS];
-    a.heights = met->heights_dev;
     a.n = n;
     a.nx = (uint32_t)met->nx; a.ny = (uint32_t)met->ny; a.nz = (uint32_t)met->nz;
-    a.has_heights = met->heights_set && met->heights[met->nz - 1] > 0.0f;
-    a.monotonic = met->monotonic;
-    cell_key_kernel<<<(n + 255) / 256, 256, met->nz * sizeof(float), st>>>(a, s->keys[0], s->vals[0]);
+    a.lv = Levels{met->heights_dev, met->level_table_dev, met->level_inv_w, a.nz,
+                  met->heights_set && met->heights[met->nz - 1] > 0.0f, level_mode(met)};
+    cell_key_kernel<<<(unsigned)(((uint64_t)n + 511u) / 512u), 256, 0, st>>>(a, s->keys[0], s->vals[0]);
     ctx->count();
     FPG_CHECK_LAUNCH();
     cub::DoubleBuffer<uint32_t> kb(s->keys[0], s->keys[1]), vb(s->vals[0], s->vals[1]);
