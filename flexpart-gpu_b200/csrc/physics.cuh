@@ -69,6 +69,56 @@ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1
     return c;
 }
 
+// The first three rounds when only the first counter word differs between
+// the blocks of a launch (the other three are uniform because no block's sum
+// carries): of their six products three depend on uniform words alone and
+// are formed once on the host.
+struct PhiloxHead { uint32_t z1, x2, z2, z3, y3, k0, k1; };
+
+inline void mulhilo(uint32_t m, uint32_t x, uint32_t& hi, uint32_t& lo) {
+    const uint64_t p = (uint64_t)m * x;
+    hi = (uint32_t)(p >> 32);
+    lo = (uint32_t)p;
+}
+
+inline PhiloxHead philox_head(const u32x4& c, uint32_t k0, uint32_t k1) {
+    PhiloxHead h;
+    uint32_t hi1, lo1, hi0, lo0;
+    mulhilo(0xCD9E8D57u, c.z, hi1, lo1);                 // round 1: x = hi1 ^ c.y ^ k0, y = lo1, both uniform
+    const uint32_t x1 = hi1 ^ c.y ^ k0;
+    h.z1 = c.w ^ k1;
+    k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
+    mulhilo(0xD2511F53u, x1, hi0, lo0);                  // round 2
+    h.x2 = lo1 ^ k0;
+    h.z2 = hi0 ^ k1;
+    k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
+    h.y3 = k0;                                           // round 3: x = hi(z2) ^ y2 ^ k0
+    h.z3 = lo0 ^ k1;
+    h.k0 = k0 + 0x9E3779B9u; h.k1 = k1 + 0xBB67AE85u;    // the keys of round 4
+    return h;
+}
+
+__device__ __forceinline__ u32x4 philox_from_head(const PhiloxHead& h, uint32_t cx) {
+    const uint32_t z1 = __umulhi(0xD2511F53u, cx) ^ h.z1, w1 = 0xD2511F53u * cx;
+    const uint32_t x2 = __umulhi(0xCD9E8D57u, z1) ^ h.x2, y2 = 0xCD9E8D57u * z1;
+    const uint32_t z2 = w1 ^ h.z2;
+    u32x4 c;
+    c.x = __umulhi(0xCD9E8D57u, z2) ^ y2 ^ h.y3;
+    c.y = 0xCD9E8D57u * z2;
+    c.z = __umulhi(0xD2511F53u, x2) ^ h.z3;
+    c.w = 0xD2511F53u * x2;
+    uint32_t k0 = h.k0, k1 = h.k1;
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
+        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
+        c = u32x4{hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0};
+        k0 += 0x9E3779B9u;
+        k1 += 0xBB67AE85u;
+    }
+    return c;
+}
+
 // counter_add with a u32 offset (langevin_fused.wgsl:171-180).
 __device__ __forceinline__ u32x4 counter_add(u32x4 b, uint32_t offset) {
     u32x4 r;
@@ -98,6 +148,58 @@ __device__ __forceinline__ float2 box_muller(float u0, float u1) {
     float sn, cs;
     bm_sincos(theta, &sn, &cs);
     return make_float2(radius * cs, radius * sn);
+}
+
+// Two Box-Muller pairs at once with the packed FP32 instructions of sm_100
+// (each lane the IEEE operation of bm_log and bm_sincos, in their order, so
+// the same bits).  a, b: the raw words of two pairs, (.x, .y) each.  The
+// uniform (v >> 8) 2^-24 never exceeds 1 - 2^-24, so box_muller's upper
+// clamps are the identity and only ln's lower one is kept; rintf of the
+// quadrant is an addition of 1.5 2^23, whose low bits are the quadrant.
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float c) { return __ffma2_rn(a, b, f2(c)); }
+
+__device__ __forceinline__ void box_muller2(uint2 a, uint2 b, float2& na, float2& nb) {
+    const float2 ru = make_float2(fmaxf(u32_to_uniform01(a.x), 1.17549435e-38f),
+                                  fmaxf(u32_to_uniform01(b.x), 1.17549435e-38f));
+    // bm_log
+    const uint32_t ba = __float_as_uint(ru.x), bb = __float_as_uint(ru.y);
+    const int32_t ea = (int32_t)(ba - 0x3f3504f3u) >> 23, eb = (int32_t)(bb - 0x3f3504f3u) >> 23;
+    const float2 m = make_float2(__uint_as_float(ba - ((uint32_t)ea << 23)), __uint_as_float(bb - ((uint32_t)eb << 23)));
+    const float2 f = __fadd2_rn(m, f2(-1.0f));
+    const float2 ff = __fmul2_rn(f, f);
+    float2 q = ffma2(f2(-0x1.383114p-4f), f, 0x1.0848f6p-3f);
+    q = ffma2(q, f, -0x1.0f377cp-3f);
+    q = ffma2(q, f, 0x1.227186p-3f);
+    q = ffma2(q, f, -0x1.542768p-3f);
+    q = ffma2(q, f, 0x1.99a3f4p-3f);
+    q = ffma2(q, f, -0x1.000426p-2f);
+    q = ffma2(q, f, 0x1.555550p-2f);
+    q = ffma2(q, f, -0x1.fffff8p-2f);
+    const float2 r = __ffma2_rn(ff, q, f);
+    const float2 fe = make_float2((float)ea, (float)eb);
+    const float2 lg = __ffma2_rn(fe, f2(0x1.62e400p-1f), __ffma2_rn(fe, f2(0x1.7f7d1cp-20f), r));
+    const float2 lr = __fmul2_rn(f2(-2.0f), lg);
+    const float ra = sqrtf(lr.x), rb = sqrtf(lr.y);
+    // bm_sincos
+    const float2 th = __fmul2_rn(f2(6.2831855f), make_float2(u32_to_uniform01(a.y), u32_to_uniform01(b.y)));
+    const float2 qm = __fadd2_rn(__fmul2_rn(th, f2(0x1.45f306p-1f)), f2(12582912.0f));
+    const float2 qf = __fadd2_rn(qm, f2(-12582912.0f));
+    const float2 nq = __fmul2_rn(qf, f2(-1.0f));
+    const float2 t1 = __ffma2_rn(nq, f2(0x1.921fb6p+0f), th);
+    const float2 x = __ffma2_rn(nq, f2(-0x1.ee59dap-50f), __ffma2_rn(nq, f2(-0x1.777a5cp-25f), t1));
+    const float2 x2 = __fmul2_rn(x, x);
+    const float2 ps = ffma2(ffma2(f2(-0x1.994068p-13f), x2, 0x1.110730p-7f), x2, -0x1.555546p-3f);
+    const float2 sn = __ffma2_rn(__fmul2_rn(x, x2), ps, x);
+    const float2 pc = ffma2(ffma2(f2(0x1.99e86ap-16f), x2, -0x1.6c0c28p-10f), x2, 0x1.55554ap-5f);
+    const float2 x4 = __fmul2_rn(__fmul2_rn(x2, f2(-1.0f)), x2);
+    const float2 hc = __ffma2_rn(x2, f2(0.5f), __fmul2_rn(x4, pc));
+    const float2 cs = __ffma2_rn(hc, f2(-1.0f), f2(1.0f));
+    const uint32_t qa = __float_as_uint(qm.x), qb = __float_as_uint(qm.y);
+    const float sa = (qa & 1u) ? cs.x : sn.x, ca = (qa & 1u) ? sn.x : cs.x;
+    const float sb = (qb & 1u) ? cs.y : sn.y, cb = (qb & 1u) ? sn.y : cs.y;
+    na = make_float2(ra * (((qa + 1u) & 2u) ? -ca : ca), ra * ((qa & 2u) ? -sa : sa));
+    nb = make_float2(rb * (((qb + 1u) & 2u) ? -cb : cb), rb * ((qb & 2u) ? -sb : sb));
 }
 
 // ---- scalar helpers of the templated physics --------------------------------
@@ -170,11 +272,18 @@ __device__ __forceinline__ int hanna_regime(float ol, float h) {
 //   unstable: k0 = sigma_u, k1 = T_Lu, k2 = 1.2 w* w*, k3 = -1.4 u* u*,
 //             k4 = w* w*, k5 = 0.15 h
 //   stable:   k0 = 2 u*,  k1 = 1.3 u*, k2 = dsigma_w/dz, k5 = 0.15 h, k6 = 0.1 h
+// A record in memory carries REGIME_PLAIN beside its regime when every
+// parameter lies inside the bounds of plain_cell, which no real boundary
+// layer leaves; the step then runs without the checks that cannot fire.
+enum { REGIME_MASK = 3, REGIME_PLAIN = 4 };
+
 struct __align__(16) CellHanna {
     float ust, wst, h, ol;
     float k0, k1, k2, k3;
     float k4, k5, k6;
     int regime;
+    __device__ __forceinline__ int kind() const { return regime & REGIME_MASK; }
+    __device__ __forceinline__ bool plain() const { return (regime & REGIME_PLAIN) != 0; }
 };
 
 // The constants of `regime` for a cell (ust, wst, h unfloored; ol = L).
@@ -230,7 +339,19 @@ __device__ __forceinline__ CellHanna ld_cell_hanna(const CellHanna* p) {
     return c;
 }
 
-__device__ __forceinline__ void st_cell_hanna(CellHanna* p, const CellHanna& c) {
+// Whether the finite and sign checks of the Hanna profiles and Langevin
+// updates are the identity for a cell (see turbulence_plain): bounded u*, w*
+// and h, and for the unstable branch a bounded Obukhov length, which make
+// sigma_w >= 0.01 and every time scale and gradient finite.  False for NaN.
+__device__ __forceinline__ bool plain_cell(const CellHanna& c) {
+    const bool scales = c.ust >= 1.0e-4f && c.ust <= 1.0e3f && c.wst >= 0.0f && c.wst <= 1.0e3f && c.h >= 1.0f &&
+                        c.h <= 1.0e6f;
+    return scales && (c.kind() != REGIME_UNSTABLE || (c.ol <= -1.0e-3f && c.ol >= -1.0e6f));
+}
+
+__device__ __forceinline__ void st_cell_hanna(CellHanna* p, const CellHanna& cell) {
+    CellHanna c = cell;
+    c.regime |= plain_cell(c) ? REGIME_PLAIN : 0;
     float4* q = reinterpret_cast<float4*>(p);
     q[0] = make_float4(c.ust, c.wst, c.h, c.ol);
     q[1] = make_float4(c.k0, c.k1, c.k2, c.k3);
@@ -260,8 +381,8 @@ __device__ __forceinline__ HannaT<T> compute_hanna_cell_t(const CellHanna& c, T 
     const T z = xclamp(z_in, 0.0f, h);
     const T zeta = xclamp(xdiv(z, h), 0.0f, 1.0f);
     T sigu, sigv, sigw, dsigwdz, tlu, tlv, tlw;
-    o.regime = c.regime;
-    if (c.regime == REGIME_NEUTRAL) {
+    o.regime = c.kind();
+    if (c.kind() == REGIME_NEUTRAL) {
         const T corr = xdiv(z, ust);
         sigu = 1.0e-2f + c.k0 * xexp(-3.0e-4f * corr);
         sigw = c.k1 * xexp(-2.0e-4f * corr);
@@ -282,7 +403,7 @@ __device__ __forceinline__ HannaT<T> compute_hanna_cell_t(const CellHanna& c, T 
         if (!finitef(val(tlv))) tlv = T(10.0f);
         if (!finitef(val(tlw))) tlw = T(30.0f);
         if (!finitef(val(dsigwdz))) dsigwdz = T(1.0e-10f);
-    } else if (c.regime == REGIME_UNSTABLE) {
+    } else if (c.kind() == REGIME_UNSTABLE) {
         // sigma_u, sigma_v, T_Lu, T_Lv: the cell's, already final
         sigu = T(c.k0);
         sigv = sigu;
@@ -336,13 +457,13 @@ __device__ __forceinline__ void hanna_short_cell_t(const CellHanna& c, T z_in, T
     const T z = xclamp(z_in, 0.0f, c.h);
     const T zeta = xclamp(xdiv(z, c.h), 0.0f, 1.0f);
     T sigw, dsigwdz, tlw;
-    if (c.regime == REGIME_NEUTRAL) {
+    if (c.kind() == REGIME_NEUTRAL) {
         const T corr = xdiv(z, c.ust);
         sigw = c.k1 * xexp(-2.0e-4f * corr);
         dsigwdz = -2.0e-4f * sigw;
         sigw = sigw + 1.0e-2f;
         tlw = xdiv(xdiv(0.5f * z, sigw), (1.0f + 1.5e-3f * corr));
-    } else if (c.regime == REGIME_UNSTABLE) {
+    } else if (c.kind() == REGIME_UNSTABLE) {
         hanna_unstable_w<T>(c, z, zeta, sigw, dsigwdz, tlw);
     } else {
         sigw = 1.0e-2f + c.k1 * (1.0f - zeta);
@@ -350,7 +471,7 @@ __device__ __forceinline__ void hanna_short_cell_t(const CellHanna& c, T z_in, T
         tlw = xdiv(c.k6, sigw) * xpow(zeta, 0.8f);
     }
     tlw = xmax(tlw, 30.0f);
-    if (c.regime != REGIME_STABLE) {
+    if (c.kind() != REGIME_STABLE) {
         if (val(dsigwdz) == 0.0f) dsigwdz = T(1.0e-10f);
         if (!finitef(val(dsigwdz))) dsigwdz = T(1.0e-10f);
     }
@@ -412,6 +533,115 @@ __device__ __forceinline__ float langevin_h(float prev, float sigma, float tl, f
 __device__ __forceinline__ float langevin_v(float prev, float sigma_w, float tlw, float dsigwdz, float dt,
                                             float rho, float eta) {
     return langevin_v_t<float>(prev, sigma_w, tlw, dsigwdz, dt, rho, eta);
+}
+
+// ---- the same without the checks that cannot fire ---------------------------
+// For a cell inside plain_cell's bounds and a finite height, sigma and every
+// time scale come out finite and positive, so the reference's sanitising of
+// them (hanna.rs:113-141) and of the updated velocity (langevin.rs:128,168)
+// returns its argument: the functions below leave it out and take the
+// approximate reciprocals once.  sdiv(a, b) is a times rcp(b) in the step's
+// units (the same bits over 3e9 random pairs with |b| in [1e-4, 1e6]), so
+// z / h with a kept 1 / h, or two quotients over one sigma_w, round as
+// written there.  d(sigma_w)/dz can still be zero (a neutral cell far above
+// its scale height, or an exact cancellation) and keeps its test.
+__device__ __forceinline__ float rcp_of(float b) {
+#ifdef FPG_RECIPROCAL_DIVISION
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+#else
+    return 1.0f / b;
+#endif
+}
+
+struct PlainRates { float h, other; };     // 1 / h, and 1 / u* (neutral) or 1 / L (unstable)
+
+__device__ __forceinline__ PlainRates plain_rates(const CellHanna& c) {
+    return PlainRates{rcp_of(c.h), rcp_of(c.kind() == REGIME_NEUTRAL ? c.ust : c.ol)};
+}
+
+struct PlainHanna { float sigu, sigv, tlu, tlv; };
+
+// sigma_w, d(sigma_w)/dz and T_Lw at a height z in [0, h], and with `first`
+// the horizontal parameters too (compute_hanna_cell_t and hanna_short_cell_t give
+// the same vertical ones).
+__device__ __forceinline__ void plain_hanna(const CellHanna& c, const PlainRates& r, float z, bool first,
+                                            float& sigw, float& dsigwdz, float& tlw, PlainHanna& o) {
+    const float zeta = fminf(z * r.h, 1.0f);
+    if (c.kind() == REGIME_UNSTABLE) {
+        const float cz = xcbrt(zeta);
+        const float z23 = cz * cz;
+        const float sigw_sq = c.k2 * (1.0f - 0.9f * zeta) * z23 + (1.8f - 1.4f * zeta) * c.ust * c.ust;
+        sigw = sqrtf(sigw_sq) + 1.0e-2f;
+        const float rs = rcp_of(sigw);
+        const float zm13 = rcp_of(zeta >= 1.0e-3f ? cz : pow_third(1.0e-3f));
+        dsigwdz = 0.5f * rs * r.h * (c.k3 + c.k4 * (0.8f * zm13 - 1.8f * z23));
+        if (z < fabsf(c.ol)) tlw = 0.1f * z * rcp_of(sigw * (0.55f - 0.38f * fabsf(z * r.other)));
+        else if (zeta < 0.1f) tlw = 0.59f * z * rs;
+        else tlw = c.k5 * rs * (1.0f - xexp(-5.0f * zeta));
+        dsigwdz = dsigwdz == 0.0f ? 1.0e-10f : dsigwdz;
+        if (first) { o.sigu = c.k0; o.sigv = c.k0; o.tlu = c.k1; o.tlv = c.k1; }
+    } else if (c.kind() == REGIME_NEUTRAL) {
+        const float corr = z * r.other;
+        sigw = c.k1 * xexp(-2.0e-4f * corr);
+        dsigwdz = -2.0e-4f * sigw;
+        sigw = sigw + 1.0e-2f;
+        tlw = 0.5f * z * rcp_of(sigw) * rcp_of(1.0f + 1.5e-3f * corr);
+        dsigwdz = dsigwdz == 0.0f ? 1.0e-10f : dsigwdz;
+        if (first) {
+            o.sigu = 1.0e-2f + c.k0 * xexp(-3.0e-4f * corr);
+            o.sigv = sigw;
+            o.tlu = o.tlv = fmaxf(tlw, 10.0f);
+        }
+    } else {
+        const float one_minus = 1.0f - zeta;
+        sigw = 1.0e-2f + c.k1 * one_minus;
+        dsigwdz = c.k2;
+        tlw = c.k6 * rcp_of(sigw) * __powf(zeta, 0.8f);          // 0 at zeta = 0, as powf
+        if (first) {
+            o.sigu = 1.0e-2f + c.k0 * one_minus;
+            o.sigv = sigw;
+            const float tlu = c.k5 * rcp_of(o.sigu) * sqrtf(zeta);
+            o.tlu = fmaxf(tlu, 10.0f);
+            o.tlv = fmaxf(0.467f * tlu, 10.0f);
+        }
+    }
+    tlw = fmaxf(tlw, 30.0f);
+}
+
+// The decay and noise factors of the Ornstein-Uhlenbeck update over dt at
+// time scale tl (langevin_h_t, langevin_v_t): exp(-r) <= 0.61 for r >= 0.5.
+__device__ __forceinline__ void plain_factors(float dt, float tl, float& decay, float& noise, bool& linear) {
+    const float ratio = sdiv(dt, tl);
+    linear = ratio < 0.5f;
+    if (linear) {
+        decay = 1.0f - ratio;
+        noise = sqrtf(2.0f * ratio);
+    } else {
+        decay = xexp(-ratio);
+        noise = sqrtf(1.0f - decay * decay);
+    }
+}
+
+// langevin_h_t of both horizontal components: the factors depend on the time
+// scale only, which the components share except in stable cells.
+__device__ __forceinline__ void plain_langevin_h(const PlainHanna& o, float dt, float2 eta, float& tu, float& tv) {
+    float decay, noise;
+    bool linear;
+    plain_factors(dt, o.tlu, decay, noise, linear);
+    tu = decay * tu + eta.x * o.sigu * noise;
+    if (o.tlv != o.tlu) plain_factors(dt, o.tlv, decay, noise, linear);
+    tv = decay * tv + eta.y * o.sigv * noise;
+}
+
+__device__ __forceinline__ float plain_langevin_v(float prev, float sigma_w, float tlw, float dsigwdz, float dt,
+                                                  float rho, float eta) {
+    const float drift = sigma_w * (dsigwdz + rho * sigma_w);
+    float decay, noise;
+    bool linear;
+    plain_factors(dt, tlw, decay, noise, linear);
+    return decay * prev + eta * sigma_w * noise + (linear ? dt : tlw * (1.0f - decay)) * drift;
 }
 
 // ---- Deposition --------------------------------------------------------------

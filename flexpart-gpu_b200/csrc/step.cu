@@ -48,6 +48,44 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
     particle_step(a, lv, p, p, a.alpha, a.counter, a.key0, a.key1);
 }
 
+// The production form of the pass (production_form in step_core.cuh), what
+// the forward loop launches.  Instruction issue binds it: 1,480 warp
+// instructions per 32 particles against 1,771 of the general body, 0.77-0.79
+// of the issue slots used.  At 10 M particles of the global run 609 -> 532 us
+// in a mixed population and 577 -> 479 us right after a reorder.
+template <bool kWet, int BLOCK, int MINB>
+__global__ void __launch_bounds__(BLOCK, MINB) production_step_kernel(StepArgs a) {
+    const uint32_t p = blockIdx.x * BLOCK + threadIdx.x;
+    if (p < a.n) production_step<kWet, true>(a, p, p, a.alpha, a.counter, a.key0, a.key1);
+}
+
+// Its block size and registers by the number of slots.  Small CTAs measure
+// best throughout: a warp that waits for its gathers or takes a rare branch
+// holds back one other at most.  Up to one wave of 24 warps per SM (113,664
+// slots on 148 SMs) one-warp CTAs with the 74 registers the body wants, spread
+// over all SMs: 6.4 us at 1,003 slots and 10.6 us at 100 k, against 7.5 and
+// 11.4 us with 40 or 48 registers.  Above, 56 registers (18 CTAs of 64):
+// 22.9 us at 300 k and 58.5 us at 1 M, against 24.4 and 66.1 us with one-warp
+// CTAs and 24.4 and 60.7 us with 40 registers.  From 4 M slots on, 40
+// registers and 48 warps per SM, which hide the gathers of a mixed population
+// better: equal at 3 M (171 us), 533 against 541 us at 10 M.
+struct ProductionShape {
+    uint32_t block;
+    void (*dry)(StepArgs);
+    void (*wet)(StepArgs);
+};
+
+template <int BLOCK, int MINB>
+constexpr ProductionShape production_shape() {
+    return ProductionShape{BLOCK, production_step_kernel<false, BLOCK, MINB>, production_step_kernel<true, BLOCK, MINB>};
+}
+
+ProductionShape production_shape_for(uint32_t n, int sm_count) {
+    if (n <= (uint32_t)sm_count * 24u * 32u) return production_shape<32, 24>();
+    if (n < 4000000u) return production_shape<64, 18>();
+    return production_shape<64, 24>();
+}
+
 // The same pass under another launch shape: BLOCK threads per CTA compiled
 // for MINB resident CTAs per SM, PPT particles per thread (slots of one CTA
 // are contiguous; thread t takes t, t + BLOCK, ...); with several particles
@@ -77,7 +115,9 @@ struct StepShape {
     void (*kernel)(StepArgs);
 };
 
-// Shape 0 is fused_step_kernel itself (the default).
+// Shape 0 (the default) is the general body for everything outside the
+// production form, which has its own launch shapes; the others run the
+// general body always.
 const StepShape kStepShapes[] = {
     {256, 5, 1, fused_step_kernel},
     {256, 4, 1, fused_step_shape_kernel<256, 4, 1>},
@@ -599,8 +639,16 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     a.wet_prob = prm->wet_probability_dev;
 
     cudaStream_t s = ctx->pick(stream);
-    const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
-    sh.kernel<<<blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s>>>(a);
+    // no block's counter carries out of its first word
+    const bool no_carry = (uint64_t)prm->counter[0] + 2u * (uint64_t)n <= (1ull << 32);
+    if (ctx->step_shape == 0 && no_carry && production_form(a)) {
+        a.head = philox_head(a.counter, a.key0, a.key1);
+        const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
+        (wet ? ps.wet : ps.dry)<<<blocks_for(n, ps.block), ps.block, 0, s>>>(a);
+    } else {
+        const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
+        sh.kernel<<<blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s>>>(a);
+    }
     ctx->count();
     FPG_CHECK_LAUNCH();
     if (turb && next_counter) {
@@ -792,7 +840,7 @@ __global__ void __launch_bounds__(256) langevin_record_kernel(RecordTurbArgs a) 
     // the vertical re-evaluation's constants; its branch is hanna_short_w's
     // test on (L, max(h, 1))
     const CellHanna cell = cell_hanna(r.ust, r.wst, r.ol, r.h);
-    hn.regime = cell.regime;
+    hn.regime = cell.kind();
     float pz = a.pos_z[p], tu = a.turb_u[p], tv = a.turb_v[p], tw = a.turb_w[p];
     const int32_t cbt_in = a.n_sub == 0u ? 0 : a.cbt[p];
     int32_t cbt = cbt_in;

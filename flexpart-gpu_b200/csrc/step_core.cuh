@@ -9,6 +9,11 @@
 
 namespace fpg {
 
+// How the level search runs: the reference's linear scan (heights not
+// sorted), a binary search (sorted), or a bucket table plus a short scan
+// (sorted with h[nz-1] > h[0]).  All three return the scan's index.
+enum { LEVELS_SCAN = 0, LEVELS_BISECT = 1, LEVELS_TABLE = 2 };
+
 struct StepArgs {
     int32_t* cell_x; int32_t* cell_y;
     float* pos_x; float* pos_y; float* pos_z;
@@ -48,12 +53,32 @@ struct StepArgs {
     const float2* wet_cells;
     uint32_t wnx, wny;
     float* wet_prob;
+    PhiloxHead head;                     // of the launch's counter and key, for the production form
 };
 
-// How the level search runs: the reference's linear scan (heights not
-// sorted), a binary search (sorted), or a bucket table plus a short scan
-// (sorted with h[nz-1] > h[0]).  All three return the scan's index.
-enum { LEVELS_SCAN = 0, LEVELS_BISECT = 1, LEVELS_TABLE = 2 };
+// The production form of the step (production_step below): the forward
+// loop's own settings.  It is taken when every one of these holds, which the
+// host sees from the arguments; anything else runs the general body, and
+// both give the same bits.
+//   * all of advection, turbulence with four sub-steps and uniform dry
+//     deposition, with per-cell wet deposition or none, no probability
+//     outputs and one species;
+//   * level heights searched by the bucket table (finite, sorted, top > 0);
+//   * PBL and wet cells on the met's horizontal grid, so a particle's cell
+//     indices are the cell it was advected into;
+//   * a bounded time step and density gradient, and a reflection floor in
+//     [0, 1) m, below any mixing height (turbulence_plain);
+//   * a bracket below 4 GB (32-bit node offsets).
+inline bool production_form(const StepArgs& a) {
+    const uint32_t most = FPG_STAGE_ADVECT | FPG_STAGE_TURBULENCE | FPG_STAGE_DRY;
+    const bool wet = a.stages == (most | FPG_STAGE_WET);
+    if (!wet && a.stages != most) return false;
+    if (a.n_sub != 4u || a.dry_mode != FPG_FORCING_UNIFORM || a.dry_prob || a.n_species != 1) return false;
+    if (wet && (a.wet_mode != FPG_FORCING_PER_CELL || a.wet_prob || a.wnx != a.nx || a.wny != a.ny)) return false;
+    if (!a.has_heights || a.level_mode != LEVELS_TABLE || a.pnx != a.nx || a.pny != a.ny) return false;
+    if ((uint64_t)a.nx * a.ny * a.nz >= (1ull << 27)) return false;
+    return a.tdt > 0.0f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f && a.rho <= 1.0e3f && a.zmin >= 0.0f && a.zmin < 1.0f;
+}
 
 // The search a met's heights allow (host side).
 inline int level_mode(const fpg_met* m) {
@@ -158,6 +183,15 @@ __device__ __forceinline__ Node ld_node(const float4* br, uint32_t n) {
     asm("{\n.reg .f32 pad<2>;\nld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,pad0,pad1}, [%6];\n}"
         : "=f"(v.uv0.x), "=f"(v.uv0.y), "=f"(v.uv1.x), "=f"(v.uv1.y), "=f"(v.w01.x), "=f"(v.w01.y)
         : "l"(br + 2u * n));
+    return v;
+}
+
+// The same at a byte offset.
+__device__ __forceinline__ Node ld_node(const char* br, uint32_t offset) {
+    Node v;
+    asm("{\n.reg .f32 pad<2>;\nld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,pad0,pad1}, [%6];\n}"
+        : "=f"(v.uv0.x), "=f"(v.uv0.y), "=f"(v.uv1.x), "=f"(v.uv1.y), "=f"(v.w01.x), "=f"(v.w01.y)
+        : "l"(br + offset));
     return v;
 }
 
@@ -465,6 +499,149 @@ __device__ __forceinline__ void particle_step(const StepArgs& a, const Levels& l
     particle_step_t<NoTape>(a, lv, p, rng_index, alpha, counter, key0, key1, t);
 }
 
+
+// Turbulence of one particle with four sub-steps in a cell inside
+// plain_cell's bounds, for |tu| + |tv| + |tw| < 1e30, a finite height and
+// |rho| <= 1e3, dt <= 1e6: turbulence_update's values without its checks.
+// With u*, w* <= 1e3 and h >= 1, sigma is at most 2.5e3 and d(sigma)/dz at
+// most 6e8, so a velocity gains at most 1e19 and stays finite.  The Hanna
+// evaluation opens each sub-step, so the loop holds one copy of it.
+__device__ __forceinline__ void turbulence_plain(const StepArgs& a, const CellHanna& cell, float2 e_uv, float2 e_w01,
+                                                 float2 e_w23, float& pz, float& tu, float& tv, float& tw,
+                                                 int32_t& cbt) {
+    const PlainRates rates = plain_rates(cell);
+    const float dt_sub = a.tdt * 0.25f, h = cell.h, zmin = a.zmin;
+    float e0 = e_w01.x, e1 = e_w01.y, e2 = e_w23.x;
+#pragma unroll 1
+    for (uint32_t sub = 0; sub < 4u; ++sub) {
+        float sigw, dsigwdz, tlw;
+        PlainHanna o;
+        plain_hanna(cell, rates, fminf(pz, h), sub == 0u, sigw, dsigwdz, tlw, o);
+        if (sub == 0u) plain_langevin_h(o, a.tdt, e_uv, tu, tv);
+        tw = plain_langevin_v(tw, sigw, tlw, dsigwdz, dt_sub, a.rho, e0);
+        e0 = e1; e1 = e2; e2 = e_w23.y;
+        pz = pz + tw * dt_sub;
+        // the first bounce by selects, as in turbulence_from_hanna (2 zmin
+        // and 2 h are exact, so the fused form rounds once, as there)
+        float z = pz;
+        const bool lo = z < zmin, any = lo || z > h;
+        z = any ? fmaf(2.0f, lo ? zmin : h, -z) : z;
+        cbt = any ? -cbt : cbt;
+        tw = any ? -tw : tw;
+        if (any && (z < zmin || z > h)) {
+            for (int bounce = 1; bounce < 10; ++bounce) {
+                if (z < zmin) { z = 2.0f * zmin - z; cbt = -cbt; tw = -tw; }
+                else if (z > h) { z = 2.0f * h - z; cbt = -cbt; tw = -tw; }
+                else break;
+            }
+            z = clampf(z, zmin, h);
+        }
+        pz = z;
+    }
+}
+
+// sample_dual of the production form: 32-bit byte offsets from the bracket's
+// base, the far corners one stride on unless the near one is the last, and
+// with kInside (x, y in the grid and z >= 0) no clamps, which leave a
+// coordinate there as it is.
+template <bool kInside>
+__device__ __forceinline__ float3 sample_production(const StepArgs& a, const Levels& lv, float x, float y, float z,
+                                                    float alpha) {
+    float l = meters_to_level(lv, z);
+    if constexpr (!kInside) {
+        x = clampf(x, 0.0f, (float)(a.nx - 1u));
+        y = clampf(y, 0.0f, (float)(a.ny - 1u));
+        l = fmaxf(l, 0.0f);
+    }
+    l = fminf(l, (float)(a.nz - 1u));          // a quotient at a level's top may exceed one by its rounding
+    const uint32_t ix = (uint32_t)x, iy = (uint32_t)y, iz = (uint32_t)l;
+    const float tx = x - (float)ix, ty = y - (float)iy, tz = l - (float)iz;
+    const uint32_t sy = 32u * a.nz, sx = sy * a.ny;
+    const uint32_t dx = ix + 1u < a.nx ? sx : 0u, dy = iy + 1u < a.ny ? sy : 0u, dz = iz + 1u < a.nz ? 32u : 0u;
+    const uint32_t o00 = ix * sx + iy * sy + iz * 32u, o01 = o00 + dy;
+    const char* br = reinterpret_cast<const char*>(a.bracket);
+    const float2 tx2 = make_float2(tx, tx), sx2 = make_float2(1.0f - tx, 1.0f - tx);
+    const float2 ty2 = make_float2(ty, ty), sy2 = make_float2(1.0f - ty, 1.0f - ty);
+    const float2 tz2 = make_float2(tz, tz), sz2 = make_float2(1.0f - tz, 1.0f - tz);
+    const Node l00 = lerp_node(ld_node(br, o00), ld_node(br, o00 + dx), sx2, tx2);
+    const Node l10 = lerp_node(ld_node(br, o01), ld_node(br, o01 + dx), sx2, tx2);
+    const Node l0 = lerp_node(l00, l10, sy2, ty2);
+    const Node l01 = lerp_node(ld_node(br, o00 + dz), ld_node(br, o00 + dx + dz), sx2, tx2);
+    const Node l11 = lerp_node(ld_node(br, o01 + dz), ld_node(br, o01 + dx + dz), sx2, tx2);
+    const Node l1 = lerp_node(l01, l11, sy2, ty2);
+    const Node t = lerp_node(l0, l1, sz2, tz2);
+    const float2 ta = make_float2(alpha, alpha), sa = make_float2(1.0f - alpha, 1.0f - alpha);
+    const float2 uv = lerp2(t.uv0, t.uv1, sa, ta);
+    return make_float3(uv.x, uv.y, lerpf(t.w01.x, t.w01.y, alpha));
+}
+
+// particle_step for arguments in the production form: the same operations
+// with the settings known at compile time, the cell of the PBL and wet
+// lookups taken from the advected position, the counter's uniform rounds
+// from the host (`kHead`: a.head holds them and no block's counter carries)
+// and the turbulence without checks wherever the cell and the velocities
+// allow it.
+template <bool kWet, bool kHead>
+__device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, uint32_t rng_index, float alpha,
+                                                u32x4 counter, uint32_t key0, uint32_t key1) {
+    if (!(a.flags[p] & FLAG_ACTIVE)) return;
+    const Levels lv{a.heights, a.level_table, a.level_inv_w, a.nz, 1, LEVELS_TABLE};
+    float tu = a.turb_u[p], tv = a.turb_v[p];
+    const float x0 = (float)a.cell_x[p] + a.pos_x[p];
+    const float y0 = (float)a.cell_y[p] + a.pos_y[p];
+    const float z0 = a.pos_z[p];
+    const float3 s0 = sample_production<false>(a, lv, x0, y0, z0, alpha);
+    const float u0 = s0.x + tu, v0 = s0.y + tv, w0 = s0.z;
+    const float xmax = (float)(a.nx - 1u), ymax = (float)(a.ny - 1u), ztop = lv.h[a.nz - 1u];
+    const float3 s1 = sample_production<true>(a, lv, clampf(x0 + (u0 * a.xs) * a.dt, 0.0f, xmax),
+                                  clampf(y0 + (v0 * a.ys) * a.dt, 0.0f, ymax),
+                                  clampf(z0 + (w0 * a.zs) * a.dt, 0.0f, ztop), alpha);
+    const float cu = 0.5f * (u0 + (s1.x + tu)), cv = 0.5f * (v0 + (s1.y + tv)), cw = 0.5f * (w0 + s1.z);
+    const float x1 = clampf(x0 + (cu * a.xs) * a.dt, 0.0f, xmax);
+    const float y1 = clampf(y0 + (cv * a.ys) * a.dt, 0.0f, ymax);
+    float pz = clampf(z0 + (cw * a.zs) * a.dt, 0.0f, ztop);
+    // split_coord of a coordinate inside the grid: on the last cell the
+    // remainder is zero already
+    const int32_t cx = (int32_t)x1, cy = (int32_t)y1;
+    a.cell_x[p] = cx; a.cell_y[p] = cy;
+    a.pos_x[p] = x1 - (float)cx; a.pos_y[p] = y1 - (float)cy;
+    a.vel_u[p] = cu; a.vel_v[p] = cv; a.vel_w[p] = cw;
+
+    // cell + fraction is the advected coordinate again, whose floor is the cell
+    const uint32_t c = (uint32_t)cx * a.ny + (uint32_t)cy;
+    const CellHanna cell = ld_cell_hanna(a.hcell + c);
+    u32x4 b0, b1;
+    if constexpr (kHead) {
+        const uint32_t w = counter.x + 2u * rng_index;
+        b0 = philox_from_head(a.head, w);
+        b1 = philox_from_head(a.head, w + 1u);
+    } else {
+        b0 = philox4x32_10(counter_add(counter, rng_index * 2u), key0, key1);
+        b1 = philox4x32_10(counter_add(counter, rng_index * 2u + 1u), key0, key1);
+    }
+    float2 e_uv, e_w01;
+    box_muller2(make_uint2(b0.x, b0.y), make_uint2(b0.z, b0.w), e_uv, e_w01);
+    const float2 e_w23 = box_muller(u32_to_uniform01(b1.x), u32_to_uniform01(b1.y));
+    float tw = a.turb_w[p];
+    const int32_t cbt_in = a.cbt[p];
+    int32_t cbt = cbt_in;
+    if (cell.plain() && fabsf(tu) + fabsf(tv) + fabsf(tw) < 1.0e30f)
+        turbulence_plain(a, cell, e_uv, e_w01, e_w23, pz, tu, tv, tw, cbt);
+    else
+        turbulence_update<float>(a, cell, e_uv, e_w01, e_w23, pz, tu, tv, tw, cbt);
+    if (cbt != cbt_in) a.cbt[p] = cbt;
+    a.turb_u[p] = tu; a.turb_v[p] = tv; a.turb_w[p] = tw;
+    a.pos_z[p] = pz;
+
+    // dry, then wet survival
+    float m = a.mass[0][p];
+    if (!(pz >= 2.0f * a.href)) m = m * dry_survival(a.dry_v, a.tdt, a.href);
+    if constexpr (kWet) {
+        const float2 w = __ldg(a.wet_cells + c);
+        m = m * (1.0f - wet_probability(w.x, a.tdt, w.y));
+    }
+    a.mass[0][p] = m;
+}
 
 __device__ __forceinline__ float sp_(float v, float fb) { return (finitef(v) && v > 0.0f) ? v : fb; }
 __device__ __forceinline__ float snn_(float v, float fb) { return (finitef(v) && v >= 0.0f) ? v : fb; }

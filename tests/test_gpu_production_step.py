@@ -1,0 +1,108 @@
+"""The step's production form (its own kernels, compile-time settings, no
+sanitising where it cannot fire) against the general body, bit for bit: the
+general body runs when a launch shape is selected by hand."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from flexpart_gpu import api
+from flexpart_gpu.records import FIELDS
+from helpers import population, production_params, small_met
+
+pytestmark = pytest.mark.gpu
+
+GENERAL = {"block_threads": 256, "min_blocks_per_sm": 4, "particles_per_thread": 1}
+PRODUCTION = {"block_threads": 256, "min_blocks_per_sm": 5, "particles_per_thread": 1}
+ODD = np.array([0.0, -1.0, np.nan, np.inf, 1e-30, 5e2, 2e3, 1e12], np.float32)
+
+
+@pytest.fixture(scope="module")
+def world():
+    ctx = api.Context(0)
+    spec, frames, met = small_met()
+    m = api.Met(ctx, spec.nx, spec.ny, spec.nz)
+    m.upload_frame(0, met["u0"], met["v0"], met["w0"])
+    m.upload_frame(1, met["u1"], met["v1"], met["w1"])
+    m.set_level_heights(met["heights"])
+    cells = spec.nx * spec.ny
+    rng = np.random.default_rng(3)
+    # every regime, and some cells outside any real boundary layer
+    ust = rng.uniform(0.05, 0.8, cells).astype(np.float32)
+    wst = np.where(rng.random(cells) < 0.5, rng.uniform(0, 2.5, cells), 0).astype(np.float32)
+    h = rng.uniform(60, 2500, cells).astype(np.float32)
+    oli = rng.normal(0, 0.02, cells).astype(np.float32)
+    for field in (ust, wst, h, oli):
+        at = rng.choice(cells, 24, replace=False)
+        field[at] = np.resize(ODD, 24)
+    pbl = api.Pbl(ctx, spec.nx, spec.ny)
+    pbl.upload(ust, wst, h, oli)
+    wet = api.CellField(ctx, spec.nx, spec.ny)
+    lam = np.where(rng.random(cells) < 0.4, rng.uniform(0, 5e-4, cells), 0).astype(np.float32)
+    frac = rng.uniform(-0.1, 1.1, cells).astype(np.float32)
+    lam[:6], frac[6:12] = np.resize(ODD, 6), np.resize(ODD, 6)
+    wet.upload(lam, frac)
+    return ctx, spec, m, pbl, wet
+
+
+def _records(spec, n):
+    rec = population(spec.nx, spec.ny, n, seed=n)
+    rng = np.random.default_rng(n)
+    if n > 64:
+        for k, name in enumerate(("turb_u", "turb_v", "turb_w", "pos_z")):
+            at = rng.choice(np.arange(16, n), 12, replace=False)
+            rec[name][at] = np.resize(np.array([np.nan, np.inf, -np.inf, 1e35, -3e29, 2e4], np.float32), 12)
+        rec["cell_x"][20:24] = [-3, 1000, spec.nx - 1, 0]
+        rec["pos_x"][22:24] = [0.7, -0.5]
+    rec["mass"][:, 1:] = 0.0
+    rec["cbt"] = np.where(rng.random(n) < 0.5, 1, -1)
+    return rec
+
+
+def _run(world, rec, shape, steps, **kw):
+    ctx, spec, m, pbl, wet = world
+    p = api.Particles(ctx, len(rec))
+    p.upload(rec)
+    api.set_step_tuning(ctx, shape)
+    prm = production_params(**kw)
+    for _ in range(steps):
+        prm.counter[:] = api.step(ctx, p, m, pbl, prm, wet if prm.wet_mode == 3 else None)
+        prm.dt_seconds = -prm.dt_seconds
+    api.set_step_tuning(ctx, PRODUCTION)
+    return {name: p.read_field(name).view(np.uint32) for name, _ in FIELDS}
+
+
+def _same(a, b):
+    for name in a:
+        if not np.array_equal(a[name], b[name]):
+            at = np.flatnonzero(a[name] != b[name])
+            raise AssertionError(f"{name}: {at.size} slots differ, first {at[:5]}: "
+                                 f"{a[name][at[:5]].view(np.float32)} {b[name][at[:5]].view(np.float32)}")
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1003, 148 * 24 * 32, 148 * 24 * 32 + 1])
+@pytest.mark.parametrize("wet", [0, 3])
+def test_production_form_gives_the_general_bits(world, n, wet):
+    rec = _records(world[1], n)
+    kw = dict(wet_mode=wet, rho_grad_over_rho=-1e-4)
+    _same(_run(world, rec, PRODUCTION, 3, **kw), _run(world, rec, GENERAL, 3, **kw))
+
+
+@pytest.mark.parametrize("counter", [(0xFFFFFFFF - 2005, 0xFFFFFFFF, 3, 4), (0xFFFFFFFF - 2006, 7, 0xFFFFFFFF, 1),
+                                     (0xFFFFFFF0, 0xFFFFFFFF, 0xFFFFFFFF, 2)])
+def test_counters_at_the_edge_of_a_carry(world, counter):
+    rec = _records(world[1], 1003)
+    kw = dict(counter=counter, key=(0xDECAFBAD, 0x12345678))
+    _same(_run(world, rec, PRODUCTION, 2, **kw), _run(world, rec, GENERAL, 2, **kw))
+
+
+def test_largest_shape(world):
+    rec = np.resize(_records(world[1], 50_021), 4_000_001)
+    _same(_run(world, rec, PRODUCTION, 1, wet_mode=3), _run(world, rec, GENERAL, 1, wet_mode=3))
+
+
+@pytest.mark.parametrize("kw", [dict(n_substeps=2), dict(min_height_m=1.5), dict(dry_mode=0), dict(rho_grad_over_rho=5e3),
+                                dict(turb_dt_seconds=2e6)])
+def test_settings_outside_the_form_run_the_general_body(world, kw):
+    rec = _records(world[1], 1003)
+    _same(_run(world, rec, PRODUCTION, 2, **kw), _run(world, rec, GENERAL, 2, **kw))
