@@ -34,6 +34,8 @@ struct ScenDev {
     uint32_t instance;               // source-inversion instance (0 outside inversions)
     uint32_t key0, key1;
     u32x4 counter;
+    PhiloxHead head;                 // of the coming step's counter, and whether no block's counter
+    uint32_t head_ok;                // carries out of its first word (batch_advance_kernel)
     uint32_t released, rel_lo, rel_hi;
     float mass_per_particle;
     int64_t start, end;

@@ -72,16 +72,16 @@ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1
 // The first three rounds when only the first counter word differs between
 // the blocks of a launch (the other three are uniform because no block's sum
 // carries): of their six products three depend on uniform words alone and
-// are formed once on the host.
+// are formed once, on the host or per scenario of a batch.
 struct PhiloxHead { uint32_t z1, x2, z2, z3, y3, k0, k1; };
 
-inline void mulhilo(uint32_t m, uint32_t x, uint32_t& hi, uint32_t& lo) {
+__host__ __device__ inline void mulhilo(uint32_t m, uint32_t x, uint32_t& hi, uint32_t& lo) {
     const uint64_t p = (uint64_t)m * x;
     hi = (uint32_t)(p >> 32);
     lo = (uint32_t)p;
 }
 
-inline PhiloxHead philox_head(const u32x4& c, uint32_t k0, uint32_t k1) {
+__host__ __device__ inline PhiloxHead philox_head(const u32x4& c, uint32_t k0, uint32_t k1) {
     PhiloxHead h;
     uint32_t hi1, lo1, hi0, lo0;
     mulhilo(0xCD9E8D57u, c.z, hi1, lo1);                 // round 1: x = hi1 ^ c.y ^ k0, y = lo1, both uniform

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
 template <bool kWet, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) production_step_kernel(StepArgs a) {
     const uint32_t p = blockIdx.x * BLOCK + threadIdx.x;
-    if (p < a.n) production_step<kWet, true>(a, p, p, a.alpha, a.counter, a.key0, a.key1);
+    if (p < a.n) production_step<kWet>(a, p, p, a.alpha, a.counter, 0u, 0u, a.head, true);
 }
 
 // Its block size and registers by the number of slots.  Small CTAs measure

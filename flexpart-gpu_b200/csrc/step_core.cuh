@@ -577,13 +577,13 @@ __device__ __forceinline__ float3 sample_production(const StepArgs& a, const Lev
 
 // particle_step for arguments in the production form: the same operations
 // with the settings known at compile time, the cell of the PBL and wet
-// lookups taken from the advected position, the counter's uniform rounds
-// from the host (`kHead`: a.head holds them and no block's counter carries)
-// and the turbulence without checks wherever the cell and the velocities
-// allow it.
-template <bool kWet, bool kHead>
+// lookups taken from the advected position, Philox from its uniform rounds
+// (`head` of the counter and key; `head_ok`: no block's counter carries) and
+// the turbulence without checks wherever the cell and the velocities allow.
+template <bool kWet>
 __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, uint32_t rng_index, float alpha,
-                                                u32x4 counter, uint32_t key0, uint32_t key1) {
+                                                u32x4 counter, uint32_t key0, uint32_t key1, const PhiloxHead& head,
+                                                bool head_ok) {
     if (!(a.flags[p] & FLAG_ACTIVE)) return;
     const Levels lv{a.heights, a.level_table, a.level_inv_w, a.nz, 1, LEVELS_TABLE};
     float tu = a.turb_u[p], tv = a.turb_v[p];
@@ -611,10 +611,10 @@ __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, u
     const uint32_t c = (uint32_t)cx * a.ny + (uint32_t)cy;
     const CellHanna cell = ld_cell_hanna(a.hcell + c);
     u32x4 b0, b1;
-    if constexpr (kHead) {
+    if (head_ok) {
         const uint32_t w = counter.x + 2u * rng_index;
-        b0 = philox_from_head(a.head, w);
-        b1 = philox_from_head(a.head, w + 1u);
+        b0 = philox_from_head(head, w);
+        b1 = philox_from_head(head, w + 1u);
     } else {
         b0 = philox4x32_10(counter_add(counter, rng_index * 2u), key0, key1);
         b1 = philox4x32_10(counter_add(counter, rng_index * 2u + 1u), key0, key1);
