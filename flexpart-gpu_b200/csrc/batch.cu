@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) batch_production_kernel(S
     const ScenDev& d = sc[w.x];
     const uint32_t local = w.y + threadIdx.x;
     if (local < d.released)
-        production_step<kWet>(a, d.offset + local, local, st->alpha, d.counter, d.key0, d.key1, d.head, d.head_ok != 0u);
+        production_step<kWet>(a, d.offset + local, local, st->alpha, d.counter, d.key0, d.key1, d.head,
+                              HeadKeys{d.head.k0, d.head.k1}, d.head_ok != 0u);
 }
 
 // The launch shapes the particle pass is compiled for; the tuner picks one,

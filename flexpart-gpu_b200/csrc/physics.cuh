@@ -98,7 +98,29 @@ __host__ __device__ inline PhiloxHead philox_head(const u32x4& c, uint32_t k0, u
     return h;
 }
 
-__device__ __forceinline__ u32x4 philox_from_head(const PhiloxHead& h, uint32_t cx) {
+// The keys of rounds 4 to 10, added up per round, or held by the launch.
+struct HeadKeys {
+    uint32_t k0, k1;
+    __device__ __forceinline__ uint32_t a(int r) const { return k0 + 0x9E3779B9u * (uint32_t)r; }
+    __device__ __forceinline__ uint32_t b(int r) const { return k1 + 0xBB67AE85u * (uint32_t)r; }
+};
+struct PhiloxKeys {
+    uint32_t k[14];
+    __device__ __forceinline__ uint32_t a(int r) const { return k[2 * r]; }
+    __device__ __forceinline__ uint32_t b(int r) const { return k[2 * r + 1]; }
+};
+
+inline PhiloxKeys philox_keys(const PhiloxHead& h) {
+    PhiloxKeys q;
+    for (uint32_t r = 0; r < 7u; ++r) {
+        q.k[2u * r] = h.k0 + 0x9E3779B9u * r;
+        q.k[2u * r + 1u] = h.k1 + 0xBB67AE85u * r;
+    }
+    return q;
+}
+
+template <class Keys>
+__device__ __forceinline__ u32x4 philox_from_head(const PhiloxHead& h, const Keys& keys, uint32_t cx) {
     const uint32_t z1 = __umulhi(0xD2511F53u, cx) ^ h.z1, w1 = 0xD2511F53u * cx;
     const uint32_t x2 = __umulhi(0xCD9E8D57u, z1) ^ h.x2, y2 = 0xCD9E8D57u * z1;
     const uint32_t z2 = w1 ^ h.z2;
@@ -107,14 +129,11 @@ __device__ __forceinline__ u32x4 philox_from_head(const PhiloxHead& h, uint32_t 
     c.y = 0xCD9E8D57u * z2;
     c.z = __umulhi(0xD2511F53u, x2) ^ h.z3;
     c.w = 0xD2511F53u * x2;
-    uint32_t k0 = h.k0, k1 = h.k1;
 #pragma unroll
-    for (int r = 3; r < 10; ++r) {
+    for (int r = 0; r < 7; ++r) {
         const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
         const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-        c = u32x4{hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0};
-        k0 += 0x9E3779B9u;
-        k1 += 0xBB67AE85u;
+        c = u32x4{hi1 ^ c.y ^ keys.a(r), lo1, hi0 ^ c.w ^ keys.b(r), lo0};
     }
     return c;
 }
@@ -150,12 +169,50 @@ __device__ __forceinline__ float2 box_muller(float u0, float u1) {
     return make_float2(radius * cs, radius * sn);
 }
 
-// Two Box-Muller pairs at once with the packed FP32 instructions of sm_100
-// (each lane the IEEE operation of bm_log and bm_sincos, in their order, so
-// the same bits).  a, b: the raw words of two pairs, (.x, .y) each.  The
-// uniform (v >> 8) 2^-24 never exceeds 1 - 2^-24, so box_muller's upper
-// clamps are the identity and only ln's lower one is kept; rintf of the
+// The correctly rounded square root of x in [2^-100, 2^100]: the hardware's
+// approximate 1/sqrt, then one Newton step on the root with the exact
+// residual x - g^2 from a fused multiply-add (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34,
+// 1990).  No range test and no branch: five instructions.  Equal to sqrtf for
+// every float of that range (checked exhaustively on a B200).
+__device__ __forceinline__ float rsqrt_of(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float plain_sqrt(float x) {
+    const float y = rsqrt_of(x);
+    const float g = x * y, h = 0.5f * y;
+    return fmaf(fmaf(-g, g, x), h, g);
+}
+
+// box_muller for the step's production form: the uniform (v >> 8) 2^-24
+// never exceeds 1 - 2^-24, so the upper clamps are the identity and only ln's
+// lower one is kept; -2 ln u lies in [1.1e-7, 175]; 2 pi 2^-24 is formed
+// before its product with the integer, which scales exactly; and rintf of the
 // quadrant is an addition of 1.5 2^23, whose low bits are the quadrant.
+__device__ __forceinline__ float2 box_muller_plain(uint32_t va, uint32_t vb) {
+    const float ru = fmaxf(u32_to_uniform01(va), 1.17549435e-38f);
+    const float radius = plain_sqrt(-2.0f * bm_log(ru));
+    const float th = (6.2831855f * (1.0f / 16777216.0f)) * (float)(vb >> 8);
+    const float qm = th * 0x1.45f306p-1f + 12582912.0f;
+    const float qf = qm - 12582912.0f;
+    const float t1 = fmaf(-qf, 0x1.921fb6p+0f, th);
+    const float x = fmaf(-qf, -0x1.ee59dap-50f, fmaf(-qf, -0x1.777a5cp-25f, t1));
+    const float x2 = x * x;
+    const float ps = fmaf(fmaf(-0x1.994068p-13f, x2, 0x1.110730p-7f), x2, -0x1.555546p-3f);
+    const float sn = fmaf(x * x2, ps, x);
+    const float pc = fmaf(fmaf(0x1.99e86ap-16f, x2, -0x1.6c0c28p-10f), x2, 0x1.55554ap-5f);
+    const float cs = 1.0f - fmaf(x2, 0.5f, -(x2 * x2) * pc);
+    const uint32_t q = __float_as_uint(qm);
+    const float s = (q & 1u) ? cs : sn, c = (q & 1u) ? sn : cs;
+    return make_float2(radius * (((q + 1u) & 2u) ? -c : c), radius * ((q & 2u) ? -s : s));
+}
+
+// Two pairs at once with the packed FP32 instructions of sm_100 (each lane
+// the IEEE operation of box_muller_plain, in its order, so the same bits).
+// a, b: the raw words of two pairs, (.x, .y) each.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float c) { return __ffma2_rn(a, b, f2(c)); }
 
@@ -179,10 +236,13 @@ __device__ __forceinline__ void box_muller2(uint2 a, uint2 b, float2& na, float2
     const float2 r = __ffma2_rn(ff, q, f);
     const float2 fe = make_float2((float)ea, (float)eb);
     const float2 lg = __ffma2_rn(fe, f2(0x1.62e400p-1f), __ffma2_rn(fe, f2(0x1.7f7d1cp-20f), r));
-    const float2 lr = __fmul2_rn(f2(-2.0f), lg);
-    const float ra = sqrtf(lr.x), rb = sqrtf(lr.y);
+    // plain_sqrt of -2 ln u
+    const float2 lr = __fmul2_rn(f2(-2.0f), lg), nlr = __fmul2_rn(f2(2.0f), lg);
+    const float2 y = make_float2(rsqrt_of(lr.x), rsqrt_of(lr.y));
+    const float2 g = __fmul2_rn(lr, y), nh = __fmul2_rn(f2(-0.5f), y);
+    const float2 rad = __ffma2_rn(__ffma2_rn(g, g, nlr), nh, g);
     // bm_sincos
-    const float2 th = __fmul2_rn(f2(6.2831855f), make_float2(u32_to_uniform01(a.y), u32_to_uniform01(b.y)));
+    const float2 th = __fmul2_rn(f2(6.2831855f * (1.0f / 16777216.0f)), make_float2((float)(a.y >> 8), (float)(b.y >> 8)));
     const float2 qm = __fadd2_rn(__fmul2_rn(th, f2(0x1.45f306p-1f)), f2(12582912.0f));
     const float2 qf = __fadd2_rn(qm, f2(-12582912.0f));
     const float2 nq = __fmul2_rn(qf, f2(-1.0f));
@@ -198,8 +258,8 @@ __device__ __forceinline__ void box_muller2(uint2 a, uint2 b, float2& na, float2
     const uint32_t qa = __float_as_uint(qm.x), qb = __float_as_uint(qm.y);
     const float sa = (qa & 1u) ? cs.x : sn.x, ca = (qa & 1u) ? sn.x : cs.x;
     const float sb = (qb & 1u) ? cs.y : sn.y, cb = (qb & 1u) ? sn.y : cs.y;
-    na = make_float2(ra * (((qa + 1u) & 2u) ? -ca : ca), ra * ((qa & 2u) ? -sa : sa));
-    nb = make_float2(rb * (((qb + 1u) & 2u) ? -cb : cb), rb * ((qb & 2u) ? -sb : sb));
+    na = make_float2(rad.x * (((qa + 1u) & 2u) ? -ca : ca), rad.x * ((qa & 2u) ? -sa : sa));
+    nb = make_float2(rad.y * (((qb + 1u) & 2u) ? -cb : cb), rad.y * ((qb & 2u) ? -sb : sb));
 }
 
 // ---- scalar helpers of the templated physics --------------------------------
@@ -573,9 +633,9 @@ __device__ __forceinline__ void plain_hanna(const CellHanna& c, const PlainRates
         const float cz = xcbrt(zeta);
         const float z23 = cz * cz;
         const float sigw_sq = c.k2 * (1.0f - 0.9f * zeta) * z23 + (1.8f - 1.4f * zeta) * c.ust * c.ust;
-        sigw = sqrtf(sigw_sq) + 1.0e-2f;
+        sigw = plain_sqrt(sigw_sq) + 1.0e-2f;
         const float rs = rcp_of(sigw);
-        const float zm13 = rcp_of(zeta >= 1.0e-3f ? cz : pow_third(1.0e-3f));
+        const float zm13 = rcp_of(zeta >= 1.0e-3f ? cz : 0.1f);      // cbrtf(1e-3) is 0.1
         dsigwdz = 0.5f * rs * r.h * (c.k3 + c.k4 * (0.8f * zm13 - 1.8f * z23));
         if (z < fabsf(c.ol)) tlw = 0.1f * z * rcp_of(sigw * (0.55f - 0.38f * fabsf(z * r.other)));
         else if (zeta < 0.1f) tlw = 0.59f * z * rs;
@@ -610,17 +670,18 @@ __device__ __forceinline__ void plain_hanna(const CellHanna& c, const PlainRates
     tlw = fmaxf(tlw, 30.0f);
 }
 
-// The decay and noise factors of the Ornstein-Uhlenbeck update over dt at
-// time scale tl (langevin_h_t, langevin_v_t): exp(-r) <= 0.61 for r >= 0.5.
+// The decay and noise factors of the Ornstein-Uhlenbeck update over dt in
+// [1e-3, 1e6] at time scale tl in [10, 1e8] (langevin_h_t, langevin_v_t):
+// exp(-r) <= 0.61 for r >= 0.5.
 __device__ __forceinline__ void plain_factors(float dt, float tl, float& decay, float& noise, bool& linear) {
     const float ratio = sdiv(dt, tl);
     linear = ratio < 0.5f;
     if (linear) {
         decay = 1.0f - ratio;
-        noise = sqrtf(2.0f * ratio);
+        noise = plain_sqrt(2.0f * ratio);
     } else {
         decay = xexp(-ratio);
-        noise = sqrtf(1.0f - decay * decay);
+        noise = plain_sqrt(1.0f - decay * decay);
     }
 }
 

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
 template <bool kWet, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) production_step_kernel(StepArgs a) {
     const uint32_t p = blockIdx.x * BLOCK + threadIdx.x;
-    if (p < a.n) production_step<kWet>(a, p, p, a.alpha, a.counter, 0u, 0u, a.head, true);
+    if (p < a.n) production_step<kWet>(a, p, p, a.alpha, a.counter, 0u, 0u, a.head, a.keys, true);
 }
 
 // Its block size and registers by the number of slots.  Small CTAs measure
@@ -643,6 +643,7 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     const bool no_carry = (uint64_t)prm->counter[0] + 2u * (uint64_t)n <= (1ull << 32);
     if (ctx->step_shape == 0 && no_carry && production_form(a)) {
         a.head = philox_head(a.counter, a.key0, a.key1);
+        a.keys = philox_keys(a.head);
         const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
         (wet ? ps.wet : ps.dry)<<<blocks_for(n, ps.block), ps.block, 0, s>>>(a);
     } else {

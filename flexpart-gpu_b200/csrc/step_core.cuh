@@ -53,7 +53,8 @@ struct StepArgs {
     const float2* wet_cells;
     uint32_t wnx, wny;
     float* wet_prob;
-    PhiloxHead head;                     // of the launch's counter and key, for the production form
+    PhiloxHead head;                     // of the launch's counter and key, and its round keys,
+    PhiloxKeys keys;                     // for the production form
 };
 
 // The production form of the step (production_step below): the forward
@@ -77,7 +78,7 @@ inline bool production_form(const StepArgs& a) {
     if (wet && (a.wet_mode != FPG_FORCING_PER_CELL || a.wet_prob || a.wnx != a.nx || a.wny != a.ny)) return false;
     if (!a.has_heights || a.level_mode != LEVELS_TABLE || a.pnx != a.nx || a.pny != a.ny) return false;
     if ((uint64_t)a.nx * a.ny * a.nz >= (1ull << 27)) return false;
-    return a.tdt > 0.0f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f && a.rho <= 1.0e3f && a.zmin >= 0.0f && a.zmin < 1.0f;
+    return a.tdt >= 1.0e-3f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f && a.rho <= 1.0e3f && a.zmin >= 0.0f && a.zmin < 1.0f;
 }
 
 // The search a met's heights allow (host side).
@@ -580,10 +581,10 @@ __device__ __forceinline__ float3 sample_production(const StepArgs& a, const Lev
 // lookups taken from the advected position, Philox from its uniform rounds
 // (`head` of the counter and key; `head_ok`: no block's counter carries) and
 // the turbulence without checks wherever the cell and the velocities allow.
-template <bool kWet>
+template <bool kWet, class Keys>
 __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, uint32_t rng_index, float alpha,
                                                 u32x4 counter, uint32_t key0, uint32_t key1, const PhiloxHead& head,
-                                                bool head_ok) {
+                                                const Keys& keys, bool head_ok) {
     if (!(a.flags[p] & FLAG_ACTIVE)) return;
     const Levels lv{a.heights, a.level_table, a.level_inv_w, a.nz, 1, LEVELS_TABLE};
     float tu = a.turb_u[p], tv = a.turb_v[p];
@@ -613,15 +614,15 @@ __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, u
     u32x4 b0, b1;
     if (head_ok) {
         const uint32_t w = counter.x + 2u * rng_index;
-        b0 = philox_from_head(head, w);
-        b1 = philox_from_head(head, w + 1u);
+        b0 = philox_from_head(head, keys, w);
+        b1 = philox_from_head(head, keys, w + 1u);
     } else {
         b0 = philox4x32_10(counter_add(counter, rng_index * 2u), key0, key1);
         b1 = philox4x32_10(counter_add(counter, rng_index * 2u + 1u), key0, key1);
     }
     float2 e_uv, e_w01;
     box_muller2(make_uint2(b0.x, b0.y), make_uint2(b0.z, b0.w), e_uv, e_w01);
-    const float2 e_w23 = box_muller(u32_to_uniform01(b1.x), u32_to_uniform01(b1.y));
+    const float2 e_w23 = box_muller_plain(b1.x, b1.y);
     float tw = a.turb_w[p];
     const int32_t cbt_in = a.cbt[p];
     int32_t cbt = cbt_in;
