@@ -243,7 +243,8 @@ __device__ __forceinline__ void box_muller2(uint2 a, uint2 b, float2& na, float2
     const float2 rad = __ffma2_rn(__ffma2_rn(g, g, nlr), nh, g);
     // bm_sincos
     const float2 th = __fmul2_rn(f2(6.2831855f * (1.0f / 16777216.0f)), make_float2((float)(a.y >> 8), (float)(b.y >> 8)));
-    const float2 qm = __fadd2_rn(__fmul2_rn(th, f2(0x1.45f306p-1f)), f2(12582912.0f));
+    // scalar: the compiler contracts a packed product and sum, which would round the quadrant's ties another way
+    const float2 qm = make_float2(th.x * 0x1.45f306p-1f + 12582912.0f, th.y * 0x1.45f306p-1f + 12582912.0f);
     const float2 qf = __fadd2_rn(qm, f2(-12582912.0f));
     const float2 nq = __fmul2_rn(qf, f2(-1.0f));
     const float2 t1 = __ffma2_rn(nq, f2(0x1.921fb6p+0f), th);

@@ -96,6 +96,21 @@ def test_counters_at_the_edge_of_a_carry(world, counter):
     _same(_run(world, rec, PRODUCTION, 2, **kw), _run(world, rec, GENERAL, 2, **kw))
 
 
+# Philox blocks under key (42, 0) whose word (1 or 3: the angle of a pair) lies
+# exactly between two quadrants, where the rounding of the quadrant is a tie
+TIES = [(1, 34705893), (1, 7291534), (1, 49559575), (1, 15432739), (3, 16559396), (3, 34779132), (3, 15007975),
+        (3, 1106156)]
+
+
+@pytest.mark.parametrize("word,block", TIES)
+def test_box_muller_at_quadrant_ties(world, word, block):
+    rec = _records(world[1], 33)
+    rec["flags"] = 1
+    for first in (block - 16, block - 17):          # slot 8's first block, and its second
+        kw = dict(counter=(first, 0, 0, 0), key=(42, 0))
+        _same(_run(world, rec, PRODUCTION, 1, **kw), _run(world, rec, GENERAL, 1, **kw))
+
+
 def test_largest_shape(world):
     rec = np.resize(_records(world[1], 50_021), 4_000_001)
     _same(_run(world, rec, PRODUCTION, 1, wet_mode=3), _run(world, rec, GENERAL, 1, wet_mode=3))
