@@ -29,7 +29,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -160,15 +159,6 @@ struct TapeRec {
         if (output) { t.f[T_X2][p] = x; t.f[T_Y2][p] = y; t.f[T_Z2][p] = z; t.f[T_M2][p] = m; }
     }
 };
-
-// Post-advance clock and scenario state of the step, kept per tape slice.
-__global__ void inverse_snapshot_kernel(const BatchState* st, const ScenDev* __restrict__ sc, uint32_t n_scen,
-                                        uint32_t slices, BatchState* st_all, ScenDev* sc_all) {
-    const uint32_t j = st->step % slices;
-    if (threadIdx.x == 0 && blockIdx.x == 0) st_all[j] = *st;
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_scen; s += gridDim.x * blockDim.x)
-        sc_all[(size_t)j * n_scen + s] = sc[s];
-}
 
 // `live` (the recompute of a checkpoint window; NULL in the forward): a slot
 // whose last receptor hit came before this step has a zero adjoint from this
@@ -532,6 +522,43 @@ constexpr int kCkptFields[] = {FPG_FIELD_POS_X, FPG_FIELD_POS_Y,  FPG_FIELD_POS_
                                FPG_FIELD_TURB_V, FPG_FIELD_TURB_W, FPG_FIELD_CBT};
 constexpr int kNumCkptFields = sizeof(kCkptFields) / sizeof(kCkptFields[0]);
 
+// A checkpoint saved or restored in one launch: a field per grid row and the
+// clock and scenario state in the last one (13 copies took 23 us and their
+// gaps at 160 k slots, where the bytes take 2 us).  HBM-bound above that, 88
+// B a slot.
+struct CheckpointArgs {
+    uint4* field[kNumCkptFields];
+    uint4* saved[kNumCkptFields];
+    size_t quads;
+    BatchState* st;
+    BatchState* st_saved;
+    ScenDev* sc;
+    ScenDev* sc_saved;
+    uint32_t n_scen;
+    int restore;
+};
+
+__global__ void __launch_bounds__(256) inverse_checkpoint_kernel(CheckpointArgs a) {
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    if (blockIdx.y == kNumCkptFields) {
+        for (size_t s = first; s < a.n_scen; s += step) {
+            if (a.restore) a.sc[s] = a.sc_saved[s]; else a.sc_saved[s] = a.sc[s];
+        }
+        if (first == 0) {
+            if (a.restore) {
+                *a.st = *a.st_saved;
+                a.st->changed = 1;                   // the packed bracket is another step's: repack it
+            } else {
+                *a.st_saved = *a.st;
+            }
+        }
+        return;
+    }
+    const uint4* __restrict__ from = a.restore ? a.saved[blockIdx.y] : a.field[blockIdx.y];
+    uint4* __restrict__ to = a.restore ? a.field[blockIdx.y] : a.saved[blockIdx.y];
+    for (size_t i = first; i < a.quads; i += step) to[i] = from[i];
+}
+
 struct InverseData {
     fpg_inverse_config cfg{};
     uint32_t n_instances = 1;
@@ -568,10 +595,11 @@ struct InverseData {
     bool forward_done = false;
     uint64_t bytes = 0;
     uint32_t grid_adj = 0;               // the reverse's persistent grid: SMs x resident CTAs
-    // one taped step (pre, snapshot, tape pass, [sampling], end), captured
-    cudaGraph_t tape_graph[2] = {nullptr, nullptr};
-    cudaGraphExec_t tape_exec[2] = {nullptr, nullptr};
-    uint64_t tape_launches[2] = {0, 0};
+    // one taped step (pre, tape pass, [sampling], turn), captured: the
+    // recompute's (0), the forward's (1) and the forward's sampling steps (2)
+    cudaGraph_t tape_graph[3] = {nullptr, nullptr, nullptr};
+    cudaGraphExec_t tape_exec[3] = {nullptr, nullptr, nullptr};
+    uint64_t tape_launches[3] = {0, 0, 0};
 
     Receptors receptors_args(uint32_t nx, uint32_t ny) const {
         Receptors r;
@@ -586,6 +614,12 @@ struct InverseData {
         return r;
     }
 };
+
+bool inverse_sample_step(const fpg_batch* b, uint64_t step) {
+    if (!b->inv) return false;
+    const uint32_t every = b->inv->cfg.sample_every_steps;
+    return every != 0 && (step + 1) % every == 0;
+}
 
 void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s) {
     InverseData* inv = b->inv;
@@ -612,37 +646,40 @@ static LamArrays lam_arrays(fpg_inverse* v) {
     return l;
 }
 
+enum { TAPE_RECOMPUTE = 0, TAPE_FORWARD = 1, TAPE_FORWARD_SAMPLE = 2 };
+
 // One taped step: the forward step with the tape pass in place of the plain
-// particle pass; `sample` adds the receptor sampling (forward runs).
-// The recompute (sample == false) steps only the slots whose adjoint is still
-// non-zero (live).
-static void enqueue_taped_step(fpg_inverse* v, bool sample, cudaStream_t s) {
+// particle pass and, on the forward's sampling steps, the receptor sampling.
+// The recompute steps only the slots whose adjoint is still non-zero (live).
+static void enqueue_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
     fpg_batch* b = v->b;
     InverseData& d = v->d;
-    enqueue_pre(b, s);
-    inverse_snapshot_kernel<<<1, 256, 0, s>>>(b->st, b->sc, (uint32_t)b->scen.size(), d.slices, d.st_all, d.sc_all);
+    enqueue_pre(b, s, false, d.st_all, d.sc_all, d.slices);
     inverse_tape_kernel<<<std::max(d.n_items, 1u), 256, 0, s>>>(make_step_args(b), b->st, b->sc, d.items, d.n_items,
                                                                 tape_base(v), d.cfg.sample_every_steps,
-                                                                sample ? nullptr : d.last_hit);
-    b->ctx->count(2);
-    if (sample) enqueue_inverse_sample(b, s);
-    enqueue_end(b, s);
+                                                                kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
+    b->ctx->count(1);
+    if (kind == TAPE_FORWARD_SAMPLE) enqueue_inverse_sample(b, s);
+    enqueue_turn(b, s, true);
 }
 
-static fpg_status ensure_tape_graph(fpg_inverse* v, int sample) {
+static fpg_status launch_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
     InverseData& d = v->d;
-    if (d.tape_exec[sample]) return FPG_OK;
-    cudaStream_t s = v->b->ctx->stream;
-    FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const uint64_t before = v->b->ctx->launches.load();
-    enqueue_taped_step(v, sample != 0, s);
-    d.tape_launches[sample] = v->b->ctx->launches.load() - before;
-    v->b->ctx->launches.fetch_sub(d.tape_launches[sample]);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(s, &g);
-    if (e != cudaSuccess) return cuda_status(e);
-    d.tape_graph[sample] = g;
-    FPG_CUDA(cudaGraphInstantiate(&d.tape_exec[sample], g, 0));
+    fpg_ctx* ctx = v->b->ctx;
+    if (!d.tape_exec[kind]) {
+        FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        const uint64_t before = ctx->launches.load();
+        enqueue_taped_step(v, kind, s);
+        d.tape_launches[kind] = ctx->launches.load() - before;
+        ctx->launches.fetch_sub(d.tape_launches[kind]);
+        cudaGraph_t g = nullptr;
+        cudaError_t e = cudaStreamEndCapture(s, &g);
+        if (e != cudaSuccess) return cuda_status(e);
+        d.tape_graph[kind] = g;
+        FPG_CUDA(cudaGraphInstantiate(&d.tape_exec[kind], g, 0));
+    }
+    FPG_CUDA(cudaGraphLaunch(d.tape_exec[kind], s));
+    ctx->count(d.tape_launches[kind]);
     return FPG_OK;
 }
 
@@ -657,38 +694,25 @@ static fpg_status rebuild_ring(fpg_inverse* v) {
     return FPG_OK;
 }
 
-static cudaError_t save_checkpoint(fpg_inverse* v, uint32_t c) {
+static cudaError_t enqueue_checkpoint(fpg_inverse* v, uint32_t c, bool restore) {
     fpg_batch* b = v->b;
-    cudaStream_t s = b->ctx->stream;
-    const size_t cap = b->capacity;
-    cudaError_t e = cudaSuccess;
-    for (int f = 0; f < kNumCkptFields && e == cudaSuccess; ++f)
-        e = cudaMemcpyAsync(v->d.ckpt + ((size_t)c * kNumCkptFields + f) * cap, b->pop->field[kCkptFields[f]],
-                            cap * 4, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(v->d.ckpt_st + c, b->st, sizeof(BatchState), cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(v->d.ckpt_sc + (size_t)c * b->scen.size(), b->sc, b->scen.size() * sizeof(ScenDev),
-                            cudaMemcpyDeviceToDevice, s);
-    return e;
-}
-
-static cudaError_t restore_checkpoint(fpg_inverse* v, uint32_t c) {
-    fpg_batch* b = v->b;
-    cudaStream_t s = b->ctx->stream;
-    const size_t cap = b->capacity;
-    cudaError_t e = cudaSuccess;
-    for (int f = 0; f < kNumCkptFields && e == cudaSuccess; ++f)
-        e = cudaMemcpyAsync(b->pop->field[kCkptFields[f]], v->d.ckpt + ((size_t)c * kNumCkptFields + f) * cap,
-                            cap * 4, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b->st, v->d.ckpt_st + c, sizeof(BatchState), cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b->sc, v->d.ckpt_sc + (size_t)c * b->scen.size(), b->scen.size() * sizeof(ScenDev),
-                            cudaMemcpyDeviceToDevice, s);
-    // the device bracket and wet fields hold whatever was packed last: make
-    // the next step repack them
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(reinterpret_cast<char*>(b->st) + offsetof(BatchState, have_bracket), 0, sizeof(int32_t), s);
-    return e;
+    CheckpointArgs a;
+    for (int f = 0; f < kNumCkptFields; ++f) {
+        a.field[f] = static_cast<uint4*>(b->pop->field[kCkptFields[f]]);
+        a.saved[f] = reinterpret_cast<uint4*>(v->d.ckpt + ((size_t)c * kNumCkptFields + f) * b->capacity);
+    }
+    a.quads = b->capacity / 4;                       // the capacity is a multiple of a tile
+    a.st = b->st;
+    a.st_saved = v->d.ckpt_st + c;
+    a.sc = b->sc;
+    a.sc_saved = v->d.ckpt_sc + (size_t)c * b->scen.size();
+    a.n_scen = (uint32_t)b->scen.size();
+    a.restore = restore ? 1 : 0;
+    const size_t per = 4 * 256;
+    const unsigned x = (unsigned)std::min<size_t>((a.quads + per - 1) / per, (size_t)b->ctx->sm_count * 8);
+    inverse_checkpoint_kernel<<<dim3(std::max(x, 1u), kNumCkptFields + 1), 256, 0, b->ctx->stream>>>(a);
+    b->ctx->count(1);
+    return cudaGetLastError();
 }
 
 extern "C" fpg_status fpg_inverse_destroy(fpg_inverse* v) {
@@ -698,7 +722,7 @@ extern "C" fpg_status fpg_inverse_destroy(fpg_inverse* v) {
         v->b->inv = nullptr;
     }
     InverseData& d = v->d;
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 3; ++k) {
         if (d.tape_exec[k]) cudaGraphExecDestroy(d.tape_exec[k]);
         if (d.tape_graph[k]) cudaGraphDestroy(d.tape_graph[k]);
     }
@@ -860,27 +884,17 @@ extern "C" fpg_status fpg_inverse_forward(fpg_inverse* v, double* simulated) {
     if (st != FPG_OK) return st;
     FPG_CUDA(cudaMemsetAsync(d.sim, 0, std::max<size_t>(d.receptors.size(), 1) * 8, s));
     FPG_CUDA(cudaMemsetAsync(d.last_hit, 0, v->b->capacity * 4, s));
-    if (d.tape_in_forward) {
-        if ((st = ensure_tape_graph(v, 1)) != FPG_OK) return st;
-        for (uint64_t k = 0; k < b->total_steps; ++k) {
-            FPG_CUDA(cudaGraphLaunch(d.tape_exec[1], s));
-            b->ctx->count(d.tape_launches[1]);
+    // steps from here on are taped in the forward
+    const uint64_t K = d.window;
+    const uint64_t k_tail = d.tape_in_forward ? 0 : (uint64_t)(d.n_windows - d.tail_windows) * K;
+    for (uint64_t k = 0; k < b->total_steps; ++k) {
+        if (k < k_tail) {
+            if (k % K == 0) FPG_CUDA(enqueue_checkpoint(v, (uint32_t)(k / K), false));
+            st = launch_step_graph(b, k, s);
+        } else {
+            st = launch_taped_step(v, inverse_sample_step(b, k) ? TAPE_FORWARD_SAMPLE : TAPE_FORWARD, s);
         }
-    } else {
-        if ((st = ensure_graph(b)) != FPG_OK) return st;
-        if (d.tail_windows && (st = ensure_tape_graph(v, 1)) != FPG_OK) return st;
-        const uint32_t K = d.window;
-        const uint64_t k_tail = (uint64_t)(d.n_windows - d.tail_windows) * K;
-        for (uint64_t k = 0; k < b->total_steps; ++k) {
-            if (k < k_tail) {
-                if (k % K == 0) FPG_CUDA(save_checkpoint(v, (uint32_t)(k / K)));
-                FPG_CUDA(cudaGraphLaunch(b->exec, s));
-                b->ctx->count(b->graph_launches);
-            } else {                         // a tail window: record its tape now
-                FPG_CUDA(cudaGraphLaunch(d.tape_exec[1], s));
-                b->ctx->count(d.tape_launches[1]);
-            }
-        }
+        if (st != FPG_OK) return st;
     }
     b->steps_done = b->total_steps;
     // the step kernels left the bracket of the last step packed
@@ -919,17 +933,15 @@ extern "C" fpg_status fpg_inverse_backward(fpg_inverse* v, const double* d_sim, 
     const int64_t windows = d.n_windows;
     // windows below this one are recomputed from their checkpoints
     const int64_t first_taped = d.tape_in_forward ? 0 : (int64_t)(d.n_windows - d.tail_windows);
-    fpg_status st = FPG_OK;
-    if (first_taped > 0 && (st = ensure_tape_graph(v, 0)) != FPG_OK) return st;
     for (int64_t w = windows - 1; w >= 0; --w) {
         const uint64_t k0 = (uint64_t)w * K, k1 = std::min<uint64_t>(k0 + K, n);
         if (w < first_taped) {
             // taped recompute of the window from its checkpoint; it leaves the
             // bracket of its last step packed
-            FPG_CUDA(restore_checkpoint(v, (uint32_t)w));
+            FPG_CUDA(enqueue_checkpoint(v, (uint32_t)w, true));
             for (uint64_t k = k0; k < k1; ++k) {
-                FPG_CUDA(cudaGraphLaunch(d.tape_exec[0], s));
-                b->ctx->count(d.tape_launches[0]);
+                const fpg_status st = launch_taped_step(v, TAPE_RECOMPUTE, s);
+                if (st != FPG_OK) return st;
             }
             d.packed_ta = step_bracket_start(b, k1 - 1);
         }

@@ -10,17 +10,18 @@
 // [offset_s, offset_s + capacity_s) of one structure-of-arrays population;
 // tile t (256 slots) belongs to exactly one scenario.
 //
-// One step is a fixed kernel sequence that reads its per-step values
+// One step is a short kernel sequence that reads its per-step values
 // (clock, alpha, bracket, release ranges, counters) from device memory, so
-// it is captured once into a CUDA graph and replayed:
-//   batch_advance   clock -> bracket + alpha; per-scenario release ranges
-//   batch_pack      repack the bracket from the ring when it changed
-//   batch_pbl       surface lerp + PBL per cell (+ wet forcing on a change)
-//   batch_release   new particles of every scenario (lattice in f64)
-//   batch_step      persistent: CTAs pull 256-slot tiles from a work queue
-//                   and run the fused per-particle step (step_core.cuh)
-//   batch_grid_*    per-scenario grids at output steps
-//   batch_end       counters += capacity * blocks; clock += dt
+// it is captured into CUDA graphs (one for steps that end with grids or
+// receptor samples, one for the others) and replayed:
+//   batch_pre       bracket from the ring when it changed, PBL (and wet
+//                   forcing) per cell, new particles of every scenario
+//                   (lattice in f64), grids cleared before an output step
+//   batch_step      the fused per-particle step (step_core.cuh): one CTA per
+//                   work item, or persistent CTAs that pull items
+//   batch_grid      per-scenario grids at output steps
+//   batch_turn      counters += capacity * blocks; clock += dt; then the
+//                   bracket, alpha and release ranges of the next step
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -43,25 +44,33 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a);
 namespace {
 
 
-__global__ void batch_advance_kernel(BatchState* st, ScenDev* sc, BatchConst c) {
+// The state of the coming step from the clock: bracket and alpha, and per
+// scenario the release range and the Philox head.
+__device__ __forceinline__ void advance_clock(BatchState* st, const BatchConst& c) {
     const int64_t t = st->t;
-    if (threadIdx.x == 0) {
-        // bracket holding t; at a frame time stay in the bracket ending there
-        int64_t k = (t - c.start) / c.frame_seconds;
-        if (t - c.start == k * c.frame_seconds && k > 0) k -= 1;
-        const int32_t fa = (int32_t)(k % c.n_frames), fb = (int32_t)((k + 1) % c.n_frames);
-        const int64_t ta = c.start + k * c.frame_seconds;
-        st->changed = !st->have_bracket || fa != st->fa || fb != st->fb || ta != st->ta;
-        st->fa = fa;
-        st->fb = fb;
-        st->ta = ta;
-        st->have_bracket = 1;
-        // interpolation_alpha (timeloop.rs:2117-2119)
-        st->alpha = (float)((double)(t - ta) / (double)c.frame_seconds);
-        st->work = 0;
-    }
+    // bracket holding t; at a frame time stay in the bracket ending there
+    int64_t k = (t - c.start) / c.frame_seconds;
+    if (t - c.start == k * c.frame_seconds && k > 0) k -= 1;
+    const int32_t fa = (int32_t)(k % c.n_frames), fb = (int32_t)((k + 1) % c.n_frames);
+    const int64_t ta = c.start + k * c.frame_seconds;
+    st->changed = !st->have_bracket || fa != st->fa || fb != st->fb || ta != st->ta;
+    st->fa = fa;
+    st->fb = fb;
+    st->ta = ta;
+    st->have_bracket = 1;
+    // interpolation_alpha (timeloop.rs:2117-2119)
+    st->alpha = (float)((double)(t - ta) / (double)c.frame_seconds);
+    st->work = 0;
+}
+
+// Ends a step (`end`: counters and clock move on) and prepares the next one,
+// so that a step is one launch before its particle pass and one after it.
+// Runs once without `end` when the state is (re)set.
+__global__ void __launch_bounds__(256) batch_turn_kernel(BatchState* st, ScenDev* sc, BatchConst c, int end) {
+    const int64_t t = st->t + (end ? c.dt : 0);
     for (uint32_t s = threadIdx.x; s < c.n_scen; s += blockDim.x) {
         ScenDev& d = sc[s];
+        if (end) d.counter = counter_add64(d.counter, (uint64_t)d.capacity * c.bpp);
         const uint32_t lo = d.released;
         uint32_t hi = target_emitted(d.start, d.end, d.count, t, lo);
         if (hi < lo) hi = lo;
@@ -71,39 +80,22 @@ __global__ void batch_advance_kernel(BatchState* st, ScenDev* sc, BatchConst c) 
         d.head = philox_head(d.counter, d.key0, d.key1);
         d.head_ok = (uint64_t)d.counter.x + 2u * (uint64_t)d.capacity <= (1ull << 32);
     }
-}
-
-__global__ void __launch_bounds__(256) batch_pack_kernel(const BatchState* st, const float4* __restrict__ ring,
-                                                         uint32_t nodes, float4* __restrict__ bracket) {
-    if (!st->changed) return;
-    const float4* f0 = ring + (size_t)st->fa * nodes;
-    const float4* f1 = ring + (size_t)st->fb * nodes;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < nodes; n += gridDim.x * blockDim.x) {
-        st_node(bracket, n, f0[n], f1[n]);
+    __syncthreads();                                    // every thread has read the old clock
+    if (threadIdx.x == 0) {
+        st->t = t;
+        st->step += end ? 1u : 0u;
+        advance_clock(st, c);
     }
-}
-
-__global__ void __launch_bounds__(256) batch_pbl_kernel(const BatchState* st, const fpg_surface_cell* __restrict__ sring,
-                                                        const float* __restrict__ precip, fpg_pbl_options o,
-                                                        uint32_t ncell, float* f0, float* f1, float* f2, float* f3,
-                                                        float* f4, float* f5, float* f6, float4* packed,
-                                                        CellHanna* hanna, int wet_on,
-                                                        float wa, float wb, float2* wet) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    pbl_cell(sring + (size_t)st->fa * ncell, sring + (size_t)st->fb * ncell, st->alpha, o, c, f0, f1, f2, f3, f4, f5,
-             f6, packed, hanna);
-    if (wet_on && st->changed) wet[c] = wet_cell_forcing(precip[(size_t)st->fa * ncell + c], 0.0f, 1.0f, wa, wb);
 }
 
 // ReleaseManager::inject_for_time + geo_to_grid + to_relative
 // (release/mod.rs:103-146, coords/mod.rs:92-114,169-178) on the device, in
-// the same f64 arithmetic as the host release manager.
-__global__ void __launch_bounds__(256) batch_release_kernel(BatchState* st, const ScenDev* __restrict__ sc,
-                                                            BatchConst c, PopFields F) {
-    const ScenDev& d = sc[blockIdx.y];
+// the same f64 arithmetic as the host release manager.  CTA `part` of `parts`
+// of one scenario.
+__device__ __forceinline__ void release_particles(BatchState* st, const ScenDev& d, const BatchConst& c,
+                                                  const PopFields& F, uint32_t part, uint32_t parts) {
     const int32_t now = (int32_t)st->t;
-    for (uint32_t k = d.rel_lo + blockIdx.x * blockDim.x + threadIdx.x; k < d.rel_hi; k += gridDim.x * blockDim.x) {
+    for (uint32_t k = d.rel_lo + part * blockDim.x + threadIdx.x; k < d.rel_hi; k += parts * blockDim.x) {
         const uint64_t idx = k;
         const uint64_t ix = idx % d.lat_nx, iy = (idx / d.lat_nx) % d.lat_nx, iz = (idx / d.lat_nxy) % d.lat_nz;
         const double fx = ((double)ix + 0.5) / (double)d.lat_nx;
@@ -131,6 +123,76 @@ __global__ void __launch_bounds__(256) batch_release_kernel(BatchState* st, cons
         F.f[FPG_FIELD_TIME_MEM][p] = (uint32_t)now;
         // every other field of a fresh slot is zero (the population starts zeroed)
     }
+}
+
+// Everything a step does before its particle pass, one launch: the CTAs are
+// shared out over independent parts that read the state the turn kernel left.
+// A step of a small ensemble is bound by its launches (separate advance,
+// pack, PBL, release and end kernels took 11 us of device time and five
+// launches a step beside an 11 us pass at 160 k particles).
+struct PreArgs {
+    const float4* ring;                  // pack the bracket when it changed
+    float4* bracket;
+    uint32_t nodes, pack_ctas;
+    const fpg_surface_cell* sring;       // PBL cells, and the wet cells when the bracket changed
+    const float* precip;
+    fpg_pbl_options pbl;
+    uint32_t ncell, pbl_ctas;
+    float* field[7];
+    float4* packed;
+    CellHanna* hanna;
+    int wet_on;
+    float wet_a, wet_b;
+    float2* wet;
+    uint32_t parts;                      // release CTAs per scenario
+    PopFields F;
+    BatchState* st_out;                  // inversion: the step's state kept per tape slice (NULL: not kept)
+    ScenDev* sc_out;
+    uint32_t slices;
+    uint32_t* clear[2];                  // the output grids, cleared on output steps
+    size_t clear_n;
+    uint32_t clear_ctas;
+};
+constexpr uint32_t kPreThreads = 128;
+
+__global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, const ScenDev* __restrict__ sc, BatchConst c,
+                                                                PreArgs a) {
+    uint32_t b = blockIdx.x;
+    if (b < a.pbl_ctas) {
+        const uint32_t i = b * kPreThreads + threadIdx.x;
+        if (i >= a.ncell) return;
+        pbl_cell(a.sring + (size_t)st->fa * a.ncell, a.sring + (size_t)st->fb * a.ncell, st->alpha, a.pbl, i, a.field[0],
+                 a.field[1], a.field[2], a.field[3], a.field[4], a.field[5], a.field[6], a.packed, a.hanna);
+        if (a.wet_on && st->changed)
+            a.wet[i] = wet_cell_forcing(a.precip[(size_t)st->fa * a.ncell + i], 0.0f, 1.0f, a.wet_a, a.wet_b);
+        return;
+    }
+    b -= a.pbl_ctas;
+    if (b < c.n_scen * a.parts) {
+        release_particles(st, sc[b / a.parts], c, a.F, b % a.parts, a.parts);
+        return;
+    }
+    b -= c.n_scen * a.parts;
+    if (b < a.pack_ctas) {
+        if (!st->changed) return;
+        const float4* f0 = a.ring + (size_t)st->fa * a.nodes;
+        const float4* f1 = a.ring + (size_t)st->fb * a.nodes;
+        for (uint32_t n = b * kPreThreads + threadIdx.x; n < a.nodes; n += a.pack_ctas * kPreThreads)
+            st_node(a.bracket, n, f0[n], f1[n]);
+        return;
+    }
+    b -= a.pack_ctas;
+    if (b < a.clear_ctas) {
+        for (size_t i = (size_t)b * kPreThreads + threadIdx.x; i < a.clear_n; i += (size_t)a.clear_ctas * kPreThreads) {
+            a.clear[0][i] = 0u;
+            a.clear[1][i] = 0u;
+        }
+        return;
+    }
+    // the last CTA: the post-advance clock and scenario state of the step's tape slice
+    const uint32_t j = st->step % a.slices;
+    if (threadIdx.x == 0) a.st_out[j] = *st;
+    for (uint32_t s = threadIdx.x; s < c.n_scen; s += kPreThreads) a.sc_out[(size_t)j * c.n_scen + s] = sc[s];
 }
 
 // One work item is a chunk of BLOCK * PPT consecutive slots of one scenario
@@ -234,15 +296,6 @@ struct GridConst {
     float lower[kSortedLevels - 1];     // level_sorted's table when `sorted`
 };
 
-__global__ void __launch_bounds__(256) batch_grid_clear_kernel(const BatchState* st, uint32_t every, uint32_t* counts,
-                                                               uint32_t* mass, size_t total) {
-    if (every == 0 || (st->step + 1u) % every != 0u) return;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        counts[i] = 0u;
-        mass[i] = 0u;
-    }
-}
-
 // concentration_gridding.wgsl:323-345 per scenario.  Each CTA bins a
 // contiguous range of tiles (a tile is 256 slots of one scenario); the key of
 // a particle is its index in the scenario-major grid, so one CTA table holds
@@ -291,15 +344,6 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(const BatchState* st, c
             atomicAdd(counts + k, t_cnt[i]);
             atomicAdd(mass + k, t_mass[i]);
         }
-    }
-}
-
-__global__ void batch_end_kernel(BatchState* st, ScenDev* sc, BatchConst c) {
-    for (uint32_t s = threadIdx.x; s < c.n_scen; s += blockDim.x)
-        sc[s].counter = counter_add64(sc[s].counter, (uint64_t)sc[s].capacity * c.bpp);
-    if (threadIdx.x == 0) {
-        st->t += c.dt;
-        st->step += 1u;
     }
 }
 
@@ -389,44 +433,70 @@ PopFields pop_fields(fpg_batch* b) {
     return F;
 }
 
-// The per-step kernels before and after the particle pass (shared by the
-// batched and sequential paths).
-void enqueue_pre(fpg_batch* b, cudaStream_t s) {
-    const BatchConst c = make_const(b);
-    const uint32_t nodes = (uint32_t)(b->met->nx * b->met->ny * b->met->nz);
-    const uint32_t cells = (uint32_t)(b->pbl->nx * b->pbl->ny);
-    batch_advance_kernel<<<1, 256, 0, s>>>(b->st, b->sc, c);
-    batch_pack_kernel<<<b->ctx->sm_count * 4, 256, 0, s>>>(b->st, b->ring, nodes, b->met->bracket);
-    batch_pbl_kernel<<<(cells + 255) / 256, 256, 0, s>>>(
-        b->st, b->sring, b->pring, b->cfg.pbl_options, cells, b->pbl->field[0], b->pbl->field[1], b->pbl->field[2],
-        b->pbl->field[3], b->pbl->field[4], b->pbl->field[5], b->pbl->field[6], b->pbl->packed, b->pbl->hanna,
-        b->cfg.wet_from_precipitation, b->cfg.wet_gas_a, b->cfg.wet_gas_b, b->wet ? b->wet->lf : nullptr);
-    batch_release_kernel<<<dim3(16, (unsigned)b->scen.size()), 256, 0, s>>>(b->st, b->sc, c, pop_fields(b));
-    b->ctx->count(4);
+static bool grid_step(const fpg_batch* b, uint64_t step) {
+    const fpg_batch_config& c = b->cfg;
+    return c.output_every_steps && c.out_nx && c.out_ny && c.out_nz && b->n_tiles &&
+           (step + 1) % c.output_every_steps == 0;
 }
 
-void enqueue_post(fpg_batch* b, cudaStream_t s) {
+bool output_step(const fpg_batch* b, uint64_t step) { return grid_step(b, step) || inverse_sample_step(b, step); }
+
+// Everything before the particle pass; `output`: the step ends with grids.
+// st_out, sc_out: where an inversion keeps the step's state.
+void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, ScenDev* sc_out, uint32_t slices) {
     const BatchConst c = make_const(b);
-    const GridConst g = make_grid_const(b);
-    const size_t total = (size_t)g.cells * b->scen.size();
-    if (g.every && g.cells && b->n_tiles) {
-        batch_grid_clear_kernel<<<b->ctx->sm_count * 4, 256, 0, s>>>(b->st, g.every, b->grid_counts, b->grid_mass,
-                                                                     total);
+    PreArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.ring = b->ring;
+    a.bracket = b->met->bracket;
+    a.nodes = (uint32_t)(b->met->nx * b->met->ny * b->met->nz);
+    a.pack_ctas = std::min<uint32_t>((a.nodes + kPreThreads - 1u) / kPreThreads, (uint32_t)b->ctx->sm_count * 8u);
+    a.sring = b->sring;
+    a.precip = b->pring;
+    a.pbl = b->cfg.pbl_options;
+    a.ncell = (uint32_t)(b->pbl->nx * b->pbl->ny);
+    a.pbl_ctas = (a.ncell + kPreThreads - 1u) / kPreThreads;
+    for (int k = 0; k < 7; ++k) a.field[k] = b->pbl->field[k];
+    a.packed = b->pbl->packed;
+    a.hanna = b->pbl->hanna;
+    a.wet_on = b->cfg.wet_from_precipitation;
+    a.wet_a = b->cfg.wet_gas_a;
+    a.wet_b = b->cfg.wet_gas_b;
+    a.wet = b->wet ? b->wet->lf : nullptr;
+    a.parts = std::max<uint32_t>(1u, std::min<uint32_t>(32u, 1024u / c.n_scen));
+    a.F = pop_fields(b);
+    a.st_out = st_out;
+    a.sc_out = sc_out;
+    a.slices = std::max(slices, 1u);
+    if (output && b->cfg.output_every_steps) {
+        a.clear[0] = b->grid_counts;
+        a.clear[1] = b->grid_mass;
+        a.clear_n = (size_t)b->cfg.out_nx * b->cfg.out_ny * b->cfg.out_nz * b->scen.size();
+        a.clear_ctas = (uint32_t)b->ctx->sm_count * 8u;
+    }
+    const uint32_t ctas = a.pbl_ctas + c.n_scen * a.parts + a.pack_ctas + a.clear_ctas + (st_out ? 1u : 0u);
+    batch_pre_kernel<<<ctas, kPreThreads, 0, s>>>(b->st, b->sc, c, a);
+    b->ctx->count(1);
+}
+
+// Everything after it; `output`: the step ends with grids or receptor samples.
+void enqueue_post(fpg_batch* b, cudaStream_t s, bool output) {
+    if (output && b->cfg.output_every_steps) {
+        const GridConst g = make_grid_const(b);
         // 8 resident CTAs per SM, each over a contiguous range of tiles
         const uint32_t ctas = std::max<uint32_t>(1u, std::min<uint32_t>(b->n_tiles, (uint32_t)b->ctx->sm_count * 8u));
         const uint32_t per = (b->n_tiles + ctas - 1u) / ctas;
         const uint32_t blocks = std::max<uint32_t>(1u, (b->n_tiles + per - 1u) / per);
         batch_grid_kernel<<<blocks, 256, 0, s>>>(b->st, b->sc, b->tile_scen, pop_fields(b), g, b->n_tiles, per,
                                                  b->grid_counts, b->grid_mass);
-        b->ctx->count(2);
+        b->ctx->count(1);
     }
-    if (b->inv) enqueue_inverse_sample(b, s);
-    batch_end_kernel<<<1, 256, 0, s>>>(b->st, b->sc, c);
-    b->ctx->count(1);
+    if (output && b->inv) enqueue_inverse_sample(b, s);
+    enqueue_turn(b, s, true);
 }
 
-void enqueue_end(fpg_batch* b, cudaStream_t s) {
-    batch_end_kernel<<<1, 256, 0, s>>>(b->st, b->sc, make_const(b));
+void enqueue_turn(fpg_batch* b, cudaStream_t s, bool end) {
+    batch_turn_kernel<<<1, 256, 0, s>>>(b->st, b->sc, make_const(b), end ? 1 : 0);
     b->ctx->count(1);
 }
 
@@ -443,10 +513,19 @@ void enqueue_step_kernel(fpg_batch* b, cudaStream_t s) {
     b->ctx->count(1);
 }
 
-void enqueue_batched_step(fpg_batch* b, cudaStream_t s) {
-    enqueue_pre(b, s);
+void enqueue_batched_step(fpg_batch* b, cudaStream_t s, bool output) {
+    enqueue_pre(b, s, output, nullptr, nullptr, 0);
     enqueue_step_kernel(b, s);
-    enqueue_post(b, s);
+    enqueue_post(b, s, output);
+}
+
+static void drop_graphs(fpg_batch* b) {
+    for (int o = 0; o < 2; ++o) {
+        if (b->exec[o]) cudaGraphExecDestroy(b->exec[o]);
+        if (b->graph[o]) cudaGraphDestroy(b->graph[o]);
+        b->exec[o] = nullptr;
+        b->graph[o] = nullptr;
+    }
 }
 
 // Work items of shape `v`: every scenario cut into chunks of block * ppt slots.
@@ -467,9 +546,7 @@ fpg_status build_items(fpg_batch* b, uint32_t v) {
     FPG_CUDA(cudaStreamSynchronize(b->ctx->stream));
     b->n_items = (uint32_t)items.size();
     b->variant = v;
-    // a captured graph holds the old shape
-    if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
-    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
+    drop_graphs(b);                                      // the captured graphs hold the old shape
     return FPG_OK;
 }
 
@@ -496,6 +573,8 @@ fpg_status batch_reset(fpg_batch* b) {
     s0.t = b->cfg.start_seconds;
     FPG_CUDA(cudaMemcpyAsync(b->st, &s0, sizeof(s0), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(b->sc, b->scen.data(), b->scen.size() * sizeof(ScenDev), cudaMemcpyHostToDevice, s));
+    enqueue_turn(b, s, false);
+    FPG_CHECK_LAUNCH();
     FPG_CUDA(cudaStreamSynchronize(s));
     b->steps_done = 0;
     b->t_h = b->cfg.start_seconds;
@@ -506,20 +585,30 @@ fpg_status batch_reset(fpg_batch* b) {
     return FPG_OK;
 }
 
-fpg_status ensure_graph(fpg_batch* b) {
-    if (b->exec) return FPG_OK;
+// The graph of a step, without (0) and with (1) grids or receptor samples.
+fpg_status ensure_graph(fpg_batch* b, int output) {
+    if (b->exec[output]) return FPG_OK;
     cudaStream_t s = b->ctx->stream;
     FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = b->ctx->launches.load();
-    enqueue_batched_step(b, s);
+    enqueue_batched_step(b, s, output != 0);
     // capture launches nothing: take the count back, keep it per replay
-    b->graph_launches = b->ctx->launches.load() - before;
-    b->ctx->launches.fetch_sub(b->graph_launches);
+    b->graph_launches[output] = b->ctx->launches.load() - before;
+    b->ctx->launches.fetch_sub(b->graph_launches[output]);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess) return cuda_status(e);
-    b->graph = g;
-    FPG_CUDA(cudaGraphInstantiate(&b->exec, g, 0));
+    b->graph[output] = g;
+    FPG_CUDA(cudaGraphInstantiate(&b->exec[output], g, 0));
+    return FPG_OK;
+}
+
+fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
+    const int output = output_step(b, step) ? 1 : 0;
+    const fpg_status st = ensure_graph(b, output);
+    if (st != FPG_OK) return st;
+    FPG_CUDA(cudaGraphLaunch(b->exec[output], s));
+    b->ctx->count(b->graph_launches[output]);
     return FPG_OK;
 }
 
@@ -547,8 +636,7 @@ using namespace fpg;
 extern "C" fpg_status fpg_batch_destroy(fpg_batch* b) {
     if (!b) return FPG_OK;
     cudaStreamSynchronize(b->ctx->stream);
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
+    drop_graphs(b);
     fpg_particles_destroy(b->pop);
     fpg_met_destroy(b->met);
     fpg_pbl_destroy(b->pbl);
@@ -649,6 +737,10 @@ extern "C" fpg_status fpg_batch_create(fpg_ctx* ctx, const fpg_batch_config* cfg
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->tile_scen, b->tile_scen_h.data(), b->n_tiles * sizeof(uint32_t), cudaMemcpyHostToDevice,
                             ctx->stream);
+    if (e == cudaSuccess) {
+        enqueue_turn(b, ctx->stream, false);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { fpg_batch_destroy(b); return cuda_status(e); }
     for (uint32_t v = 0; v < kNumVariants; ++v) {
@@ -696,16 +788,13 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
     if (b->steps_done >= b->total_steps) return FPG_ERR_SIMULATION_COMPLETE;
     const uint64_t n = std::min<uint64_t>(n_steps, b->total_steps - b->steps_done);
     cudaStream_t s = b->ctx->stream;
-    if (use_graph) {
-        const fpg_status st = ensure_graph(b);
-        if (st != FPG_OK) return st;
-    }
     for (uint64_t i = 0; i < n; ++i) {
+        const uint64_t step = b->steps_done + i;
         if (use_graph) {
-            FPG_CUDA(cudaGraphLaunch(b->exec, s));
-            b->ctx->count(b->graph_launches);
+            const fpg_status st = launch_step_graph(b, step, s);
+            if (st != FPG_OK) return st;
         } else {
-            enqueue_batched_step(b, s);
+            enqueue_batched_step(b, s, output_step(b, step));
             FPG_CHECK_LAUNCH();
         }
     }
@@ -733,7 +822,8 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
     StepArgs base = make_step_args(b);
     // alpha of the step comes from the host clock (same formula as the device)
     for (uint64_t i = 0; i < n; ++i) {
-        enqueue_pre(b, s);
+        const bool output = output_step(b, b->steps_done + i);
+        enqueue_pre(b, s, output, nullptr, nullptr, 0);
         int64_t k = (b->t_h - b->cfg.start_seconds) / b->cfg.frame_seconds;
         if (b->t_h - b->cfg.start_seconds == k * b->cfg.frame_seconds && k > 0) k -= 1;
         const int64_t ta = b->cfg.start_seconds + k * b->cfg.frame_seconds;
@@ -760,7 +850,7 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
             fused_step_kernel<<<(released + 255) / 256, 256, 0, s>>>(a);
             b->ctx->count();
         }
-        enqueue_post(b, s);
+        enqueue_post(b, s, output);
         FPG_CHECK_LAUNCH();
         b->t_h += b->cfg.timestep_seconds;
     }
@@ -870,7 +960,7 @@ extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_
         for (uint32_t r = 0; status == FPG_OK && e == cudaSuccess && r < reps; ++r) {
             e = restore();
             if (e != cudaSuccess) break;
-            enqueue_pre(b, s);
+            enqueue_pre(b, s, false, nullptr, nullptr, 0);
             e = cudaEventRecord(e0, s);
             if (e != cudaSuccess) break;
             enqueue_step_kernel(b, s);

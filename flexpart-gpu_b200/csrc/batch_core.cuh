@@ -35,7 +35,7 @@ struct ScenDev {
     uint32_t key0, key1;
     u32x4 counter;
     PhiloxHead head;                 // of the coming step's counter, and whether no block's counter
-    uint32_t head_ok;                // carries out of its first word (batch_advance_kernel)
+    uint32_t head_ok;                // carries out of its first word (batch_turn_kernel)
     uint32_t released, rel_lo, rel_hi;
     float mass_per_particle;
     int64_t start, end;
@@ -115,9 +115,10 @@ struct fpg_batch {
     float tuned_ms = 0.0f;
     uint32_t* grid_counts = nullptr;
     uint32_t* grid_mass = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    uint64_t graph_launches = 0;          // kernels in one replay of the step graph
+    // the step's graphs: without (0) and with (1) grids or receptor samples at its end
+    cudaGraph_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    uint64_t graph_launches[2] = {0, 0};  // kernels in one replay
     std::vector<uint32_t> released_h;     // host mirror of the release counts (sequential path)
     std::vector<fpg::u32x4> counter_h;
     int64_t t_h = 0;
@@ -130,19 +131,24 @@ namespace fpg {
 StepArgs make_step_args(fpg_batch* b);
 BatchConst make_const(const fpg_batch* b);
 PopFields pop_fields(fpg_batch* b);
-// Per-step kernels before the particle pass (clock, bracket, PBL, release),
-// the particle pass in the chosen launch shape, and the kernels after it
-// (grids, inversion sampling, counter and clock advance).
-void enqueue_pre(fpg_batch* b, cudaStream_t s);
+// Whether step `step` ends with grids or receptor samples.
+bool output_step(const fpg_batch* b, uint64_t step);
+// The launch before the particle pass (bracket, PBL, releases, cleared grids;
+// with st_out and sc_out the step's state kept in slice step % slices), the
+// particle pass in the chosen launch shape, and the launches after it (grids
+// or receptor samples, counter and clock advance).
+void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, ScenDev* sc_out, uint32_t slices);
 void enqueue_step_kernel(fpg_batch* b, cudaStream_t s);
-void enqueue_post(fpg_batch* b, cudaStream_t s);
+void enqueue_post(fpg_batch* b, cudaStream_t s, bool output);
+// Counters and clock to the next step (`end`), and that step's bracket, alpha
+// and release ranges.
+void enqueue_turn(fpg_batch* b, cudaStream_t s, bool end);
 // Repacks the bracket of state st's frames whether or not it changed.
 void enqueue_pack_forced(fpg_batch* b, const BatchState* st, cudaStream_t s);
 fpg_status build_items(fpg_batch* b, uint32_t variant);
-// The counter and clock advance alone (batch_end_kernel).
-void enqueue_end(fpg_batch* b, cudaStream_t s);
-// Captures the step graph (pre, particle pass, post) if none is held.
-fpg_status ensure_graph(fpg_batch* b);
+// Launches step `step` from its graph (pre, particle pass, post), captured
+// when none is held.
+fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s);
 // FPG_ERR_OUT_OF_GRID when the scenario's release lattice leaves the grid.
 fpg_status check_release_grid(const ScenDev& d, const fpg_grid_domain& g);
 size_t particles_block_bytes(size_t capacity);
@@ -150,6 +156,7 @@ size_t particles_block_bytes(size_t capacity);
 // scenarios' initial counters, no bracket on the device.
 fpg_status batch_reset(fpg_batch* b);
 // Receptor sampling of a source inversion at output steps (adjoint.cu).
+bool inverse_sample_step(const fpg_batch* b, uint64_t step);
 void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s);
 
 }  // namespace fpg
