@@ -103,9 +103,10 @@ __device__ __forceinline__ int receptor_at(const Receptors& r, uint32_t inst, in
 
 // ---- forward sampling ---------------------------------------------------------
 
-__global__ void __launch_bounds__(256) inverse_sample_kernel(const BatchState* st, const ScenDev* __restrict__ sc,
+__global__ void __launch_bounds__(256) inverse_sample_kernel(const BatchState* st, const ScenDev* sc,
                                                              const uint2* __restrict__ items, uint32_t n_items,
                                                              PopFields F, Receptors r) {
+    chain_begin();
     if (r.every == 0 || (st->step + 1u) % r.every != 0u) return;
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
         const uint2 w = items[it];
@@ -167,10 +168,11 @@ struct TapeRec {
 // One CTA per 256-slot work item, launched over all items; the level arrays
 // are read from global memory (no staging, no barrier).
 __global__ void __launch_bounds__(256, 4) inverse_tape_kernel(StepArgs a, const BatchState* st,
-                                                              const ScenDev* __restrict__ sc,
+                                                              const ScenDev* sc,
                                                               const uint2* __restrict__ items, uint32_t n_items,
                                                               TapeBase tb, uint32_t every,
-                                                              const uint32_t* __restrict__ live) {
+                                                              const uint32_t* live) {
+    chain_begin();
     if (blockIdx.x >= n_items) return;
     const uint2 w = items[blockIdx.x];
     const ScenDev& d = sc[w.x];
@@ -385,12 +387,13 @@ __device__ __forceinline__ void receptor_seed(const Receptors& r, uint32_t inst,
 // scenario, so a warp's lanes share the scenario: the release gradients are
 // summed across the warp first.
 __global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, const BatchState* st,
-                                                                 const ScenDev* __restrict__ sc,
+                                                                 const ScenDev* sc,
                                                                  const uint2* __restrict__ items, uint32_t n_items,
                                                                  uint32_t* work, TapeBase tb, uint32_t slice,
                                                                  LamArrays lam, Receptors r,
                                                                  double* __restrict__ dbias,
                                                                  double* __restrict__ dsrc) {
+    chain_begin();
     extern __shared__ float s_levels[];
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_bias_key[kBiasTable];
@@ -539,6 +542,7 @@ struct CheckpointArgs {
 };
 
 __global__ void __launch_bounds__(256) inverse_checkpoint_kernel(CheckpointArgs a) {
+    chain_begin();
     const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     if (blockIdx.y == kNumCkptFields) {
         for (size_t s = first; s < a.n_scen; s += step) {
@@ -554,8 +558,8 @@ __global__ void __launch_bounds__(256) inverse_checkpoint_kernel(CheckpointArgs 
         }
         return;
     }
-    const uint4* __restrict__ from = a.restore ? a.saved[blockIdx.y] : a.field[blockIdx.y];
-    uint4* __restrict__ to = a.restore ? a.field[blockIdx.y] : a.saved[blockIdx.y];
+    const uint4* from = a.restore ? a.saved[blockIdx.y] : a.field[blockIdx.y];
+    uint4* to = a.restore ? a.field[blockIdx.y] : a.saved[blockIdx.y];
     for (size_t i = first; i < a.quads; i += step) to[i] = from[i];
 }
 
@@ -624,8 +628,7 @@ bool inverse_sample_step(const fpg_batch* b, uint64_t step) {
 void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s) {
     InverseData* inv = b->inv;
     const Receptors r = inv->receptors_args((uint32_t)b->met->nx, (uint32_t)b->met->ny);
-    inverse_sample_kernel<<<b->ctx->sm_count * 8, 256, 0, s>>>(b->st, b->sc, inv->items, inv->n_items,
-                                                              pop_fields(b), r);
+    launch_chained(inverse_sample_kernel, b->ctx->sm_count * 8, 256, 0, s, b->st, b->sc, inv->items, inv->n_items, pop_fields(b), r);
     b->ctx->count(1);
 }
 
@@ -655,9 +658,7 @@ static void enqueue_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
     fpg_batch* b = v->b;
     InverseData& d = v->d;
     enqueue_pre(b, s, false, d.st_all, d.sc_all, d.slices);
-    inverse_tape_kernel<<<std::max(d.n_items, 1u), 256, 0, s>>>(make_step_args(b), b->st, b->sc, d.items, d.n_items,
-                                                                tape_base(v), d.cfg.sample_every_steps,
-                                                                kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
+    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u), 256, 0, s, make_step_args(b), b->st, b->sc, d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps, kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
     b->ctx->count(1);
     if (kind == TAPE_FORWARD_SAMPLE) enqueue_inverse_sample(b, s);
     enqueue_turn(b, s, true);
@@ -710,7 +711,7 @@ static cudaError_t enqueue_checkpoint(fpg_inverse* v, uint32_t c, bool restore) 
     a.restore = restore ? 1 : 0;
     const size_t per = 4 * 256;
     const unsigned x = (unsigned)std::min<size_t>((a.quads + per - 1) / per, (size_t)b->ctx->sm_count * 8);
-    inverse_checkpoint_kernel<<<dim3(std::max(x, 1u), kNumCkptFields + 1), 256, 0, b->ctx->stream>>>(a);
+    launch_chained(inverse_checkpoint_kernel, dim3(std::max(x, 1u), kNumCkptFields + 1), 256, 0, b->ctx->stream, a);
     b->ctx->count(1);
     return cudaGetLastError();
 }
@@ -955,9 +956,7 @@ extern "C" fpg_status fpg_inverse_backward(fpg_inverse* v, const double* d_sim, 
                 enqueue_pack_forced(b, d.st_all + j, s);
                 d.packed_ta = ta;
             }
-            inverse_adjoint_kernel<<<d.grid_adj, 256, smem, s>>>(a, d.st_all + j, d.sc_all + (size_t)j * n_src,
-                                                                 d.items, d.n_items, d.work_rev + j, tb, j, lam,
-                                                                 rargs, d_bias ? d.dbias : nullptr, d.dsrc);
+            launch_chained(inverse_adjoint_kernel, d.grid_adj, 256, smem, s, a, d.st_all + j, d.sc_all + (size_t)j * n_src, d.items, d.n_items, d.work_rev + j, tb, j, lam, rargs, d_bias ? d.dbias : nullptr, d.dsrc);
             b->ctx->count(1);
             FPG_CHECK_LAUNCH();
         }

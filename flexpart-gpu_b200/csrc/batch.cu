@@ -67,6 +67,7 @@ __device__ __forceinline__ void advance_clock(BatchState* st, const BatchConst& 
 // so that a step is one launch before its particle pass and one after it.
 // Runs once without `end` when the state is (re)set.
 __global__ void __launch_bounds__(256) batch_turn_kernel(BatchState* st, ScenDev* sc, BatchConst c, int end) {
+    chain_begin();
     const int64_t t = st->t + (end ? c.dt : 0);
     for (uint32_t s = threadIdx.x; s < c.n_scen; s += blockDim.x) {
         ScenDev& d = sc[s];
@@ -155,8 +156,9 @@ struct PreArgs {
 };
 constexpr uint32_t kPreThreads = 128;
 
-__global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, const ScenDev* __restrict__ sc, BatchConst c,
+__global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, const ScenDev* sc, BatchConst c,
                                                                 PreArgs a) {
+    chain_begin();
     uint32_t b = blockIdx.x;
     if (b < a.pbl_ctas) {
         const uint32_t i = b * kPreThreads + threadIdx.x;
@@ -201,8 +203,9 @@ __global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, 
 // scenarios share the machine without a per-scenario launch.
 template <int BLOCK, int MINB, int PPT>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_step_kernel(StepArgs a, BatchState* st,
-                                                                 const ScenDev* __restrict__ sc,
+                                                                 const ScenDev* sc,
                                                                  const uint2* __restrict__ items, uint32_t n_items) {
+    chain_begin();
     extern __shared__ float s_levels[];
     __shared__ uint32_t s_item;
     const Levels lv = stage_levels(a, s_levels);
@@ -231,9 +234,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step_kernel(StepArgs a, Bat
 // block scheduler spreading the items of small and large scenarios.
 template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_step_flat_kernel(StepArgs a, BatchState* st,
-                                                                      const ScenDev* __restrict__ sc,
+                                                                      const ScenDev* sc,
                                                                       const uint2* __restrict__ items,
                                                                       uint32_t n_items) {
+    chain_begin();
     if (blockIdx.x >= n_items) return;
     const uint2 w = items[blockIdx.x];
     const ScenDev& d = sc[w.x];
@@ -249,9 +253,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step_flat_kernel(StepArgs a
 // and 12 CTAs of 128 threads; 150 scenarios 697 us, against 757, 724, 699.
 template <bool kWet, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) batch_production_kernel(StepArgs a, BatchState* st,
-                                                                       const ScenDev* __restrict__ sc,
+                                                                       const ScenDev* sc,
                                                                        const uint2* __restrict__ items,
                                                                        uint32_t n_items) {
+    chain_begin();
     if (blockIdx.x >= n_items) return;
     const uint2 w = items[blockIdx.x];
     const ScenDev& d = sc[w.x];
@@ -302,10 +307,11 @@ struct GridConst {
 // the cells of every scenario its tiles touch.  Runs of equal keys in a warp
 // are summed by the segmented scan, the run ends add to the table, and the
 // table goes to the grids once per cell per CTA (grid_core.cuh).
-__global__ void __launch_bounds__(256) batch_grid_kernel(const BatchState* st, const ScenDev* __restrict__ sc,
+__global__ void __launch_bounds__(256) batch_grid_kernel(const BatchState* st, const ScenDev* sc,
                                                          const uint32_t* __restrict__ tile_scen, PopFields F,
                                                          GridConst g, uint32_t n_tiles, uint32_t tiles_per_cta,
                                                          uint32_t* counts, uint32_t* mass) {
+    chain_begin();
     if (g.every == 0 || (st->step + 1u) % g.every != 0u) return;
     __shared__ float s_h[FPG_MAX_LEVELS];
     __shared__ uint32_t t_key[kTable], t_cnt[kTable], t_mass[kTable];
@@ -475,7 +481,7 @@ void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, 
         a.clear_ctas = (uint32_t)b->ctx->sm_count * 8u;
     }
     const uint32_t ctas = a.pbl_ctas + c.n_scen * a.parts + a.pack_ctas + a.clear_ctas + (st_out ? 1u : 0u);
-    batch_pre_kernel<<<ctas, kPreThreads, 0, s>>>(b->st, b->sc, c, a);
+    launch_chained(batch_pre_kernel, ctas, kPreThreads, 0, s, b->st, b->sc, c, a);
     b->ctx->count(1);
 }
 
@@ -487,8 +493,7 @@ void enqueue_post(fpg_batch* b, cudaStream_t s, bool output) {
         const uint32_t ctas = std::max<uint32_t>(1u, std::min<uint32_t>(b->n_tiles, (uint32_t)b->ctx->sm_count * 8u));
         const uint32_t per = (b->n_tiles + ctas - 1u) / ctas;
         const uint32_t blocks = std::max<uint32_t>(1u, (b->n_tiles + per - 1u) / per);
-        batch_grid_kernel<<<blocks, 256, 0, s>>>(b->st, b->sc, b->tile_scen, pop_fields(b), g, b->n_tiles, per,
-                                                 b->grid_counts, b->grid_mass);
+        launch_chained(batch_grid_kernel, blocks, 256, 0, s, b->st, b->sc, b->tile_scen, pop_fields(b), g, b->n_tiles, per, b->grid_counts, b->grid_mass);
         b->ctx->count(1);
     }
     if (output && b->inv) enqueue_inverse_sample(b, s);
@@ -496,7 +501,7 @@ void enqueue_post(fpg_batch* b, cudaStream_t s, bool output) {
 }
 
 void enqueue_turn(fpg_batch* b, cudaStream_t s, bool end) {
-    batch_turn_kernel<<<1, 256, 0, s>>>(b->st, b->sc, make_const(b), end ? 1 : 0);
+    launch_chained(batch_turn_kernel, 1, 256, 0, s, b->st, b->sc, make_const(b), end ? 1 : 0);
     b->ctx->count(1);
 }
 
@@ -505,10 +510,10 @@ void enqueue_step_kernel(fpg_batch* b, cudaStream_t s) {
     const StepArgs a = make_step_args(b);
     if (v.ppt == 0) {
         const StepKernel kernel = production_form(a) ? v.production[a.wet_mode == FPG_FORCING_PER_CELL] : v.kernel;
-        kernel<<<std::max(b->n_items, 1u), v.block, 0, s>>>(a, b->st, b->sc, b->items, b->n_items);
+        launch_chained(kernel, std::max(b->n_items, 1u), v.block, 0, s, a, b->st, b->sc, b->items, b->n_items);
     } else {
         const uint32_t grid = (uint32_t)b->ctx->sm_count * std::max(b->resident[b->variant], 1u);
-        v.kernel<<<grid, v.block, level_smem_bytes(b->met), s>>>(a, b->st, b->sc, b->items, b->n_items);
+        launch_chained(v.kernel, grid, v.block, level_smem_bytes(b->met), s, a, b->st, b->sc, b->items, b->n_items);
     }
     b->ctx->count(1);
 }

@@ -102,18 +102,19 @@ __device__ __forceinline__ void store_zero_output(fpg_cbl_sampling_output* out, 
 }
 
 // cbl.wgsl:251-298: PDF from the slot's Hanna record, sample from its uniforms.
-__global__ void __launch_bounds__(256) cbl_sample_kernel(SlotView v, const fpg_hanna_params* __restrict__ hanna,
-                                                         const fpg_cbl_sampling_input* __restrict__ in,
-                                                         fpg_cbl_sampling_output* __restrict__ out) {
+__global__ void __launch_bounds__(256) cbl_sample_kernel(SlotView v, const fpg_hanna_params* hanna,
+                                                         const fpg_cbl_sampling_input* in,
+                                                         fpg_cbl_sampling_output* out) {
+    chain_begin();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.n) return;
     if ((v.flags[p] & FLAG_ACTIVE) == 0u) {
         store_zero_output(out, p);
         return;
     }
-    const float4 h0 = __ldg(reinterpret_cast<const float4*>(hanna + p));       // ust, wst, ol, h
-    const float sigw = __ldg(&hanna[p].sigw);
-    const float4 u = __ldg(reinterpret_cast<const float4*>(in + p));
+    const float4 h0 = *reinterpret_cast<const float4*>(hanna + p);       // ust, wst, ol, h
+    const float sigw = hanna[p].sigw;
+    const float4 u = *reinterpret_cast<const float4*>(in + p);
     const CblPdf pdf = cbl_pdf(v.pos_z[p], h0.w, h0.y, sigw, h0.z);
     store_output(out, p, cbl_draw(pdf, u.x, u.y, u.z), pdf);
 }
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(256) cbl_sample_philox_kernel(SlotView v, cons
                                                                 uint32_t pnx, uint32_t pny, uint32_t k0,
                                                                 uint32_t k1, u32x4 counter,
                                                                 fpg_cbl_sampling_output* __restrict__ out) {
+    chain_begin();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.n) return;
     if ((v.flags[p] & FLAG_ACTIVE) == 0u) {
@@ -212,16 +214,17 @@ __device__ __forceinline__ void mix_slot(size_t p, float z_in, float* __restrict
 // slots is written with one 16-byte store per field, otherwise only the
 // active slots are written.  The last n % 4 slots take scalar loads.
 template <bool kSorted>
-__global__ void __launch_bounds__(256) conv_apply_kernel(size_t n, const uint32_t* __restrict__ flags,
-                                                         float* __restrict__ pos_z, int32_t* __restrict__ cbt,
+__global__ void __launch_bounds__(256) conv_apply_kernel(size_t n, const uint32_t* flags,
+                                                         float* pos_z, int32_t* cbt,
                                                          uint32_t L, const float* __restrict__ iface,
                                                          const float* __restrict__ heights,
                                                          const uint32_t* __restrict__ has_weight) {
+    chain_begin();
     const size_t p0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4u;
     if (p0 >= n) return;
     const float z_min = __ldg(iface), z_max = __ldg(iface + L);
     if (p0 + 4u <= n) {
-        const uint4 f = __ldg(reinterpret_cast<const uint4*>(flags + p0));
+        const uint4 f = *reinterpret_cast<const uint4*>(flags + p0);
         const float4 z = *reinterpret_cast<const float4*>(pos_z + p0);
         if (f.x & f.y & f.z & f.w & FLAG_ACTIVE) {
             int4 lv;
@@ -273,8 +276,7 @@ extern "C" fpg_status fpg_cbl_sample(fpg_ctx* ctx, const fpg_particles* P, const
     if (!hanna_dev || !inputs_dev || !out_dev) return FPG_ERR_INVALID_ARGUMENT;
     if (!aligned16(hanna_dev) || !aligned16(inputs_dev) || !aligned16(out_dev)) return FPG_ERR_INVALID_ARGUMENT;
     if (v.n > UINT32_MAX) return FPG_ERR_VALUE_TOO_LARGE;
-    cbl_sample_kernel<<<(unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream)>>>(v, hanna_dev, inputs_dev,
-                                                                                   out_dev);
+    launch_chained(cbl_sample_kernel, (unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream), v, hanna_dev, inputs_dev, out_dev);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;
@@ -291,8 +293,7 @@ extern "C" fpg_status fpg_cbl_sample_philox(fpg_ctx* ctx, const fpg_particles* P
     if (v.n == 0) return FPG_OK;
     if (!out_dev || !aligned16(out_dev)) return FPG_ERR_INVALID_ARGUMENT;
     const u32x4 c{counter[0], counter[1], counter[2], counter[3]};
-    cbl_sample_philox_kernel<<<(unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream)>>>(
-        v, pbl->hanna, (uint32_t)pbl->nx, (uint32_t)pbl->ny, key[0], key[1], c, out_dev);
+    launch_chained(cbl_sample_philox_kernel, (unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream), v, pbl->hanna, (uint32_t)pbl->nx, (uint32_t)pbl->ny, key[0], key[1], c, out_dev);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;
@@ -393,11 +394,9 @@ extern "C" fpg_status fpg_convective_mixing(fpg_ctx* ctx, fpg_particles* P, cons
     auto* cbt = static_cast<int32_t*>(P->field[FPG_FIELD_CBT]);
     const unsigned grid = (unsigned)(((n + 3) / 4 + 255) / 256);
     if (c->sorted)
-        conv_apply_kernel<true><<<grid, 256, 0, ctx->pick(stream)>>>(n, flags, pos_z, cbt, (uint32_t)c->levels,
-                                                                    c->iface, c->heights, c->has_weight);
+        launch_chained(conv_apply_kernel<true>, grid, 256, 0, ctx->pick(stream), n, flags, pos_z, cbt, (uint32_t)c->levels, c->iface, c->heights, c->has_weight);
     else
-        conv_apply_kernel<false><<<grid, 256, 0, ctx->pick(stream)>>>(n, flags, pos_z, cbt, (uint32_t)c->levels,
-                                                                     c->iface, c->heights, c->has_weight);
+        launch_chained(conv_apply_kernel<false>, grid, 256, 0, ctx->pick(stream), n, flags, pos_z, cbt, (uint32_t)c->levels, c->iface, c->heights, c->has_weight);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;

@@ -36,8 +36,9 @@ constexpr int CT_TILE = CT_THREADS * CT_ITEMS;
 // Per-tile active count.  Slot order inside a tile: item-major chunks of 256
 // (chunk c covers slots tile*TILE + c*256 .. +255), warp w of the chunk
 // covers 32 consecutive slots.
-__global__ void __launch_bounds__(CT_THREADS) compact_count_kernel(const uint32_t* __restrict__ flags, uint32_t n,
-                                                                   uint32_t* __restrict__ tile_counts) {
+__global__ void __launch_bounds__(CT_THREADS) compact_count_kernel(const uint32_t* flags, uint32_t n,
+                                                                   uint32_t* tile_counts) {
+    chain_begin();
     __shared__ uint32_t s_warp[CT_THREADS / 32];
     const uint32_t tile = blockIdx.x;
     uint32_t local = 0;
@@ -57,7 +58,8 @@ __global__ void __launch_bounds__(CT_THREADS) compact_count_kernel(const uint32_
 }
 
 // Exclusive scan of the tile counts in one block of 1024 threads.
-__global__ void __launch_bounds__(1024) compact_scan_kernel(uint32_t* __restrict__ tile_counts, uint32_t n_tiles) {
+__global__ void __launch_bounds__(1024) compact_scan_kernel(uint32_t* tile_counts, uint32_t n_tiles) {
+    chain_begin();
     __shared__ uint32_t s[1024];
     const uint32_t per = (n_tiles + 1023u) / 1024u;
     const uint32_t begin = threadIdx.x * per;
@@ -100,11 +102,11 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp) {
 // (16.8 M slots, 32 KB a CTA) the scan kernel runs.
 constexpr uint32_t kSelfSumTiles = 8192;
 
-__global__ void __launch_bounds__(CT_THREADS) compact_index_kernel(const uint32_t* __restrict__ flags, uint32_t n,
-                                                                   const uint32_t* __restrict__ tiles, int scanned,
-                                                                   uint32_t* __restrict__ indices,
-                                                                   uint32_t* __restrict__ active_dev,
-                                                                   uint32_t* __restrict__ active_host) {
+__global__ void __launch_bounds__(CT_THREADS) compact_index_kernel(const uint32_t* flags, uint32_t n,
+                                                                   const uint32_t* tiles, int scanned,
+                                                                   uint32_t* indices, uint32_t* active_dev,
+                                                                   uint32_t* active_host) {
+    chain_begin();
     constexpr int kWarps = CT_THREADS / 32;
     __shared__ uint32_t s_below[kWarps];
     __shared__ uint32_t s_pre[CT_ITEMS * kWarps];       // counts, then exclusive prefix, in slot order
@@ -200,10 +202,9 @@ extern "C" fpg_status fpg_compact(fpg_ctx* ctx, fpg_particles* P, fpg_compaction
     uint32_t* indices = indices_dev ? indices_dev : static_cast<uint32_t*>(dst[FPG_FIELD_COUNT - 1]);
     const uint32_t tiles = (uint32_t)c->n_tiles;
     const bool scan = tiles > kSelfSumTiles;
-    compact_count_kernel<<<tiles, CT_THREADS, 0, s>>>(flags, n, c->tile_counts);
-    if (scan) compact_scan_kernel<<<1, 1024, 0, s>>>(c->tile_counts, tiles);
-    compact_index_kernel<<<tiles, CT_THREADS, 0, s>>>(flags, n, c->tile_counts, scan ? 1 : 0, indices,
-                                                      c->active_count_dev, c->active_count_host);
+    launch_chained(compact_count_kernel, tiles, CT_THREADS, 0, s, flags, n, c->tile_counts);
+    if (scan) launch_chained(compact_scan_kernel, 1, 1024, 0, s, c->tile_counts, tiles);
+    launch_chained(compact_index_kernel, tiles, CT_THREADS, 0, s, flags, n, c->tile_counts, scan ? 1 : 0, indices, c->active_count_dev, c->active_count_host);
     ctx->count(scan ? 3 : 2);
     FPG_CHECK_LAUNCH();
     const fpg_status st = move_fields(ctx, P->field, dst, indices, 0, c->active_count_dev, n, true, s);

@@ -25,6 +25,39 @@ fpg_status cuda_status(cudaError_t e);
 
 #define FPG_CHECK_LAUNCH() FPG_CUDA(cudaGetLastError())
 
+// A launch that may begin while the kernel before it on the stream still
+// runs (programmatic dependent launch): its CTAs are scheduled as soon as
+// every CTA of that kernel has called chain_begin, and their own chain_begin
+// waits until that kernel has completed and its writes are visible.  A
+// step's kernels are short (3 to 25 us below a million particles), and the
+// launch gap between two of them, 1 to 2 us, falls into the first one's tail.
+// Every kernel launched this way calls chain_begin before its first access
+// to memory, in every CTA, and reads what earlier kernels of the stream write
+// through plain pointers: a load marked read-only for the kernel's life
+// (__restrict__ const, __ldg) whose address does not come from memory could
+// be moved above the wait.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+#endif
+
 }  // namespace fpg
 
 struct fpg_ctx {

@@ -28,8 +28,9 @@ constexpr int kMoveBatch = 8;
 // 229-240 us; 32 registers, eight CTAs per SM, kept).
 __global__ void __launch_bounds__(kMoveThreads, 8) move_fields_kernel(MoveFields m, const uint32_t* index,
                                                                       uint32_t n_host,
-                                                                      const uint32_t* __restrict__ n_dev,
+                                                                      const uint32_t* n_dev,
                                                                       uint32_t capacity, int clear_tail) {
+    chain_begin();
     const uint32_t i = blockIdx.x * kMoveThreads + threadIdx.x;
     if (i >= capacity) return;
     const uint32_t n = n_dev ? *n_dev : n_host;
@@ -39,7 +40,7 @@ __global__ void __launch_bounds__(kMoveThreads, 8) move_fields_kernel(MoveFields
         uint32_t v[kMoveBatch];
 #pragma unroll
         for (int j = 0; j < kMoveBatch; ++j)
-            if (f0 + j < FPG_FIELD_COUNT) v[j] = __ldg(m.src[f0 + j] + from);
+            if (f0 + j < FPG_FIELD_COUNT) v[j] = m.src[f0 + j][from];
         if (FPG_FIELD_FLAGS >= f0 && FPG_FIELD_FLAGS < f0 + kMoveBatch && clear_tail && i >= n)
             v[FPG_FIELD_FLAGS % kMoveBatch] &= ~FPG_FLAG_ACTIVE;
 #pragma unroll
@@ -58,7 +59,7 @@ fpg_status move_fields(fpg_ctx* ctx, void* const* src, void* const* dst, const u
         m.dst[f] = static_cast<uint32_t*>(dst[f]);
     }
     const uint32_t blocks = (uint32_t)(((uint64_t)capacity + kMoveThreads - 1u) / kMoveThreads);
-    move_fields_kernel<<<blocks, kMoveThreads, 0, s>>>(m, index, n, n_dev, capacity, clear_tail ? 1 : 0);
+    launch_chained(move_fields_kernel, blocks, kMoveThreads, 0, s, m, index, n, n_dev, capacity, clear_tail ? 1 : 0);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;

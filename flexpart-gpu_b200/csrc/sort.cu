@@ -82,14 +82,15 @@ __device__ __forceinline__ uint32_t cell_key(const KeyArgs& a, uint32_t flags, i
 // through L1.  32 B a slot, HBM-bound.
 __global__ void __launch_bounds__(256) cell_key_kernel(KeyArgs a, uint32_t* __restrict__ keys,
                                                        uint32_t* __restrict__ vals) {
+    chain_begin();
     const uint32_t p = 2u * (blockIdx.x * blockDim.x + threadIdx.x);
     if (p + 1u < a.n) {
-        const uint2 f = __ldg(reinterpret_cast<const uint2*>(a.flags + p));
-        const int2 cx = __ldg(reinterpret_cast<const int2*>(a.cell_x + p));
-        const int2 cy = __ldg(reinterpret_cast<const int2*>(a.cell_y + p));
-        const float2 px = __ldg(reinterpret_cast<const float2*>(a.pos_x + p));
-        const float2 py = __ldg(reinterpret_cast<const float2*>(a.pos_y + p));
-        const float2 z = __ldg(reinterpret_cast<const float2*>(a.pos_z + p));
+        const uint2 f = *reinterpret_cast<const uint2*>(a.flags + p);
+        const int2 cx = *reinterpret_cast<const int2*>(a.cell_x + p);
+        const int2 cy = *reinterpret_cast<const int2*>(a.cell_y + p);
+        const float2 px = *reinterpret_cast<const float2*>(a.pos_x + p);
+        const float2 py = *reinterpret_cast<const float2*>(a.pos_y + p);
+        const float2 z = *reinterpret_cast<const float2*>(a.pos_z + p);
         *reinterpret_cast<uint2*>(keys + p) = make_uint2(cell_key(a, f.x, cx.x, cy.x, px.x, py.x, z.x),
                                                          cell_key(a, f.y, cx.y, cy.y, px.y, py.y, z.y));
         *reinterpret_cast<uint2*>(vals + p) = make_uint2(p, p + 1u);
@@ -166,7 +167,7 @@ extern "C" fpg_status fpg_sort_by_cell(fpg_ctx* ctx, fpg_particles* P, const fpg
     a.nx = (uint32_t)met->nx; a.ny = (uint32_t)met->ny; a.nz = (uint32_t)met->nz;
     a.lv = Levels{met->heights_dev, met->level_table_dev, met->level_inv_w, a.nz,
                   met->heights_set && met->heights[met->nz - 1] > 0.0f, level_mode(met)};
-    cell_key_kernel<<<(unsigned)(((uint64_t)n + 511u) / 512u), 256, 0, st>>>(a, s->keys[0], s->vals[0]);
+    launch_chained(cell_key_kernel, (unsigned)(((uint64_t)n + 511u) / 512u), 256, 0, st, a, s->keys[0], s->vals[0]);
     ctx->count();
     FPG_CHECK_LAUNCH();
     cub::DoubleBuffer<uint32_t> kb(s->keys[0], s->keys[1]), vb(s->vals[0], s->vals[1]);

@@ -42,6 +42,7 @@
 namespace fpg {
 
 __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
+    chain_begin();
     const Levels lv = global_levels(a);
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n) return;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
 // in a mixed population and 577 -> 479 us right after a reorder.
 template <bool kWet, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) production_step_kernel(StepArgs a) {
+    chain_begin();
     const uint32_t p = blockIdx.x * BLOCK + threadIdx.x;
     if (p < a.n) production_step<kWet>(a, p, p, a.alpha, a.counter, 0u, 0u, a.head, a.keys, true);
 }
@@ -94,6 +96,7 @@ ProductionShape production_shape_for(uint32_t n, int sm_count) {
 // arithmetic is the same, so the results are too.
 template <int BLOCK, int MINB, int PPT>
 __global__ void __launch_bounds__(BLOCK, MINB) fused_step_shape_kernel(StepArgs a) {
+    chain_begin();
     extern __shared__ float s_levels[];
     Levels lv{};
     if constexpr (PPT == 1) {
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(256) pbl_diag_kernel(const fpg_surface_cell* _
                                                        float* wstar_o, float* hmix_o, float* oli_o, float* sshf_o,
                                                        float* ssr_o, float* surfstr_o, float4* packed,
                                                        CellHanna* hanna) {
+    chain_begin();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncell) return;
     pbl_cell(s0, s1, alpha, o, c, ustar_o, wstar_o, hmix_o, oli_o, sshf_o, ssr_o, surfstr_o, packed, hanna);
@@ -424,10 +428,7 @@ extern "C" fpg_status fpg_pbl_diagnostics(fpg_ctx* ctx, const fpg_surface* surfa
     cudaStream_t s = ctx->pick(stream);
     const uint32_t n = (uint32_t)(pbl->nx * pbl->ny);
     // 64-thread CTAs spread the cells over more SMs (one cell per thread, a long dependent chain each)
-    pbl_diag_kernel<<<blocks_for(n, 64), 64, 0, s>>>(surface->frame[0], surface->frame[1], alpha, *options, n,
-                                                        pbl->field[0], pbl->field[1], pbl->field[2], pbl->field[3],
-                                                        pbl->field[4], pbl->field[5], pbl->field[6], pbl->packed,
-                                                        pbl->hanna);
+    launch_chained(pbl_diag_kernel, blocks_for(n, 64), 64, 0, s, surface->frame[0], surface->frame[1], alpha, *options, n, pbl->field[0], pbl->field[1], pbl->field[2], pbl->field[3], pbl->field[4], pbl->field[5], pbl->field[6], pbl->packed, pbl->hanna);
     ctx->count();
     FPG_CHECK_LAUNCH();
     pbl->ready = true;
@@ -645,10 +646,10 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
         a.head = philox_head(a.counter, a.key0, a.key1);
         a.keys = philox_keys(a.head);
         const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
-        (wet ? ps.wet : ps.dry)<<<blocks_for(n, ps.block), ps.block, 0, s>>>(a);
+        launch_chained(wet ? ps.wet : ps.dry, blocks_for(n, ps.block), ps.block, 0, s, a);
     } else {
         const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
-        sh.kernel<<<blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s>>>(a);
+        launch_chained(sh.kernel, blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s, a);
     }
     ctx->count();
     FPG_CHECK_LAUNCH();
@@ -799,6 +800,7 @@ struct RecordTurbArgs {
 __global__ void __launch_bounds__(256) hanna_params_kernel(SlotView v, const CellHanna* __restrict__ hcell,
                                                            uint32_t pnx, uint32_t pny,
                                                            fpg_hanna_params* __restrict__ out) {
+    chain_begin();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.n) return;
     float4* o = reinterpret_cast<float4*>(out + p);
@@ -823,6 +825,7 @@ __global__ void __launch_bounds__(256) hanna_params_kernel(SlotView v, const Cel
 // and backward loops), with the fused kernel's Philox block layout and
 // Gaussian assignment.
 __global__ void __launch_bounds__(256) langevin_record_kernel(RecordTurbArgs a) {
+    chain_begin();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.n || !(a.flags[p] & FLAG_ACTIVE)) return;
     const uint32_t n_vert = a.n_sub > 1u ? a.n_sub : 1u;
@@ -887,7 +890,7 @@ extern "C" fpg_status fpg_langevin_with_hanna(fpg_ctx* ctx, fpg_particles* P, co
     a.counter = u32x4{base_counter[0], base_counter[1], base_counter[2], base_counter[3]};
     a.key0 = key[0];
     a.key1 = key[1];
-    langevin_record_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->pick(stream)>>>(a);
+    launch_chained(langevin_record_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->pick(stream), a);
     ctx->count();
     FPG_CHECK_LAUNCH();
     if (next_counter) counter_add64(base_counter, (uint64_t)n * (n_substeps <= 2u ? 1u : 2u), next_counter);
@@ -905,8 +908,7 @@ extern "C" fpg_status fpg_dispatch_hanna_params(fpg_ctx* ctx, const fpg_particle
     if (!pbl->ready) return FPG_ERR_NOT_READY;
     const SlotView v = slot_view(P);
     if (v.n == 0) return FPG_OK;
-    hanna_params_kernel<<<(unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream)>>>(
-        v, pbl->hanna, (uint32_t)pbl->nx, (uint32_t)pbl->ny, out_dev);
+    launch_chained(hanna_params_kernel, (unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream), v, pbl->hanna, (uint32_t)pbl->nx, (uint32_t)pbl->ny, out_dev);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;
