@@ -13,6 +13,29 @@ namespace fpg {
 // caller must be 16-byte aligned (cudaMalloc gives 256).
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
 
+// Writes one record of kQuads 16-byte vectors per lane for the warp's 32
+// consecutive slots [first, first + 32), of which those below n exist:
+// through shared memory, so that every store covers whole 128-byte lines
+// (16-byte stores at the record's stride fill a sector by halves: twice the
+// L2 writes).  A lane's rows are kQuads + 1 vectors apart, which keeps both
+// the row writes and the line reads free of bank conflicts.  The whole warp
+// calls it.
+template <int kQuads>
+__device__ __forceinline__ void store_records(float4* out, size_t first, size_t n, const float4 (&row)[kQuads],
+                                              float4 (*s_rows)[kQuads + 1]) {
+    const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) s_rows[lane][k] = row[k];
+    __syncwarp();
+    const size_t end = n * kQuads;
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) {
+        const unsigned i = (unsigned)k * 32u + lane;
+        const size_t at = first * kQuads + i;
+        if (at < end) out[at] = s_rows[i / kQuads][i % kQuads];
+    }
+}
+
 struct SlotView {
     const int32_t* cell_x;
     const int32_t* cell_y;

@@ -88,6 +88,109 @@ ProductionShape production_shape_for(uint32_t n, int sm_count) {
     return production_shape<64, 24>();
 }
 
+// The seam calls of one stage each, in the same forms (advection_form,
+// turbulence_form): what a time loop that keeps the reference's separate
+// passes launches.  Issue-bound like the whole step.  Four calls of 999,983
+// slots, 30 % dead, three species: 119 -> 84 us, of 3 M 383 -> 237 us; CTAs of
+// 32 to 128 threads and 32 to 64 registers lie within 5 % of this shape.
+constexpr uint32_t kStageThreads = 64;
+
+__global__ void __launch_bounds__(kStageThreads, 18) advection_kernel(StepArgs a) {
+    chain_begin();
+    const uint32_t p = blockIdx.x * kStageThreads + threadIdx.x;
+    if (p >= a.n || !(a.flags[p] & FLAG_ACTIVE)) return;
+    const Advected r = advect_production(a, p, a.turb_u[p], a.turb_v[p], a.alpha);
+    int32_t cx, cy;
+    store_advected(a, p, r, cx, cy);
+    a.pos_z[p] = r.z;
+}
+
+__global__ void __launch_bounds__(kStageThreads, 18) turbulence_kernel(StepArgs a) {
+    chain_begin();
+    const uint32_t p = blockIdx.x * kStageThreads + threadIdx.x;
+    if (p >= a.n || !(a.flags[p] & FLAG_ACTIVE)) return;
+    const float x = (float)a.cell_x[p] + a.pos_x[p], y = (float)a.cell_y[p] + a.pos_y[p];
+    const uint32_t i = (uint32_t)clampf(x, 0.0f, (float)(a.pnx - 1u)), j = (uint32_t)clampf(y, 0.0f, (float)(a.pny - 1u));
+    float pz = a.pos_z[p];
+    turbulence_production(a, p, p, a.hcell + (i * a.pny + j), a.counter, 0u, 0u, a.head, a.keys, true, a.turb_u[p],
+                          a.turb_v[p], pz);
+}
+
+// One deposition stage with per-slot forcing: four slots per thread with
+// 16-byte accesses, a mass read only where a slot of the quad decays.  HBM
+// binds: 16 B a slot read and written, and 8 B a species.
+struct DepositArgs {
+    const uint32_t* flags;
+    const float* pos_z;                  // dry
+    const float* a0;                     // deposition velocity, or lambda
+    const float* a1;                     // precipitating fraction (wet)
+    float* prob;                         // may be NULL
+    float* mass[4];
+    int n_species;
+    uint32_t n;
+    float dt, href;
+};
+
+// The probability of one slot and its survival factor (dry_deposition.wgsl:
+// 89-105, wet_deposition.wgsl:203-216); false when the masses stay.
+template <bool kWet>
+__device__ __forceinline__ bool deposit(const DepositArgs& a, uint32_t flags, float z, float v0, float v1, float& prob,
+                                        float& survival) {
+    prob = 0.0f;
+    survival = 1.0f;
+    if (!(flags & FLAG_ACTIVE)) return false;
+    if constexpr (kWet) {
+        prob = wet_probability(v0, a.dt, v1);
+        survival = 1.0f - prob;
+        return true;
+    } else {
+        if (z >= 2.0f * a.href) return false;
+        survival = dry_survival(v0, a.dt, a.href);
+        prob = 1.0f - survival;
+        return true;
+    }
+}
+
+template <bool kWet>
+__global__ void __launch_bounds__(256) deposition_kernel(DepositArgs a) {
+    chain_begin();
+    const uint32_t p = 4u * (blockIdx.x * 256u + threadIdx.x);
+    if (p + 4u <= a.n) {
+        const uint4 f = *reinterpret_cast<const uint4*>(a.flags + p);
+        const float4 v0 = *reinterpret_cast<const float4*>(a.a0 + p);
+        float4 v1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), z = v1;
+        if constexpr (kWet) v1 = *reinterpret_cast<const float4*>(a.a1 + p);
+        else z = *reinterpret_cast<const float4*>(a.pos_z + p);
+        float4 pr, sv;
+        const bool b0 = deposit<kWet>(a, f.x, z.x, v0.x, v1.x, pr.x, sv.x);
+        const bool b1 = deposit<kWet>(a, f.y, z.y, v0.y, v1.y, pr.y, sv.y);
+        const bool b2 = deposit<kWet>(a, f.z, z.z, v0.z, v1.z, pr.z, sv.z);
+        const bool b3 = deposit<kWet>(a, f.w, z.w, v0.w, v1.w, pr.w, sv.w);
+        if (a.prob) *reinterpret_cast<float4*>(a.prob + p) = pr;
+        if (!(b0 || b1 || b2 || b3)) return;
+#pragma unroll
+        for (int k = 0; k < FPG_MAX_SPECIES; ++k) {
+            if (k >= a.n_species) break;
+            float4* at = reinterpret_cast<float4*>(a.mass[k] + p);
+            float4 m = *at;
+            m.x = b0 ? m.x * sv.x : m.x;
+            m.y = b1 ? m.y * sv.y : m.y;
+            m.z = b2 ? m.z * sv.z : m.z;
+            m.w = b3 ? m.w * sv.w : m.w;
+            *at = m;
+        }
+    } else {
+        for (uint32_t q = p; q < a.n; ++q) {
+            float pr, sv;
+            const bool b = deposit<kWet>(a, a.flags[q], kWet ? 0.0f : a.pos_z[q], a.a0[q], kWet ? a.a1[q] : 0.0f, pr, sv);
+            if (a.prob) a.prob[q] = pr;
+#pragma unroll
+            for (int k = 0; k < FPG_MAX_SPECIES; ++k)
+                if (b && k < a.n_species) a.mass[k][q] = a.mass[k][q] * sv;
+        }
+    }
+}
+
 // The same pass under another launch shape: BLOCK threads per CTA compiled
 // for MINB resident CTAs per SM, PPT particles per thread (slots of one CTA
 // are contiguous; thread t takes t, t + BLOCK, ...); with several particles
@@ -536,6 +639,51 @@ static void counter_add64(const uint32_t in[4], uint64_t off, uint32_t out[4]) {
     out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
 }
 
+namespace fpg {
+
+// The kernels for the arguments that have a form of their own; false when
+// they have none and the general body runs.
+static bool launch_form(fpg_ctx* ctx, StepArgs& a, bool no_carry, cudaStream_t s) {
+    if (a.stages & FPG_STAGE_TURBULENCE) {
+        if (!no_carry) return false;
+        a.head = philox_head(a.counter, a.key0, a.key1);
+        a.keys = philox_keys(a.head);
+    }
+    if (production_form(a)) {
+        const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
+        launch_chained(a.stages & FPG_STAGE_WET ? ps.wet : ps.dry, blocks_for(a.n, ps.block), ps.block, 0, s, a);
+        return true;
+    }
+    if (a.stages == FPG_STAGE_ADVECT && advection_form(a)) {
+        launch_chained(advection_kernel, blocks_for(a.n, kStageThreads), kStageThreads, 0, s, a);
+        return true;
+    }
+    if (a.stages == FPG_STAGE_TURBULENCE && turbulence_form(a)) {
+        launch_chained(turbulence_kernel, blocks_for(a.n, kStageThreads), kStageThreads, 0, s, a);
+        return true;
+    }
+    const bool dry = a.stages == FPG_STAGE_DRY && a.dry_mode == FPG_FORCING_PER_PARTICLE;
+    const bool wet = a.stages == FPG_STAGE_WET && a.wet_mode == FPG_FORCING_PER_PARTICLE;
+    DepositArgs d;
+    d.flags = a.flags;
+    d.pos_z = a.pos_z;
+    d.a0 = dry ? a.dry_v_arr : a.wet_l_arr;
+    d.a1 = a.wet_f_arr;
+    d.prob = dry ? a.dry_prob : a.wet_prob;
+    if ((dry || wet) && aligned16(d.a0) && (dry || aligned16(d.a1)) && aligned16(d.prob)) {
+        for (int k = 0; k < 4; ++k) d.mass[k] = a.mass[k];
+        d.n_species = a.n_species;
+        d.n = a.n;
+        d.dt = a.tdt;
+        d.href = a.href;
+        launch_chained(dry ? deposition_kernel<false> : deposition_kernel<true>, blocks_for(a.n, 1024), 256, 0, s, d);
+        return true;
+    }
+    return false;
+}
+
+}  // namespace fpg
+
 extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* met, const fpg_pbl* pbl,
                                const fpg_step_params* prm, uint32_t next_counter[4], void* stream) {
     if (!ctx || !P || !prm) return FPG_ERR_INVALID_ARGUMENT;
@@ -642,12 +790,7 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     cudaStream_t s = ctx->pick(stream);
     // no block's counter carries out of its first word
     const bool no_carry = (uint64_t)prm->counter[0] + 2u * (uint64_t)n <= (1ull << 32);
-    if (ctx->step_shape == 0 && no_carry && production_form(a)) {
-        a.head = philox_head(a.counter, a.key0, a.key1);
-        a.keys = philox_keys(a.head);
-        const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
-        launch_chained(wet ? ps.wet : ps.dry, blocks_for(n, ps.block), ps.block, 0, s, a);
-    } else {
+    if (ctx->step_shape != 0 || !launch_form(ctx, a, no_carry, s)) {
         const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
         launch_chained(sh.kernel, blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s, a);
     }
@@ -790,6 +933,8 @@ struct RecordTurbArgs {
     uint32_t n_sub;
     u32x4 counter;
     uint32_t key0, key1;
+    PhiloxHead head;
+    PhiloxKeys keys;
 };
 
 // hanna_params.wgsl:231-258 with compute_hanna (physics/hanna.rs:49-163):
@@ -797,27 +942,25 @@ struct RecordTurbArgs {
 // compute_hanna at the slot's height from its cell's Hanna constants (the
 // record the PBL pass builds from the same u*, w*, h and 1/L, with the same
 // operations as compute_hanna would, so the results are the same bits).
-__global__ void __launch_bounds__(256) hanna_params_kernel(SlotView v, const CellHanna* __restrict__ hcell,
-                                                           uint32_t pnx, uint32_t pny,
-                                                           fpg_hanna_params* __restrict__ out) {
+// Records leave through shared memory (store_records): HBM-bound, 88 B a slot.
+__global__ void __launch_bounds__(256) hanna_params_kernel(SlotView v, const CellHanna* hcell, uint32_t pnx, uint32_t pny,
+                                                           fpg_hanna_params* out) {
     chain_begin();
+    __shared__ float4 s_rows[8][32][5];
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= v.n) return;
-    float4* o = reinterpret_cast<float4*>(out + p);
-    if ((v.flags[p] & FLAG_ACTIVE) == 0u) {
-        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        o[0] = z; o[1] = z; o[2] = z; o[3] = z;
-        return;
+    float4 row[4] = {};
+    if (p < v.n && (v.flags[p] & FLAG_ACTIVE)) {
+        const CellHanna cell = ld_cell_hanna(hcell + pbl_cell_index(v, p, pnx, pny));
+        const float z = v.pos_z[p];
+        const Hanna hn = compute_hanna_cell_t<float>(cell, z);
+        // zeta and d(sigma_w^2)/dz as the CPU routine forms them (hanna.rs:55,145)
+        const float zeta = clampf(clampf(z, 0.0f, hn.h) / hn.h, 0.0f, 1.0f);
+        row[0] = make_float4(hn.ust, hn.wst, hn.ol, hn.h);
+        row[1] = make_float4(zeta, hn.sigu, hn.sigv, hn.sigw);
+        row[2] = make_float4(hn.dsigwdz, 2.0f * hn.sigw * hn.dsigwdz, hn.tlu, hn.tlv);
+        row[3] = make_float4(hn.tlw, 0.0f, 0.0f, 0.0f);
     }
-    const CellHanna cell = ld_cell_hanna(hcell + pbl_cell_index(v, p, pnx, pny));
-    const float z = v.pos_z[p];
-    const Hanna hn = compute_hanna_cell_t<float>(cell, z);
-    // zeta and d(sigma_w^2)/dz as the CPU routine forms them (hanna.rs:55,145)
-    const float zeta = clampf(clampf(z, 0.0f, hn.h) / hn.h, 0.0f, 1.0f);
-    o[0] = make_float4(hn.ust, hn.wst, hn.ol, hn.h);
-    o[1] = make_float4(zeta, hn.sigu, hn.sigv, hn.sigw);
-    o[2] = make_float4(hn.dsigwdz, 2.0f * hn.sigw * hn.dsigwdz, hn.tlu, hn.tlv);
-    o[3] = make_float4(hn.tlw, 0.0f, 0.0f, 0.0f);
+    store_records<4>(reinterpret_cast<float4*>(out), p & ~(size_t)31, v.n, row, s_rows[threadIdx.x >> 5]);
 }
 
 // langevin.wgsl:307-424: the turbulence update from a HannaParams record per
@@ -856,6 +999,79 @@ __global__ void __launch_bounds__(256) langevin_record_kernel(RecordTurbArgs a) 
     }
 }
 
+// The same for 1 to 4 sub-steps with the settings of turbulence_form, records
+// on 32-byte boundaries and a counter that does not carry: a record arrives
+// in two 32-byte loads (13 scalar ones at a 64-byte stride before), Philox
+// starts after its uniform rounds, and a record inside the bounds below runs
+// without the sanitising, which is then the identity: plain_cell's bounds on
+// the cell, sigma in [1e-3, 1e4], time scales in [1, 1e8] and a bounded
+// gradient.
+struct RecordWords { float w[16]; };
+
+__device__ __forceinline__ RecordWords ld_record(const fpg_hanna_params* r) {
+    RecordWords q;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(q.w[8 * k]), "=f"(q.w[8 * k + 1]), "=f"(q.w[8 * k + 2]), "=f"(q.w[8 * k + 3]),
+                       "=f"(q.w[8 * k + 4]), "=f"(q.w[8 * k + 5]), "=f"(q.w[8 * k + 6]), "=f"(q.w[8 * k + 7])
+                     : "l"(reinterpret_cast<const float*>(r) + 8 * k)
+                     : "memory");
+    return q;
+}
+
+__device__ __forceinline__ bool within(float v, float lo, float hi) { return v >= lo && v <= hi; }
+
+template <bool kTwoBlocks>
+__global__ void __launch_bounds__(64, 18) langevin_record_plain_kernel(RecordTurbArgs a) {
+    chain_begin();
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.n || !(a.flags[p] & FLAG_ACTIVE)) return;
+    const RecordWords q = ld_record(a.hanna + p);
+    float pz = a.pos_z[p], tu = a.turb_u[p], tv = a.turb_v[p], tw = a.turb_w[p];
+    const int32_t cbt_in = a.cbt[p];
+    int32_t cbt = cbt_in;
+    const uint32_t w = a.counter.x + p * (kTwoBlocks ? 2u : 1u);
+    const u32x4 b0 = philox_from_head(a.head, a.keys, w);
+    float2 e_uv, e_w01, e_w23 = make_float2(0.0f, 0.0f);
+    box_muller2(make_uint2(b0.x, b0.y), make_uint2(b0.z, b0.w), e_uv, e_w01);
+    if constexpr (kTwoBlocks) {
+        const u32x4 b1 = philox_from_head(a.head, a.keys, w + 1u);
+        e_w23 = box_muller_plain(b1.x, b1.y);
+    }
+    const CellHanna cell = cell_hanna(q.w[0], q.w[1], q.w[2], q.w[3]);
+    const PlainHanna horizontal{q.w[5], q.w[6], q.w[10], q.w[11]};
+    const PlainVertical vertical{q.w[7], q.w[8], q.w[12]};
+    // the reflections use the record's own h, the profiles its floor at 1 m
+    const bool plain = plain_cell(cell) && cell.h == q.w[3] && within(horizontal.sigu, 1.0e-3f, 1.0e4f) &&
+                       within(horizontal.sigv, 1.0e-3f, 1.0e4f) && within(vertical.sigw, 1.0e-3f, 1.0e4f) &&
+                       within(horizontal.tlu, 1.0f, 1.0e8f) && within(horizontal.tlv, 1.0f, 1.0e8f) &&
+                       within(vertical.tlw, 1.0f, 1.0e8f) && within(vertical.dsigwdz, -1.0e9f, 1.0e9f) &&
+                       fabsf(tu) + fabsf(tv) + fabsf(tw) < 1.0e30f && fabsf(pz) < 1.0e30f;
+    if (plain) {
+        turbulence_plain<true>(a, a.n_sub, sdiv(a.tdt, (float)a.n_sub), cell, horizontal, vertical, e_uv, e_w01, e_w23, pz,
+                               tu, tv, tw, cbt);
+    } else {
+        Hanna hn;
+        hn.ust = q.w[0]; hn.wst = q.w[1]; hn.ol = q.w[2]; hn.h = q.w[3];
+        hn.sigu = q.w[5]; hn.sigv = q.w[6]; hn.sigw = q.w[7]; hn.dsigwdz = q.w[8];
+        hn.tlu = q.w[10]; hn.tlv = q.w[11]; hn.tlw = q.w[12];
+        hn.regime = cell.kind();
+        turbulence_from_hanna<float, RecordLangevin>(a, cell, hn, e_uv, e_w01, e_w23, pz, tu, tv, tw, cbt);
+    }
+    a.turb_u[p] = tu; a.turb_v[p] = tv; a.turb_w[p] = tw;
+    a.pos_z[p] = pz;
+    if (cbt != cbt_in) a.cbt[p] = cbt;
+}
+
+// turbulence_form for a record call.
+bool record_form(const RecordTurbArgs& a, uint64_t blocks) {
+    const bool settings = a.n_sub >= 1u && a.n_sub <= 4u && a.tdt >= 1.0e-3f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f &&
+                          a.rho <= 1.0e3f && a.zmin >= 0.0f && a.zmin < 1.0f;
+    return settings && (reinterpret_cast<uintptr_t>(a.hanna) & 31u) == 0u &&
+           (uint64_t)a.counter.x + blocks * a.n <= (1ull << 32);
+}
+
 }  // namespace
 }  // namespace fpg
 
@@ -890,10 +1106,18 @@ extern "C" fpg_status fpg_langevin_with_hanna(fpg_ctx* ctx, fpg_particles* P, co
     a.counter = u32x4{base_counter[0], base_counter[1], base_counter[2], base_counter[3]};
     a.key0 = key[0];
     a.key1 = key[1];
-    launch_chained(langevin_record_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->pick(stream), a);
+    const uint64_t blocks = n_substeps <= 2u ? 1u : 2u;
+    if (record_form(a, blocks)) {
+        a.head = philox_head(a.counter, a.key0, a.key1);
+        a.keys = philox_keys(a.head);
+        launch_chained(blocks > 1u ? langevin_record_plain_kernel<true> : langevin_record_plain_kernel<false>,
+                       (unsigned)((n + 63) / 64), 64, 0, ctx->pick(stream), a);
+    } else {
+        launch_chained(langevin_record_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->pick(stream), a);
+    }
     ctx->count();
     FPG_CHECK_LAUNCH();
-    if (next_counter) counter_add64(base_counter, (uint64_t)n * (n_substeps <= 2u ? 1u : 2u), next_counter);
+    if (next_counter) counter_add64(base_counter, (uint64_t)n * blocks, next_counter);
     return FPG_OK;
 }
 

@@ -70,15 +70,22 @@ struct StepArgs {
 //   * a bounded time step and density gradient, and a reflection floor in
 //     [0, 1) m, below any mixing height (turbulence_plain);
 //   * a bracket below 4 GB (32-bit node offsets).
+inline bool advection_form(const StepArgs& a) {
+    return a.has_heights && a.level_mode == LEVELS_TABLE && (uint64_t)a.nx * a.ny * a.nz < (1ull << 27);
+}
+
+inline bool turbulence_form(const StepArgs& a) {
+    return a.n_sub == 4u && a.tdt >= 1.0e-3f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f && a.rho <= 1.0e3f &&
+           a.zmin >= 0.0f && a.zmin < 1.0f;
+}
+
 inline bool production_form(const StepArgs& a) {
     const uint32_t most = FPG_STAGE_ADVECT | FPG_STAGE_TURBULENCE | FPG_STAGE_DRY;
     const bool wet = a.stages == (most | FPG_STAGE_WET);
     if (!wet && a.stages != most) return false;
-    if (a.n_sub != 4u || a.dry_mode != FPG_FORCING_UNIFORM || a.dry_prob || a.n_species != 1) return false;
+    if (a.dry_mode != FPG_FORCING_UNIFORM || a.dry_prob || a.n_species != 1) return false;
     if (wet && (a.wet_mode != FPG_FORCING_PER_CELL || a.wet_prob || a.wnx != a.nx || a.wny != a.ny)) return false;
-    if (!a.has_heights || a.level_mode != LEVELS_TABLE || a.pnx != a.nx || a.pny != a.ny) return false;
-    if ((uint64_t)a.nx * a.ny * a.nz >= (1ull << 27)) return false;
-    return a.tdt >= 1.0e-3f && a.tdt <= 1.0e6f && a.rho >= -1.0e3f && a.rho <= 1.0e3f && a.zmin >= 0.0f && a.zmin < 1.0f;
+    return a.pnx == a.nx && a.pny == a.ny && advection_form(a) && turbulence_form(a);
 }
 
 // The search a met's heights allow (host side).
@@ -501,24 +508,40 @@ __device__ __forceinline__ void particle_step(const StepArgs& a, const Levels& l
 }
 
 
-// Turbulence of one particle with four sub-steps in a cell inside
-// plain_cell's bounds, for |tu| + |tv| + |tw| < 1e30, a finite height and
-// |rho| <= 1e3, dt <= 1e6: turbulence_update's values without its checks.
-// With u*, w* <= 1e3 and h >= 1, sigma is at most 2.5e3 and d(sigma)/dz at
-// most 6e8, so a velocity gains at most 1e19 and stays finite.  The Hanna
-// evaluation opens each sub-step, so the loop holds one copy of it.
-__device__ __forceinline__ void turbulence_plain(const StepArgs& a, const CellHanna& cell, float2 e_uv, float2 e_w01,
-                                                 float2 e_w23, float& pz, float& tu, float& tv, float& tw,
-                                                 int32_t& cbt) {
+// Turbulence of one particle in a cell inside plain_cell's bounds, for
+// n_sub in [1, 4], |tu| + |tv| + |tw| < 1e30, a finite height, |rho| <= 1e3 and
+// dt <= 1e6 (the argument block: any type with tdt, rho and zmin):
+// turbulence_update's values without its checks.  With u*, w* <= 1e3 and
+// h >= 1, sigma is at most 2.5e3 and d(sigma)/dz at most 6e8, so a velocity
+// gains at most 1e19 and stays finite.  The Hanna evaluation opens each
+// sub-step, so the loop holds one copy of it; with kGiven the first sub-step
+// and the horizontal update take the caller's parameters instead.
+struct PlainVertical { float sigw, dsigwdz, tlw; };
+
+template <bool kGiven, class A>
+__device__ __forceinline__ void turbulence_plain(const A& a, uint32_t n_sub, float dt_sub, const CellHanna& cell,
+                                                 const PlainHanna& given_h, const PlainVertical& given_v, float2 e_uv,
+                                                 float2 e_w01, float2 e_w23, float& pz, float& tu, float& tv,
+                                                 float& tw, int32_t& cbt) {
     const PlainRates rates = plain_rates(cell);
-    const float dt_sub = a.tdt * 0.25f, h = cell.h, zmin = a.zmin;
+    const float h = cell.h, zmin = a.zmin;
     float e0 = e_w01.x, e1 = e_w01.y, e2 = e_w23.x;
+    if constexpr (kGiven) plain_langevin_h(given_h, a.tdt, e_uv, tu, tv);
 #pragma unroll 1
-    for (uint32_t sub = 0; sub < 4u; ++sub) {
+    for (uint32_t sub = 0; sub < n_sub; ++sub) {
         float sigw, dsigwdz, tlw;
-        PlainHanna o;
-        plain_hanna(cell, rates, fminf(pz, h), sub == 0u, sigw, dsigwdz, tlw, o);
-        if (sub == 0u) plain_langevin_h(o, a.tdt, e_uv, tu, tv);
+        if constexpr (kGiven) {
+            if (sub == 0u) {
+                sigw = given_v.sigw; dsigwdz = given_v.dsigwdz; tlw = given_v.tlw;
+            } else {
+                PlainHanna o;
+                plain_hanna(cell, rates, pz, false, sigw, dsigwdz, tlw, o);
+            }
+        } else {
+            PlainHanna o;
+            plain_hanna(cell, rates, fminf(pz, h), sub == 0u, sigw, dsigwdz, tlw, o);
+            if (sub == 0u) plain_langevin_h(o, a.tdt, e_uv, tu, tv);
+        }
         tw = plain_langevin_v(tw, sigw, tlw, dsigwdz, dt_sub, a.rho, e0);
         e0 = e1; e1 = e2; e2 = e_w23.y;
         pz = pz + tw * dt_sub;
@@ -576,18 +599,12 @@ __device__ __forceinline__ float3 sample_production(const StepArgs& a, const Lev
     return make_float3(uv.x, uv.y, lerpf(t.w01.x, t.w01.y, alpha));
 }
 
-// particle_step for arguments in the production form: the same operations
-// with the settings known at compile time, the cell of the PBL and wet
-// lookups taken from the advected position, Philox from its uniform rounds
-// (`head` of the counter and key; `head_ok`: no block's counter carries) and
-// the turbulence without checks wherever the cell and the velocities allow.
-template <bool kWet, class Keys>
-__device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, uint32_t rng_index, float alpha,
-                                                u32x4 counter, uint32_t key0, uint32_t key1, const PhiloxHead& head,
-                                                const Keys& keys, bool head_ok) {
-    if (!(a.flags[p] & FLAG_ACTIVE)) return;
+// Petterssen advection of one particle (advection_dual_wind.wgsl:266-300) in
+// advection_form.
+struct Advected { float x, y, z, u, v, w; };
+
+__device__ __forceinline__ Advected advect_production(const StepArgs& a, uint32_t p, float tu, float tv, float alpha) {
     const Levels lv{a.heights, a.level_table, a.level_inv_w, a.nz, 1, LEVELS_TABLE};
-    float tu = a.turb_u[p], tv = a.turb_v[p];
     const float x0 = (float)a.cell_x[p] + a.pos_x[p];
     const float y0 = (float)a.cell_y[p] + a.pos_y[p];
     const float z0 = a.pos_z[p];
@@ -595,22 +612,38 @@ __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, u
     const float u0 = s0.x + tu, v0 = s0.y + tv, w0 = s0.z;
     const float xmax = (float)(a.nx - 1u), ymax = (float)(a.ny - 1u), ztop = lv.h[a.nz - 1u];
     const float3 s1 = sample_production<true>(a, lv, clampf(x0 + (u0 * a.xs) * a.dt, 0.0f, xmax),
-                                  clampf(y0 + (v0 * a.ys) * a.dt, 0.0f, ymax),
-                                  clampf(z0 + (w0 * a.zs) * a.dt, 0.0f, ztop), alpha);
-    const float cu = 0.5f * (u0 + (s1.x + tu)), cv = 0.5f * (v0 + (s1.y + tv)), cw = 0.5f * (w0 + s1.z);
-    const float x1 = clampf(x0 + (cu * a.xs) * a.dt, 0.0f, xmax);
-    const float y1 = clampf(y0 + (cv * a.ys) * a.dt, 0.0f, ymax);
-    float pz = clampf(z0 + (cw * a.zs) * a.dt, 0.0f, ztop);
-    // split_coord of a coordinate inside the grid: on the last cell the
-    // remainder is zero already
-    const int32_t cx = (int32_t)x1, cy = (int32_t)y1;
-    a.cell_x[p] = cx; a.cell_y[p] = cy;
-    a.pos_x[p] = x1 - (float)cx; a.pos_y[p] = y1 - (float)cy;
-    a.vel_u[p] = cu; a.vel_v[p] = cv; a.vel_w[p] = cw;
+                                              clampf(y0 + (v0 * a.ys) * a.dt, 0.0f, ymax),
+                                              clampf(z0 + (w0 * a.zs) * a.dt, 0.0f, ztop), alpha);
+    Advected r;
+    r.u = 0.5f * (u0 + (s1.x + tu));
+    r.v = 0.5f * (v0 + (s1.y + tv));
+    r.w = 0.5f * (w0 + s1.z);
+    r.x = clampf(x0 + (r.u * a.xs) * a.dt, 0.0f, xmax);
+    r.y = clampf(y0 + (r.v * a.ys) * a.dt, 0.0f, ymax);
+    r.z = clampf(z0 + (r.w * a.zs) * a.dt, 0.0f, ztop);
+    return r;
+}
 
-    // cell + fraction is the advected coordinate again, whose floor is the cell
-    const uint32_t c = (uint32_t)cx * a.ny + (uint32_t)cy;
-    const CellHanna cell = ld_cell_hanna(a.hcell + c);
+// The cell, fraction and velocity of an advected particle.  split_coord of a
+// coordinate inside the grid: on the last cell the remainder is zero already.
+__device__ __forceinline__ void store_advected(const StepArgs& a, uint32_t p, const Advected& r, int32_t& cx, int32_t& cy) {
+    cx = (int32_t)r.x;
+    cy = (int32_t)r.y;
+    a.cell_x[p] = cx; a.cell_y[p] = cy;
+    a.pos_x[p] = r.x - (float)cx; a.pos_y[p] = r.y - (float)cy;
+    a.vel_u[p] = r.u; a.vel_v[p] = r.v; a.vel_w[p] = r.w;
+}
+
+// The turbulence update of one particle in turbulence_form, from its cell's
+// Hanna constants: the noise from Philox's uniform rounds on (`head` of the
+// counter and key; `head_ok`: no block's counter carries) and the update
+// without checks wherever the cell and the velocities allow.
+template <class Keys>
+__device__ __forceinline__ void turbulence_production(const StepArgs& a, uint32_t p, uint32_t rng_index,
+                                                      const CellHanna* hcell, u32x4 counter, uint32_t key0,
+                                                      uint32_t key1, const PhiloxHead& head, const Keys& keys,
+                                                      bool head_ok, float tu, float tv, float& pz) {
+    const CellHanna cell = ld_cell_hanna(hcell);
     u32x4 b0, b1;
     if (head_ok) {
         const uint32_t w = counter.x + 2u * rng_index;
@@ -626,13 +659,32 @@ __device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, u
     float tw = a.turb_w[p];
     const int32_t cbt_in = a.cbt[p];
     int32_t cbt = cbt_in;
-    if (cell.plain() && fabsf(tu) + fabsf(tv) + fabsf(tw) < 1.0e30f)
-        turbulence_plain(a, cell, e_uv, e_w01, e_w23, pz, tu, tv, tw, cbt);
+    if (cell.plain() && fabsf(tu) + fabsf(tv) + fabsf(tw) < 1.0e30f && pz >= 0.0f && pz < 1.0e30f)
+        turbulence_plain<false>(a, 4u, a.tdt * 0.25f, cell, PlainHanna{}, PlainVertical{}, e_uv, e_w01, e_w23, pz, tu, tv, tw,
+                                cbt);
     else
         turbulence_update<float>(a, cell, e_uv, e_w01, e_w23, pz, tu, tv, tw, cbt);
     if (cbt != cbt_in) a.cbt[p] = cbt;
     a.turb_u[p] = tu; a.turb_v[p] = tv; a.turb_w[p] = tw;
     a.pos_z[p] = pz;
+}
+
+// particle_step for arguments in the production form: the same operations
+// with the settings known at compile time, the cell of the PBL and wet
+// lookups taken from the advected position.
+template <bool kWet, class Keys>
+__device__ __forceinline__ void production_step(const StepArgs& a, uint32_t p, uint32_t rng_index, float alpha,
+                                                u32x4 counter, uint32_t key0, uint32_t key1, const PhiloxHead& head,
+                                                const Keys& keys, bool head_ok) {
+    if (!(a.flags[p] & FLAG_ACTIVE)) return;
+    const float tu = a.turb_u[p], tv = a.turb_v[p];
+    const Advected r = advect_production(a, p, tu, tv, alpha);
+    int32_t cx, cy;
+    store_advected(a, p, r, cx, cy);
+    // cell + fraction is the advected coordinate again, whose floor is the cell
+    const uint32_t c = (uint32_t)cx * a.ny + (uint32_t)cy;
+    float pz = r.z;
+    turbulence_production(a, p, rng_index, a.hcell + c, counter, key0, key1, head, keys, head_ok, tu, tv, pz);
 
     // dry, then wet survival
     float m = a.mass[0][p];

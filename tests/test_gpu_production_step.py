@@ -6,7 +6,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from flexpart_gpu import api
+from flexpart_gpu import api, cbl
 from flexpart_gpu.records import FIELDS
 from helpers import population, production_params, small_met
 
@@ -94,6 +94,73 @@ def test_counters_at_the_edge_of_a_carry(world, counter):
     rec = _records(world[1], 1003)
     kw = dict(counter=counter, key=(0xDECAFBAD, 0x12345678))
     _same(_run(world, rec, PRODUCTION, 2, **kw), _run(world, rec, GENERAL, 2, **kw))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 63, 65, 1027])
+@pytest.mark.parametrize("species,shift,prob", [(1, 0, True), (3, 0, False), (4, 1, True)])
+def test_stage_kernels_give_the_general_bits(world, n, species, shift, prob):
+    """One stage per call; `shift` moves the per-slot forcing off 16 bytes,
+    where the general body runs."""
+    ctx, spec, m, pbl, _ = world
+    rec = _records(spec, n)
+    rng = np.random.default_rng(n)
+    rec["mass"][:, 1:species] = rng.uniform(0, 1, (n, species - 1))
+    arrays = []
+    for lo, hi in ((-1e-3, 4e-3), (-1e-4, 4e-4), (-0.2, 1.2)):
+        a = rng.uniform(lo, hi, n + shift).astype(np.float32)
+        a[shift::5] = np.resize(ODD, a[shift::5].size)
+        arrays.append(api.DeviceArray.from_numpy(ctx, a))
+
+    def run(shape):
+        p = api.Particles(ctx, n)
+        p.upload(rec)
+        out = [api.DeviceArray.from_numpy(ctx, np.full(n + shift, -7.0, np.float32)) for _ in range(2)]
+        at = [type("At", (), {"ptr": a.ptr + 4 * shift}) for a in arrays + out]
+        api.set_step_tuning(ctx, shape)
+        for k in range(2):
+            api.langevin_fused(ctx, p, pbl, 900.0, 0.0, 4, 0.01, (7, 9), [k, 0, 0, 0])
+            api.advect_dual_wind(ctx, p, m, 0.3, 900.0 * (1 - 2 * k), 2.5e-5, 1.8e-5)
+            api.langevin_fused(ctx, p, pbl, 900.0, -1e-4, 4, 0.01, (42, 0), [5 + k, 0, 0, 0])
+            api.dry_deposition(ctx, p, at[0], 900.0, 15.0, at[3] if prob else None)
+            api.wet_deposition(ctx, p, at[1], at[2], 900.0, at[4] if prob else None)
+        api.set_step_tuning(ctx, PRODUCTION)
+        return {name: p.read_field(name).view(np.uint32) for name, _ in FIELDS} | {
+            "dry": out[0].numpy().view(np.uint32), "wet": out[1].numpy().view(np.uint32)}
+
+    _same(run(PRODUCTION), run(GENERAL))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 2049])
+@pytest.mark.parametrize("n_sub", [1, 2, 3, 4])
+def test_record_kernel_gives_the_general_bits(world, n, n_sub):
+    """Records on a 32-byte boundary against the same records 16 bytes off it,
+    where the general kernel runs; some hold what no boundary layer does."""
+    ctx, spec, _, pbl, _ = world
+    rec = _records(spec, n)
+    rng = np.random.default_rng(n)
+
+    def particles():
+        p = api.Particles(ctx, n)
+        p.upload(rec)
+        return p
+
+    hanna = cbl.compute_hanna_params_gpu(ctx, particles(), pbl)
+    assert not hanna[(rec["flags"] & 1) == 0].view(np.uint32).any()
+    words = hanna.view(np.float32).reshape(n, 16)
+    at = rng.random((n, 13)) < 0.03
+    words[:, :13][at] = np.resize(ODD, int(at.sum()))
+
+    def run(offset):
+        p = particles()
+        d = api.DeviceArray.from_numpy(ctx, np.concatenate([np.zeros(offset, np.float32), words.reshape(-1)]))
+        at = api.DeviceArray.__new__(api.DeviceArray)
+        at.ctx, at.n, at.dtype, at.ptr = ctx, n, cbl.HANNA_PARAMS_DTYPE, d.ptr + 4 * offset
+        for k in range(2):
+            cbl.update_particles_turbulence_langevin_gpu(ctx, p, at, 900.0, -1e-4, n_sub, 0.01, (42, 0), [9 + k, 0, 0, 0])
+        at.ptr = None
+        return {name: p.read_field(name).view(np.uint32) for name, _ in FIELDS}
+
+    _same(run(0), run(4))
 
 
 # Philox blocks under key (42, 0) whose word (1 or 3: the angle of a pair) lies
