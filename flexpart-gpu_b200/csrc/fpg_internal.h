@@ -138,8 +138,9 @@ struct fpg_cellfield {
 struct fpg_grid {
     fpg_ctx* ctx = nullptr;
     size_t nx = 0, ny = 0, nz = 0;
-    uint32_t* counts = nullptr;
+    uint32_t* counts = nullptr;             // one block: counts, then (256-byte aligned) masses
     uint32_t* mass = nullptr;
+    size_t bytes = 0;                       // from counts to the end of the masses
     float mass_scale = 1.0e6f;
     // fpg_grid_download_async: the copy waits for `produced` (recorded on the
     // stream of the last accumulate); the next accumulate waits for `copied`.

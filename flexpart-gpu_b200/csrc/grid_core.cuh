@@ -36,12 +36,29 @@ __device__ __forceinline__ uint32_t level_sorted(float z, const float (&lower)[k
     return z == z ? k : nz - 1u;
 }
 
+// pos_z_to_level for any number of output heights in ascending order (metres):
+// the first k with z <= h[k], else the top level (also for a NaN height).
+__device__ __forceinline__ uint32_t level_bisect(float z, const float* h, uint32_t nz) {
+    uint32_t lo = 0u, hi = nz - 1u;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (z <= h[mid]) hi = mid; else lo = mid + 1u;
+    }
+    return lo;
+}
+
+// Host side: whether the output heights are metres in ascending order.
+inline int ascending_levels(const float* h, uint32_t nz) {
+    int ok = nz > 0 && h[nz - 1] > 0.0f;
+    for (uint32_t k = 1; ok && k < nz; ++k)
+        if (!(h[k] >= h[k - 1])) ok = 0;
+    return ok;
+}
+
 // Host side: whether level_sorted applies to the output heights h[0..nz)
 // (metres, ascending, at most kSortedLevels), and its padded table.
 inline int sorted_levels(const float* h, uint32_t nz, float (&lower)[kSortedLevels - 1]) {
-    int sorted = nz > 0 && nz <= kSortedLevels && h[nz - 1] > 0.0f;
-    for (uint32_t k = 1; sorted && k < nz; ++k)
-        if (!(h[k] >= h[k - 1])) sorted = 0;
+    const int sorted = nz <= kSortedLevels && ascending_levels(h, nz);
     for (uint32_t k = 0; k < kSortedLevels - 1; ++k) lower[k] = k + 1 < nz ? h[k] : INFINITY;
     return sorted;
 }
@@ -52,6 +69,12 @@ __device__ __forceinline__ uint32_t quantize(float m, float scale) {
     const float scaled = m * scale + 0.5f;
     if (scaled >= 4294967295.0f) return 0xffffffffu;
     return (uint32_t)scaled;
+}
+
+// quantize(max(m, 0)) without its branches: the conversion truncates,
+// saturates at 2^32 - 1 and takes a mass of zero (or NaN, by fmaxf) to zero.
+__device__ __forceinline__ uint32_t quantize_sat(float m, float scale) {
+    return __float2uint_rz(fmaxf(m, 0.0f) * scale + 0.5f);
 }
 
 // The CTA's table of the cells its chunk touches: open addressing on the
