@@ -83,22 +83,23 @@ __device__ __forceinline__ CblPdf cbl_pdf(float z_in, float h_in, float wst_in, 
 }
 
 // sample_cbl_vertical_velocity (physics/cbl.rs:274-288, cbl.wgsl:270-277).
-__device__ __forceinline__ float cbl_draw(const CblPdf& p, float ub, float u0, float u1) {
-    const float eta = box_muller(u0, u1).x;
+__device__ __forceinline__ float cbl_draw(const CblPdf& p, float ub, float eta) {
     return ub < p.aw ? p.am + p.as * eta : p.bm + p.bs * eta;
 }
 
-__device__ __forceinline__ void store_output(fpg_cbl_sampling_output* out, size_t i, float w, const CblPdf& p) {
-    float4* o = reinterpret_cast<float4*>(out + i);
-    o[0] = make_float4(w, p.aw, p.am, p.as);
-    o[1] = make_float4(p.bw, p.bm, p.bs, p.w2);
-    o[2] = make_float4(p.w3, p.skew, p.trans, p.zoh);
+// Three 16-byte stores per slot (moving them through shared memory into
+// whole lines measured 8 % slower: the kernel issues more than it stores).
+__device__ __forceinline__ void store_output(fpg_cbl_sampling_output* out, size_t p, const float4 (&row)[3]) {
+    float4* o = reinterpret_cast<float4*>(out + p);
+    o[0] = row[0];
+    o[1] = row[1];
+    o[2] = row[2];
 }
 
-__device__ __forceinline__ void store_zero_output(fpg_cbl_sampling_output* out, size_t i) {
-    float4* o = reinterpret_cast<float4*>(out + i);
-    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    o[0] = z; o[1] = z; o[2] = z;
+__device__ __forceinline__ void output_row(float w, const CblPdf& p, float4 (&row)[3]) {
+    row[0] = make_float4(w, p.aw, p.am, p.as);
+    row[1] = make_float4(p.bw, p.bm, p.bs, p.w2);
+    row[2] = make_float4(p.w3, p.skew, p.trans, p.zoh);
 }
 
 // cbl.wgsl:251-298: PDF from the slot's Hanna record, sample from its uniforms.
@@ -108,15 +109,15 @@ __global__ void __launch_bounds__(256) cbl_sample_kernel(SlotView v, const fpg_h
     chain_begin();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.n) return;
-    if ((v.flags[p] & FLAG_ACTIVE) == 0u) {
-        store_zero_output(out, p);
-        return;
+    float4 row[3] = {};
+    if (v.flags[p] & FLAG_ACTIVE) {
+        const float4 h0 = *reinterpret_cast<const float4*>(hanna + p);       // ust, wst, ol, h
+        const float sigw = hanna[p].sigw;
+        const float4 u = *reinterpret_cast<const float4*>(in + p);
+        const CblPdf pdf = cbl_pdf(v.pos_z[p], h0.w, h0.y, sigw, h0.z);
+        output_row(cbl_draw(pdf, u.x, box_muller(u.y, u.z).x), pdf, row);
     }
-    const float4 h0 = *reinterpret_cast<const float4*>(hanna + p);       // ust, wst, ol, h
-    const float sigw = hanna[p].sigw;
-    const float4 u = *reinterpret_cast<const float4*>(in + p);
-    const CblPdf pdf = cbl_pdf(v.pos_z[p], h0.w, h0.y, sigw, h0.z);
-    store_output(out, p, cbl_draw(pdf, u.x, u.y, u.z), pdf);
+    store_output(out, p, row);
 }
 
 // The fused form: sigma_w of compute_hanna at the slot's cell (the vertical
@@ -127,24 +128,27 @@ __global__ void __launch_bounds__(256) cbl_sample_kernel(SlotView v, const fpg_h
 // block at counter + slot: u0, u1, u2 of PhiloxRng::next_uniform4 on a
 // stream that starts at that counter (physics/cbl.rs:291-295,
 // physics/rng.rs:130-164).
-__global__ void __launch_bounds__(256) cbl_sample_philox_kernel(SlotView v, const CellHanna* __restrict__ hcell,
-                                                                uint32_t pnx, uint32_t pny, uint32_t k0,
-                                                                uint32_t k1, u32x4 counter,
-                                                                fpg_cbl_sampling_output* __restrict__ out) {
+// `head_ok`: no block's counter carries, and Philox starts after its uniform
+// rounds.
+__global__ void __launch_bounds__(256) cbl_sample_philox_kernel(SlotView v, const CellHanna* hcell, uint32_t pnx,
+                                                                uint32_t pny, uint32_t k0, uint32_t k1, u32x4 counter,
+                                                                PhiloxHead head, PhiloxKeys keys, int head_ok,
+                                                                fpg_cbl_sampling_output* out) {
     chain_begin();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= v.n) return;
-    if ((v.flags[p] & FLAG_ACTIVE) == 0u) {
-        store_zero_output(out, p);
-        return;
+    float4 row[3] = {};
+    if (v.flags[p] & FLAG_ACTIVE) {
+        const CellHanna cell = ld_cell_hanna(hcell + pbl_cell_index(v, p, pnx, pny));
+        const float z = v.pos_z[p];
+        float sigw, dsigwdz, tlw;
+        hanna_short_cell_t<float>(cell, z, sigw, dsigwdz, tlw);
+        const u32x4 b = head_ok ? philox_from_head(head, keys, counter.x + (uint32_t)p)
+                                : philox4x32_10(counter_add(counter, (uint32_t)p), k0, k1);
+        const CblPdf pdf = cbl_pdf(z, cell.h, cell.wst, sigw, cell.ol);
+        output_row(cbl_draw(pdf, u32_to_uniform01(b.x), box_muller_plain(b.y, b.z).x), pdf, row);
     }
-    const CellHanna cell = ld_cell_hanna(hcell + pbl_cell_index(v, p, pnx, pny));
-    const float z = v.pos_z[p];
-    float sigw, dsigwdz, tlw;
-    hanna_short_cell_t<float>(cell, z, sigw, dsigwdz, tlw);
-    const u32x4 b = philox4x32_10(counter_add(counter, (uint32_t)p), k0, k1);
-    const CblPdf pdf = cbl_pdf(z, cell.h, cell.wst, sigw, cell.ol);
-    store_output(out, p, cbl_draw(pdf, u32_to_uniform01(b.x), u32_to_uniform01(b.y), u32_to_uniform01(b.z)), pdf);
+    store_output(out, p, row);
 }
 
 // expected_destination_height_m (physics/convection.rs:398-427): one thread
@@ -152,8 +156,7 @@ __global__ void __launch_bounds__(256) cbl_sample_philox_kernel(SlotView v, cons
 // shader's per-particle loop does (convective_mixing.wgsl:98-104), then
 // clamps to the column (the shader's clamp of the quotient).
 __global__ void conv_heights_kernel(uint32_t L, const float* __restrict__ m, const float* __restrict__ centers,
-                                    float z_min, float z_max, float* __restrict__ heights,
-                                    uint32_t* __restrict__ has_weight) {
+                                    float z_min, float z_max, float* __restrict__ heights) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= L) return;
     float wh = 0.0f, ws = 0.0f;
@@ -163,88 +166,95 @@ __global__ void conv_heights_kernel(uint32_t L, const float* __restrict__ m, con
         wh = wh + w * centers[d];
         ws = ws + w;
     }
-    has_weight[s] = ws > 0.0f ? 1u : 0u;
     heights[s] = ws > 0.0f ? clampf(wh / ws, z_min, z_max) : 0.0f;
 }
 
 // convective_mixing.wgsl:87-113 per active slot.  With strictly increasing
 // finite interfaces the shader's linear scan (first level with
 // lower <= z < upper, else the top level) is the last level whose lower
-// interface is <= z, found by bisection; otherwise the scan itself runs.
-template <bool kSorted>
-__device__ __forceinline__ uint32_t source_level(float z, uint32_t L, const float* __restrict__ iface) {
-    if constexpr (kSorted) {
-        uint32_t lo = 0u, hi = L;                 // count of iface[0..L) <= z lies in [1, L]
+// interface is <= z: a bucket table gives a level at most a few below it
+// (entry b is the last level whose lower interface lies at or below the lower
+// edge of bucket b - 1, so rounding of the bucket index cannot pass it) and
+// the search scans up, one comparison or two where a bisection of 60 levels
+// takes six dependent loads.  A column whose bucket width is not a normal
+// float is bisected; otherwise the scan itself runs.
+enum { MIX_SCAN = 0, MIX_BISECT = 1, MIX_TABLE = 2 };
+constexpr uint32_t kMixBuckets = 1024;
+
+struct MixColumn {
+    const float* iface;                  // L + 1
+    const float* heights;                // L: the mixed height of every source level
+    const uint16_t* table;               // kMixBuckets
+    float inv_w;
+    uint32_t L;
+};
+
+template <int kSearch>
+__device__ __forceinline__ uint32_t source_level(float z, float z_min, const MixColumn& c) {
+    if constexpr (kSearch == MIX_TABLE) {
+        const uint32_t b = min(__float2uint_rz((z - z_min) * c.inv_w), kMixBuckets - 1u);
+        uint32_t lo = __ldg(c.table + b);
+        while (lo + 1u < c.L && __ldg(c.iface + lo + 1u) <= z) ++lo;
+        return lo;
+    } else if constexpr (kSearch == MIX_BISECT) {
+        uint32_t lo = 0u, hi = c.L;               // count of iface[0..L) <= z lies in [1, L]
         while (hi - lo > 1u) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(iface + mid) <= z) lo = mid; else hi = mid;
+            if (__ldg(c.iface + mid) <= z) lo = mid; else hi = mid;
         }
         return lo;
     } else {
-        for (uint32_t l = 0; l < L; ++l)
-            if (z >= __ldg(iface + l) && z < __ldg(iface + l + 1u)) return l;
-        return L - 1u;
+        for (uint32_t l = 0; l < c.L; ++l)
+            if (z >= __ldg(c.iface + l) && z < __ldg(c.iface + l + 1u)) return l;
+        return c.L - 1u;
     }
 }
 
-// The mixed height and the source level of one active slot.
-template <bool kSorted>
-__device__ __forceinline__ float mix_height(float z_in, uint32_t L, const float* __restrict__ iface,
-                                            const float* __restrict__ heights,
-                                            const uint32_t* __restrict__ has_weight, float z_min, float z_max,
-                                            int32_t& level_out) {
-    const float z = clampf(z_in, z_min, z_max);
-    const uint32_t level = source_level<kSorted>(z, L, iface);
+// The mixed height and the source level of one active slot (a column that
+// passed fpg_convection_set_matrix always has a positive weight).
+template <int kSearch>
+__device__ __forceinline__ float mix_height(float z_in, float z_min, float z_max, const MixColumn& c, int32_t& level_out) {
+    const uint32_t level = source_level<kSearch>(clampf(z_in, z_min, z_max), z_min, c);
     level_out = (int32_t)level;
-    return __ldg(has_weight + level) ? __ldg(heights + level) : z;
-}
-
-template <bool kSorted>
-__device__ __forceinline__ void mix_slot(size_t p, float z_in, float* __restrict__ pos_z, int32_t* __restrict__ cbt,
-                                         uint32_t L, const float* __restrict__ iface,
-                                         const float* __restrict__ heights, const uint32_t* __restrict__ has_weight,
-                                         float z_min, float z_max) {
-    int32_t level;
-    pos_z[p] = mix_height<kSorted>(z_in, L, iface, heights, has_weight, z_min, z_max, level);
-    cbt[p] = level;
+    return __ldg(c.heights + level);
 }
 
 // Four slots per thread: the flags and heights of a quad arrive in one
 // 16-byte load each (the fields are 256-byte aligned); a quad of active
 // slots is written with one 16-byte store per field, otherwise only the
 // active slots are written.  The last n % 4 slots take scalar loads.
-template <bool kSorted>
-__global__ void __launch_bounds__(256) conv_apply_kernel(size_t n, const uint32_t* flags,
-                                                         float* pos_z, int32_t* cbt,
-                                                         uint32_t L, const float* __restrict__ iface,
-                                                         const float* __restrict__ heights,
-                                                         const uint32_t* __restrict__ has_weight) {
+template <int kSearch>
+__global__ void __launch_bounds__(256) conv_apply_kernel(size_t n, const uint32_t* flags, float* pos_z, int32_t* cbt,
+                                                         MixColumn c) {
     chain_begin();
     const size_t p0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4u;
     if (p0 >= n) return;
-    const float z_min = __ldg(iface), z_max = __ldg(iface + L);
+    const float z_min = __ldg(c.iface), z_max = __ldg(c.iface + c.L);
     if (p0 + 4u <= n) {
         const uint4 f = *reinterpret_cast<const uint4*>(flags + p0);
         const float4 z = *reinterpret_cast<const float4*>(pos_z + p0);
+        int4 lv;
+        float4 zo;
+        zo.x = mix_height<kSearch>(z.x, z_min, z_max, c, lv.x);
+        zo.y = mix_height<kSearch>(z.y, z_min, z_max, c, lv.y);
+        zo.z = mix_height<kSearch>(z.z, z_min, z_max, c, lv.z);
+        zo.w = mix_height<kSearch>(z.w, z_min, z_max, c, lv.w);
         if (f.x & f.y & f.z & f.w & FLAG_ACTIVE) {
-            int4 lv;
-            float4 zo;
-            zo.x = mix_height<kSorted>(z.x, L, iface, heights, has_weight, z_min, z_max, lv.x);
-            zo.y = mix_height<kSorted>(z.y, L, iface, heights, has_weight, z_min, z_max, lv.y);
-            zo.z = mix_height<kSorted>(z.z, L, iface, heights, has_weight, z_min, z_max, lv.z);
-            zo.w = mix_height<kSorted>(z.w, L, iface, heights, has_weight, z_min, z_max, lv.w);
             *reinterpret_cast<float4*>(pos_z + p0) = zo;
             *reinterpret_cast<int4*>(cbt + p0) = lv;
             return;
         }
-        if (f.x & FLAG_ACTIVE) mix_slot<kSorted>(p0, z.x, pos_z, cbt, L, iface, heights, has_weight, z_min, z_max);
-        if (f.y & FLAG_ACTIVE) mix_slot<kSorted>(p0 + 1, z.y, pos_z, cbt, L, iface, heights, has_weight, z_min, z_max);
-        if (f.z & FLAG_ACTIVE) mix_slot<kSorted>(p0 + 2, z.z, pos_z, cbt, L, iface, heights, has_weight, z_min, z_max);
-        if (f.w & FLAG_ACTIVE) mix_slot<kSorted>(p0 + 3, z.w, pos_z, cbt, L, iface, heights, has_weight, z_min, z_max);
+        if (f.x & FLAG_ACTIVE) { pos_z[p0] = zo.x; cbt[p0] = lv.x; }
+        if (f.y & FLAG_ACTIVE) { pos_z[p0 + 1] = zo.y; cbt[p0 + 1] = lv.y; }
+        if (f.z & FLAG_ACTIVE) { pos_z[p0 + 2] = zo.z; cbt[p0 + 2] = lv.z; }
+        if (f.w & FLAG_ACTIVE) { pos_z[p0 + 3] = zo.w; cbt[p0 + 3] = lv.w; }
     } else {
         for (size_t p = p0; p < n; ++p)
-            if (flags[p] & FLAG_ACTIVE)
-                mix_slot<kSorted>(p, pos_z[p], pos_z, cbt, L, iface, heights, has_weight, z_min, z_max);
+            if (flags[p] & FLAG_ACTIVE) {
+                int32_t level;
+                pos_z[p] = mix_height<kSearch>(pos_z[p], z_min, z_max, c, level);
+                cbt[p] = level;
+            }
     }
 }
 
@@ -260,8 +270,9 @@ struct fpg_convection {
     float* iface = nullptr;         // levels + 1
     float* centers = nullptr;       // levels
     float* heights = nullptr;       // levels: expected destination height per source level
-    uint32_t* has_weight = nullptr; // levels
-    bool sorted = true;
+    uint16_t* table = nullptr;      // kMixBuckets: the level search (MIX_TABLE)
+    float inv_w = 0.0f;
+    int search = MIX_SCAN;
     bool ready = false;
 };
 
@@ -293,7 +304,10 @@ extern "C" fpg_status fpg_cbl_sample_philox(fpg_ctx* ctx, const fpg_particles* P
     if (v.n == 0) return FPG_OK;
     if (!out_dev || !aligned16(out_dev)) return FPG_ERR_INVALID_ARGUMENT;
     const u32x4 c{counter[0], counter[1], counter[2], counter[3]};
-    launch_chained(cbl_sample_philox_kernel, (unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream), v, pbl->hanna, (uint32_t)pbl->nx, (uint32_t)pbl->ny, key[0], key[1], c, out_dev);
+    const PhiloxHead head = philox_head(c, key[0], key[1]);
+    const int head_ok = (uint64_t)c.x + v.n <= (1ull << 32);
+    launch_chained(cbl_sample_philox_kernel, (unsigned)((v.n + 255) / 256), 256, 0, ctx->pick(stream), v, pbl->hanna,
+                   (uint32_t)pbl->nx, (uint32_t)pbl->ny, key[0], key[1], c, head, philox_keys(head), head_ok, out_dev);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;
@@ -313,7 +327,7 @@ extern "C" fpg_status fpg_convection_create(fpg_ctx* ctx, size_t level_count, fp
     if (e == cudaSuccess) e = cudaMalloc(&c->iface, (L + 1) * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&c->centers, L * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&c->heights, L * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&c->has_weight, L * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&c->table, kMixBuckets * sizeof(uint16_t));
     if (e != cudaSuccess) {
         fpg_convection_destroy(c);
         return cuda_status(e);
@@ -328,7 +342,7 @@ extern "C" fpg_status fpg_convection_destroy(fpg_convection* c) {
     cudaFree(c->iface);
     cudaFree(c->centers);
     cudaFree(c->heights);
-    cudaFree(c->has_weight);
+    cudaFree(c->table);
     delete c;
     return FPG_OK;
 }
@@ -360,18 +374,34 @@ extern "C" fpg_status fpg_convection_set_matrix(fpg_convection* c, const float* 
     // level_centers_from_interfaces (src/gpu/convection.rs:63-69)
     std::vector<float> centers(L);
     for (size_t l = 0; l < L; ++l) centers[l] = 0.5f * (level_interfaces_m[l] + level_interfaces_m[l + 1]);
+    // the bucket table, in double
+    std::vector<uint16_t> table(kMixBuckets);
+    int search = sorted ? MIX_BISECT : MIX_SCAN;
+    const double span = (double)level_interfaces_m[L] - (double)level_interfaces_m[0];
+    const float inv_w = sorted ? (float)(kMixBuckets / span) : 0.0f;
+    if (sorted && std::isnormal(inv_w) && std::isfinite((float)span)) {
+        search = MIX_TABLE;
+        size_t l = 0;
+        for (uint32_t b = 0; b < kMixBuckets; ++b) {
+            const double edge = (double)level_interfaces_m[0] + ((double)b - 1.0) * (span / kMixBuckets);
+            while (l + 1 < L && (double)level_interfaces_m[l + 1] <= edge) ++l;
+            table[b] = (uint16_t)l;
+        }
+    }
     cudaStream_t s = c->ctx->pick(stream);
+    FPG_CUDA(cudaMemcpyAsync(c->table, table.data(), kMixBuckets * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(c->matrix, matrix_column_major, L * L * sizeof(float), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(c->iface, level_interfaces_m, (L + 1) * sizeof(float), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(c->centers, centers.data(), L * sizeof(float), cudaMemcpyHostToDevice, s));
     conv_heights_kernel<<<(unsigned)((L + 127) / 128), 128, 0, s>>>((uint32_t)L, c->matrix, c->centers,
                                                                    level_interfaces_m[0], level_interfaces_m[L],
-                                                                   c->heights, c->has_weight);
+                                                                   c->heights);
     c->ctx->count();
     FPG_CHECK_LAUNCH();
-    // the host vector is released on return: wait for its copy
+    // the host vectors are released on return: wait for their copies
     FPG_CUDA(cudaStreamSynchronize(s));
-    c->sorted = sorted;
+    c->search = search;
+    c->inv_w = inv_w;
     c->ready = true;
     return FPG_OK;
 }
@@ -393,10 +423,11 @@ extern "C" fpg_status fpg_convective_mixing(fpg_ctx* ctx, fpg_particles* P, cons
     auto* pos_z = static_cast<float*>(P->field[FPG_FIELD_POS_Z]);
     auto* cbt = static_cast<int32_t*>(P->field[FPG_FIELD_CBT]);
     const unsigned grid = (unsigned)(((n + 3) / 4 + 255) / 256);
-    if (c->sorted)
-        launch_chained(conv_apply_kernel<true>, grid, 256, 0, ctx->pick(stream), n, flags, pos_z, cbt, (uint32_t)c->levels, c->iface, c->heights, c->has_weight);
-    else
-        launch_chained(conv_apply_kernel<false>, grid, 256, 0, ctx->pick(stream), n, flags, pos_z, cbt, (uint32_t)c->levels, c->iface, c->heights, c->has_weight);
+    const MixColumn column{c->iface, c->heights, c->table, c->inv_w, (uint32_t)c->levels};
+    const auto kernel = c->search == MIX_TABLE    ? conv_apply_kernel<MIX_TABLE>
+                        : c->search == MIX_BISECT ? conv_apply_kernel<MIX_BISECT>
+                                                  : conv_apply_kernel<MIX_SCAN>;
+    launch_chained(kernel, grid, 256, 0, ctx->pick(stream), n, flags, pos_z, cbt, column);
     ctx->count();
     FPG_CHECK_LAUNCH();
     return FPG_OK;
