@@ -165,18 +165,22 @@ struct TapeRec {
 // whose last receptor hit came before this step has a zero adjoint from this
 // step on, so its tape is never read -- it is marked inactive for the
 // reverse and not stepped.
-// One CTA per 256-slot work item, launched over all items; the level arrays
-// are read from global memory (no staging, no barrier).
-__global__ void __launch_bounds__(256, 4) inverse_tape_kernel(StepArgs a, const BatchState* st,
+// kTapeParts CTAs per 256-slot work item, launched over all items; the level
+// arrays are read from global memory (no staging, no barrier).  Small CTAs
+// fill the last wave: 160 k particles are 625 items, one more than the 592
+// CTAs of 256 threads that are resident (13.6 us a step, @@ with 64 threads).
+constexpr uint32_t kTapeThreads = 64, kTapeParts = TILE / kTapeThreads;
+
+__global__ void __launch_bounds__(kTapeThreads, 16) inverse_tape_kernel(StepArgs a, const BatchState* st,
                                                               const ScenDev* sc,
                                                               const uint2* __restrict__ items, uint32_t n_items,
                                                               TapeBase tb, uint32_t every,
                                                               const uint32_t* live) {
     chain_begin();
-    if (blockIdx.x >= n_items) return;
-    const uint2 w = items[blockIdx.x];
+    if (blockIdx.x / kTapeParts >= n_items) return;
+    const uint2 w = items[blockIdx.x / kTapeParts];
     const ScenDev& d = sc[w.x];
-    const uint32_t local = w.y + threadIdx.x;
+    const uint32_t local = w.y + blockIdx.x % kTapeParts * kTapeThreads + threadIdx.x;
     if (local >= d.released) return;
     const uint32_t slice = st->step % tb.slices;
     TapeRec rec;
@@ -383,32 +387,131 @@ __device__ __forceinline__ void receptor_seed(const Receptors& r, uint32_t inst,
         }
 }
 
-// The reverse of step `slice`'s tape.  One work item is 256 slots of one
-// scenario, so a warp's lanes share the scenario: the release gradients are
-// summed across the warp first.
-__global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, const BatchState* st,
-                                                                 const ScenDev* sc,
+// The adjoint state of one slot.
+struct Lam { float x, y, z, tu, tv, tw, m; };
+
+__device__ __forceinline__ Lam ld_lam(const LamArrays& l, uint32_t p) {
+    return Lam{l.f[L_X][p], l.f[L_Y][p], l.f[L_Z][p], l.f[L_TU][p], l.f[L_TV][p], l.f[L_TW][p], l.f[L_M][p]};
+}
+
+__device__ __forceinline__ void st_lam(const LamArrays& l, uint32_t p, const Lam& v) {
+    l.f[L_X][p] = v.x; l.f[L_Y][p] = v.y; l.f[L_Z][p] = v.z;
+    l.f[L_TU][p] = v.tu; l.f[L_TV][p] = v.tv; l.f[L_TW][p] = v.tw;
+    l.f[L_M][p] = v.m;
+}
+
+// The reverse of one step for the CTA's 256 slots of one scenario (a warp's
+// lanes share the scenario: the release gradients are summed across the warp
+// first).  `lam` is the state after the step for valid lanes and becomes the
+// state before it.  The whole warp calls it.
+__device__ __forceinline__ void reverse_step(const StepArgs& a, const Levels& lvl, const BatchState* st, const ScenDev& d,
+                                             uint32_t scen, uint32_t local, uint32_t p, uint32_t fl,
+                                             const TapeArrays& tape, Lam& lam, const Receptors& r, double* dbias,
+                                             double* dsrc, const BiasTable& table) {
+    const bool valid = (fl & TAPE_ACTIVE) != 0u;
+    const float alpha = st->alpha;
+    const bool output = r.every != 0 && (st->step + 1u) % r.every == 0u;
+    const float kx = a.xs * a.dt, ky = a.ys * a.dt, kz = a.zs * a.dt;
+    float lx = 0.0f, ly = 0.0f, lz = 0.0f, ltu = 0.0f, ltv = 0.0f, ltw = 0.0f, lm = 0.0f;
+    float zz = 0.0f, ztw = 0.0f, wz = 0.0f, wtw = 0.0f, uz = 0.0f, uu = 0.0f, vz = 0.0f, vv = 0.0f;
+    float px = 0.0f, py = 0.0f, pz = 0.0f, x0 = 0.0f, y0 = 0.0f, z0 = 0.0f;
+    if (valid) {
+        lx = lam.x; ly = lam.y; lz = lam.z;
+        ltu = lam.tu; ltv = lam.tv; ltw = lam.tw;
+        lm = lam.m;
+        if (output) {
+            // the receptor term of this step's output state
+            float sx, sy, sz, sm;
+            receptor_seed(r, d.instance, tape.f[T_X2][p], tape.f[T_Y2][p], tape.f[T_Z2][p], tape.f[T_M2][p], sx, sy, sz,
+                          sm);
+            lx += sx; ly += sy; lz += sz; lm += sm;
+        }
+        lm = lm * tape.f[T_SURV][p];
+        zz = tape.f[T_ZZ][p]; ztw = tape.f[T_ZTW][p]; wz = tape.f[T_WZ][p]; wtw = tape.f[T_WTW][p];
+        uz = tape.f[T_UZ][p]; uu = tape.f[T_UU][p]; vz = tape.f[T_VZ][p]; vv = tape.f[T_VV][p];
+        px = tape.f[T_PX][p]; py = tape.f[T_PY][p]; pz = tape.f[T_PZ][p];
+        x0 = tape.f[T_X0][p]; y0 = tape.f[T_Y0][p]; z0 = tape.f[T_Z0][p];
+    }
+    // turbulence: (z1, tu, tv, tw) -> (z2, tu', tv', tw')
+    const float lz1 = lz * zz + ltw * wz + ltu * uz + ltv * vz;
+    const float ltw0 = lz * ztw + ltw * wtw;
+    float ltu0 = ltu * uu;
+    float ltv0 = ltv * vv;
+    // advection: x1 = clamp(x0 + cu kx), cu = (u0 + u1) / 2, u0 = s0.u + tu, u1 = s1.u + tu
+    const float gx1 = (fl & ADV_X1) ? lx : 0.0f;
+    const float gy1 = (fl & ADV_Y1) ? ly : 0.0f;
+    const float gz1 = (fl & ADV_Z1) ? lz1 : 0.0f;
+    float lx0 = gx1, ly0 = gy1, lz0 = gz1;
+    float lu0 = 0.5f * gx1 * kx, lv0 = 0.5f * gy1 * ky, lw0 = 0.5f * gz1 * kz;
+    const float lu1 = lu0, lv1 = lv0, lw1 = lw0;
+    ltu0 += lu1;
+    ltv0 += lv1;
+    const float3 g1 = sample_vjp(a, lvl, valid, px, py, pz, alpha, lu1, lv1, lw1, dbias, table);
+    const float gpx = (fl & ADV_PX) ? g1.x : 0.0f;
+    const float gpy = (fl & ADV_PY) ? g1.y : 0.0f;
+    const float gpz = (fl & ADV_PZ) ? g1.z : 0.0f;
+    lx0 += gpx; lu0 += gpx * kx;
+    ly0 += gpy; lv0 += gpy * ky;
+    lz0 += gpz; lw0 += gpz * kz;
+    ltu0 += lu0;
+    ltv0 += lv0;
+    const float3 g0 = sample_vjp(a, lvl, valid, x0, y0, z0, alpha, lu0, lv0, lw0, dbias, table);
+    lx0 += g0.x; ly0 += g0.y; lz0 += g0.z;
+    if (valid) lam = Lam{lx0, ly0, lz0, ltu0, ltv0, ltw0, lm};
+    // released this step: the adjoint is the gradient of the release state
+    const bool rel = valid && local >= d.rel_lo && local < d.rel_hi;
+    if (__ballot_sync(0xffffffffu, rel)) {
+        const float sx = warp_sum(rel ? lx0 : 0.0f), sy = warp_sum(rel ? ly0 : 0.0f);
+        const float sz = warp_sum(rel ? lz0 : 0.0f), sm = warp_sum(rel ? lm : 0.0f);
+        if ((threadIdx.x & 31u) == 0u) {
+            double* g = dsrc + 4u * scen;
+            atomicAdd(g + 0, (double)sx);
+            atomicAdd(g + 1, (double)sy);
+            atomicAdd(g + 2, (double)sz);
+            atomicAdd(g + 3, (double)sm);
+        }
+    }
+}
+
+__device__ __forceinline__ void clear_bias_table(uint32_t* key, float* g) {
+    for (uint32_t i = threadIdx.x; i < kBiasTable; i += blockDim.x) {
+        key[i] = kBiasEmpty;
+        g[3u * i] = 0.0f;
+        g[3u * i + 1u] = 0.0f;
+        g[3u * i + 2u] = 0.0f;
+    }
+}
+
+// Adds the table to the gradient and empties it.
+__device__ __forceinline__ void flush_bias_table(uint32_t* key, float* g, double* dbias) {
+    for (uint32_t i = threadIdx.x; i < kBiasTable; i += blockDim.x) {
+        const uint32_t n = key[i];
+        if (n == kBiasEmpty) continue;
+        atomicAdd(dbias + 3u * n + 0u, (double)g[3u * i]);
+        atomicAdd(dbias + 3u * n + 1u, (double)g[3u * i + 1u]);
+        atomicAdd(dbias + 3u * n + 2u, (double)g[3u * i + 2u]);
+        key[i] = kBiasEmpty;
+        g[3u * i] = 0.0f;
+        g[3u * i + 1u] = 0.0f;
+        g[3u * i + 2u] = 0.0f;
+    }
+}
+
+// The reverse of step `slice`'s tape over all items: persistent CTAs, one
+// bias table per CTA for all of its items.
+__global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, const BatchState* st, const ScenDev* sc,
                                                                  const uint2* __restrict__ items, uint32_t n_items,
                                                                  uint32_t* work, TapeBase tb, uint32_t slice,
-                                                                 LamArrays lam, Receptors r,
-                                                                 double* __restrict__ dbias,
-                                                                 double* __restrict__ dsrc) {
+                                                                 LamArrays lam, Receptors r, double* dbias,
+                                                                 double* dsrc) {
     chain_begin();
     extern __shared__ float s_levels[];
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_bias_key[kBiasTable];
     __shared__ float s_bias_g[3 * kBiasTable];
     const Levels lvl = stage_levels(a, s_levels);
-    for (uint32_t i = threadIdx.x; i < kBiasTable; i += blockDim.x) {
-        s_bias_key[i] = kBiasEmpty;
-        s_bias_g[3u * i] = 0.0f;
-        s_bias_g[3u * i + 1u] = 0.0f;
-        s_bias_g[3u * i + 2u] = 0.0f;
-    }
+    clear_bias_table(s_bias_key, s_bias_g);
     const BiasTable table{s_bias_key, s_bias_g};
-    const float alpha = st->alpha;
-    const bool output = r.every != 0 && (st->step + 1u) % r.every == 0u;
-    const float kx = a.xs * a.dt, ky = a.ys * a.dt, kz = a.zs * a.dt;
     TapeArrays tape;
 #pragma unroll
     for (int f = 0; f < TAPE_FIELDS; ++f) tape.f[f] = tb.field(slice, f);
@@ -425,82 +528,70 @@ __global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, con
         const uint32_t fl = local < d.released ? reinterpret_cast<const uint32_t*>(tape.f[T_FLAGS])[p] : 0u;
         const bool valid = (fl & TAPE_ACTIVE) != 0u;
         if (__ballot_sync(0xffffffffu, valid) == 0u) continue;
-        float lx = 0.0f, ly = 0.0f, lz = 0.0f, ltu = 0.0f, ltv = 0.0f, ltw = 0.0f, lm = 0.0f;
-        float zz = 0.0f, ztw = 0.0f, wz = 0.0f, wtw = 0.0f, uz = 0.0f, uu = 0.0f, vz = 0.0f, vv = 0.0f;
-        float px = 0.0f, py = 0.0f, pz = 0.0f, x0 = 0.0f, y0 = 0.0f, z0 = 0.0f;
-        if (valid) {
-            lx = lam.f[L_X][p]; ly = lam.f[L_Y][p]; lz = lam.f[L_Z][p];
-            ltu = lam.f[L_TU][p]; ltv = lam.f[L_TV][p]; ltw = lam.f[L_TW][p];
-            lm = lam.f[L_M][p];
-            if (output) {
-                // the receptor term of this step's output state
-                float sx, sy, sz, sm;
-                receptor_seed(r, d.instance, tape.f[T_X2][p], tape.f[T_Y2][p], tape.f[T_Z2][p], tape.f[T_M2][p],
-                              sx, sy, sz, sm);
-                lx += sx; ly += sy; lz += sz; lm += sm;
-            }
-            lm = lm * tape.f[T_SURV][p];
-            zz = tape.f[T_ZZ][p]; ztw = tape.f[T_ZTW][p]; wz = tape.f[T_WZ][p]; wtw = tape.f[T_WTW][p];
-            uz = tape.f[T_UZ][p]; uu = tape.f[T_UU][p]; vz = tape.f[T_VZ][p]; vv = tape.f[T_VV][p];
-            px = tape.f[T_PX][p]; py = tape.f[T_PY][p]; pz = tape.f[T_PZ][p];
-            x0 = tape.f[T_X0][p]; y0 = tape.f[T_Y0][p]; z0 = tape.f[T_Z0][p];
-        }
-        // turbulence: (z1, tu, tv, tw) -> (z2, tu', tv', tw')
-        const float lz1 = lz * zz + ltw * wz + ltu * uz + ltv * vz;
-        const float ltw0 = lz * ztw + ltw * wtw;
-        float ltu0 = ltu * uu;
-        float ltv0 = ltv * vv;
-        // advection: x1 = clamp(x0 + cu kx), cu = (u0 + u1) / 2, u0 = s0.u + tu, u1 = s1.u + tu
-        const float gx1 = (fl & ADV_X1) ? lx : 0.0f;
-        const float gy1 = (fl & ADV_Y1) ? ly : 0.0f;
-        const float gz1 = (fl & ADV_Z1) ? lz1 : 0.0f;
-        float lx0 = gx1, ly0 = gy1, lz0 = gz1;
-        float lu0 = 0.5f * gx1 * kx, lv0 = 0.5f * gy1 * ky, lw0 = 0.5f * gz1 * kz;
-        const float lu1 = lu0, lv1 = lv0, lw1 = lw0;
-        ltu0 += lu1;
-        ltv0 += lv1;
-        const float3 g1 = sample_vjp(a, lvl, valid, px, py, pz, alpha, lu1, lv1, lw1, dbias, table);
-        const float gpx = (fl & ADV_PX) ? g1.x : 0.0f;
-        const float gpy = (fl & ADV_PY) ? g1.y : 0.0f;
-        const float gpz = (fl & ADV_PZ) ? g1.z : 0.0f;
-        lx0 += gpx; lu0 += gpx * kx;
-        ly0 += gpy; lv0 += gpy * ky;
-        lz0 += gpz; lw0 += gpz * kz;
-        ltu0 += lu0;
-        ltv0 += lv0;
-        const float3 g0 = sample_vjp(a, lvl, valid, x0, y0, z0, alpha, lu0, lv0, lw0, dbias, table);
-        lx0 += g0.x; ly0 += g0.y; lz0 += g0.z;
-        if (valid) {
-            lam.f[L_X][p] = lx0; lam.f[L_Y][p] = ly0; lam.f[L_Z][p] = lz0;
-            lam.f[L_TU][p] = ltu0; lam.f[L_TV][p] = ltv0; lam.f[L_TW][p] = ltw0;
-            lam.f[L_M][p] = lm;
-        }
-        // released this step: the adjoint is the gradient of the release state
-        const bool rel = valid && local >= d.rel_lo && local < d.rel_hi;
-        if (__ballot_sync(0xffffffffu, rel)) {
-            const float sx = warp_sum(rel ? lx0 : 0.0f), sy = warp_sum(rel ? ly0 : 0.0f);
-            const float sz = warp_sum(rel ? lz0 : 0.0f), sm = warp_sum(rel ? lm : 0.0f);
-            if ((threadIdx.x & 31u) == 0u) {
-                double* g = dsrc + 4u * w.x;
-                atomicAdd(g + 0, (double)sx);
-                atomicAdd(g + 1, (double)sy);
-                atomicAdd(g + 2, (double)sz);
-                atomicAdd(g + 3, (double)sm);
-            }
-        }
+        Lam l{};
+        if (valid) l = ld_lam(lam, p);
+        reverse_step(a, lvl, st, d, w.x, local, p, fl, tape, l, r, dbias, dsrc, table);
+        if (valid) st_lam(lam, p, l);
     }
-    // the loop ends for the whole CTA together: flush the bias table
+    // the loop ends for the whole CTA together
     if (dbias) {
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kBiasTable; i += blockDim.x) {
-            const uint32_t n = s_bias_key[i];
-            if (n != kBiasEmpty) {
-                atomicAdd(dbias + 3u * n + 0u, (double)s_bias_g[3u * i]);
-                atomicAdd(dbias + 3u * n + 1u, (double)s_bias_g[3u * i + 1u]);
-                atomicAdd(dbias + 3u * n + 2u, (double)s_bias_g[3u * i + 2u]);
-            }
+        flush_bias_table(s_bias_key, s_bias_g, dbias);
+    }
+}
+
+// The reverse of steps `last`, last - 1, ..., last - count + 1, which share
+// one met bracket, a CTA per item: the adjoint state stays in registers from
+// step to step, and the level arrays and the bias table are set up once (the
+// table goes to the gradient after every step, as above, so its float sums
+// are no longer).  One launch per bracket and window instead of one per step:
+// at 160 k particles @@ us for 25 steps, 455 us one by one.  Above
+// kReverseItems items the persistent kernel is the better one: it merges the
+// bias terms of many items before the f64 atomics.
+constexpr uint32_t kReverseItems = 4096;
+
+__global__ void __launch_bounds__(256, 4) inverse_reverse_kernel(StepArgs a, const BatchState* st_all,
+                                                                 const ScenDev* sc_all, uint32_t n_scen,
+                                                                 const uint2* __restrict__ items, TapeBase tb,
+                                                                 uint32_t last, uint32_t count, LamArrays lam,
+                                                                 Receptors r, double* dbias, double* dsrc) {
+    chain_begin();
+    extern __shared__ float s_levels[];
+    __shared__ uint32_t s_bias_key[kBiasTable];
+    __shared__ float s_bias_g[3 * kBiasTable];
+    const uint2 w = items[blockIdx.x];
+    const uint32_t local = w.y + threadIdx.x;
+    const uint32_t j0 = last % tb.slices;
+    // releases only grow: without a slot released by the last step the item is idle
+    if (w.y >= sc_all[(size_t)j0 * n_scen + w.x].released) return;
+    const Levels lvl = stage_levels(a, s_levels);
+    clear_bias_table(s_bias_key, s_bias_g);
+    const BiasTable table{s_bias_key, s_bias_g};
+    __syncthreads();
+    Lam l{};
+    bool loaded = false;
+    uint32_t p = 0;
+    for (uint32_t i = 0; i < count; ++i) {
+        const uint32_t j = (last - i) % tb.slices;
+        const ScenDev& d = sc_all[(size_t)j * n_scen + w.x];
+        p = d.offset + local;
+        TapeArrays tape;
+#pragma unroll
+        for (int f = 0; f < TAPE_FIELDS; ++f) tape.f[f] = tb.field(j, f);
+        const uint32_t fl = local < d.released ? reinterpret_cast<const uint32_t*>(tape.f[T_FLAGS])[p] : 0u;
+        const bool valid = (fl & TAPE_ACTIVE) != 0u;
+        if (valid && !loaded) {
+            l = ld_lam(lam, p);
+            loaded = true;
+        }
+        const bool warp_valid = __ballot_sync(0xffffffffu, valid) != 0u;
+        if (warp_valid) reverse_step(a, lvl, st_all + j, d, w.x, local, p, fl, tape, l, r, dbias, dsrc, table);
+        if (dbias && __syncthreads_or(warp_valid)) {
+            flush_bias_table(s_bias_key, s_bias_g, dbias);
+            __syncthreads();
         }
     }
+    if (loaded) st_lam(lam, p, l);
 }
 
 __global__ void __launch_bounds__(256) add_bias_kernel(const float4* __restrict__ raw, const float* __restrict__ bias,
@@ -658,7 +749,7 @@ static void enqueue_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
     fpg_batch* b = v->b;
     InverseData& d = v->d;
     enqueue_pre(b, s, false, d.st_all, d.sc_all, d.slices);
-    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u), 256, 0, s, make_step_args(b), b->st, b->sc, d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps, kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
+    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u) * kTapeParts, kTapeThreads, 0, s, make_step_args(b), b->st, b->sc, d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps, kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
     b->ctx->count(1);
     if (kind == TAPE_FORWARD_SAMPLE) enqueue_inverse_sample(b, s);
     enqueue_turn(b, s, true);
@@ -947,16 +1038,27 @@ extern "C" fpg_status fpg_inverse_backward(fpg_inverse* v, const double* d_sim, 
             d.packed_ta = step_bracket_start(b, k1 - 1);
         }
         // one work counter per slice, cleared once per window
-        FPG_CUDA(cudaMemsetAsync(d.work_rev, 0, (size_t)S * 4, s));
+        const bool by_bracket = d.n_items <= kReverseItems;
+        if (!by_bracket) FPG_CUDA(cudaMemsetAsync(d.work_rev, 0, (size_t)S * 4, s));
         // reverse of the window; the bracket is repacked only where it changes
-        for (uint64_t k = k1; k-- > k0;) {
-            const uint32_t j = (uint32_t)(k % S);
-            const int64_t ta = step_bracket_start(b, k);
+        for (uint64_t k = k1; k > k0;) {
+            const uint64_t last = --k;
+            const uint32_t j = (uint32_t)(last % S);
+            const int64_t ta = step_bracket_start(b, last);
             if (ta != d.packed_ta) {
                 enqueue_pack_forced(b, d.st_all + j, s);
                 d.packed_ta = ta;
             }
-            launch_chained(inverse_adjoint_kernel, d.grid_adj, 256, smem, s, a, d.st_all + j, d.sc_all + (size_t)j * n_src, d.items, d.n_items, d.work_rev + j, tb, j, lam, rargs, d_bias ? d.dbias : nullptr, d.dsrc);
+            if (by_bracket) {
+                while (k > k0 && step_bracket_start(b, k - 1) == ta) --k;
+                launch_chained(inverse_reverse_kernel, std::max(d.n_items, 1u), 256, smem, s, a, d.st_all, d.sc_all,
+                               (uint32_t)n_src, d.items, tb, (uint32_t)last, (uint32_t)(last - k + 1), lam, rargs,
+                               d_bias ? d.dbias : nullptr, d.dsrc);
+            } else {
+                launch_chained(inverse_adjoint_kernel, d.grid_adj, 256, smem, s, a, d.st_all + j,
+                               d.sc_all + (size_t)j * n_src, d.items, d.n_items, d.work_rev + j, tb, j, lam, rargs,
+                               d_bias ? d.dbias : nullptr, d.dsrc);
+            }
             b->ctx->count(1);
             FPG_CHECK_LAUNCH();
         }
