@@ -338,12 +338,14 @@ __device__ __forceinline__ float3 sample_vjp(const StepArgs& a, const Levels& lv
                 v[3 * c] = w * lu; v[3 * c + 1] = w * lv; v[3 * c + 2] = w * lw;
             }
             warp_sum24(v, lane);
-            // the group's corner set is the source lane's; lane 4c issues corner c
-            const uint32_t cx = __shfl_sync(0xffffffffu, x1, src), cy = __shfl_sync(0xffffffffu, y1, src);
-            const uint32_t cz = __shfl_sync(0xffffffffu, z1, src);
+            // the group's corner set is the source lane's (two integer divisions a
+            // corner took more instructions than these exchanges); lane 4c
+            // issues corner c
+            const uint32_t bx = __shfl_sync(0xffffffffu, x0, src), cx = __shfl_sync(0xffffffffu, x1, src);
+            const uint32_t by = __shfl_sync(0xffffffffu, y0, src), cy = __shfl_sync(0xffffffffu, y1, src);
+            const uint32_t bz = __shfl_sync(0xffffffffu, z0, src), cz = __shfl_sync(0xffffffffu, z1, src);
             if ((lane & 3u) == 0u && (v[0] != 0.0f || v[1] != 0.0f || v[2] != 0.0f)) {
                 const uint32_t c = lane >> 2;
-                const uint32_t bx = k0 / (a.ny * a.nz), by = (k0 / a.nz) % a.ny, bz = k0 % a.nz;
                 const uint32_t n = (((c >> 2) ? cx : bx) * a.ny + (((c >> 1) & 1u) ? cy : by)) * a.nz +
                                    ((c & 1u) ? cz : bz);
                 bias_add(table, n, v[0], v[1], v[2], dbias);
