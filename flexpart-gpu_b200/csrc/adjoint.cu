@@ -692,11 +692,6 @@ struct InverseData {
     bool forward_done = false;
     uint64_t bytes = 0;
     uint32_t grid_adj = 0;               // the reverse's persistent grid: SMs x resident CTAs
-    // one taped step (pre, tape pass, [sampling], turn), captured: the
-    // recompute's (0), the forward's (1) and the forward's sampling steps (2)
-    cudaGraph_t tape_graph[3] = {nullptr, nullptr, nullptr};
-    cudaGraphExec_t tape_exec[3] = {nullptr, nullptr, nullptr};
-    uint64_t tape_launches[3] = {0, 0, 0};
 
     Receptors receptors_args(uint32_t nx, uint32_t ny) const {
         Receptors r;
@@ -718,10 +713,10 @@ bool inverse_sample_step(const fpg_batch* b, uint64_t step) {
     return every != 0 && (step + 1) % every == 0;
 }
 
-void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s) {
+void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s, uint32_t side) {
     InverseData* inv = b->inv;
     const Receptors r = inv->receptors_args((uint32_t)b->met->nx, (uint32_t)b->met->ny);
-    launch_chained(inverse_sample_kernel, b->ctx->sm_count * 8, 256, 0, s, b->st, b->sc, inv->items, inv->n_items, pop_fields(b), r);
+    launch_chained(inverse_sample_kernel, b->ctx->sm_count * 8, 256, 0, s, b->st + side, b->scen_state(side), inv->items, inv->n_items, pop_fields(b), r);
     b->ctx->count(1);
 }
 
@@ -742,38 +737,23 @@ static LamArrays lam_arrays(fpg_inverse* v) {
     return l;
 }
 
-enum { TAPE_RECOMPUTE = 0, TAPE_FORWARD = 1, TAPE_FORWARD_SAMPLE = 2 };
-
 // One taped step: the forward step with the tape pass in place of the plain
 // particle pass and, on the forward's sampling steps, the receptor sampling.
 // The recompute steps only the slots whose adjoint is still non-zero (live).
-static void enqueue_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
+// The steps of an inversion are launched one by one, chained: a graph per
+// step leaves 2.5 us between two steps, and a graph per window costs its
+// capture again for every inversion.
+static fpg_status enqueue_taped_step(fpg_inverse* v, uint64_t step, bool recompute, cudaStream_t s) {
     fpg_batch* b = v->b;
     InverseData& d = v->d;
-    enqueue_pre(b, s, false, d.st_all, d.sc_all, d.slices);
-    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u) * kTapeParts, kTapeThreads, 0, s, make_step_args(b), b->st, b->sc, d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps, kind == TAPE_RECOMPUTE ? d.last_hit : nullptr);
+    const uint32_t side = (uint32_t)(step & 1u);
+    enqueue_pre(b, s, side, false, d.st_all, d.sc_all, d.slices);
+    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u) * kTapeParts, kTapeThreads, 0, s, make_step_args(b),
+                   b->st + side, b->scen_state(side), d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps,
+                   recompute ? d.last_hit : nullptr);
     b->ctx->count(1);
-    if (kind == TAPE_FORWARD_SAMPLE) enqueue_inverse_sample(b, s);
-    enqueue_turn(b, s, true);
-}
-
-static fpg_status launch_taped_step(fpg_inverse* v, int kind, cudaStream_t s) {
-    InverseData& d = v->d;
-    fpg_ctx* ctx = v->b->ctx;
-    if (!d.tape_exec[kind]) {
-        FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        const uint64_t before = ctx->launches.load();
-        enqueue_taped_step(v, kind, s);
-        d.tape_launches[kind] = ctx->launches.load() - before;
-        ctx->launches.fetch_sub(d.tape_launches[kind]);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(s, &g);
-        if (e != cudaSuccess) return cuda_status(e);
-        d.tape_graph[kind] = g;
-        FPG_CUDA(cudaGraphInstantiate(&d.tape_exec[kind], g, 0));
-    }
-    FPG_CUDA(cudaGraphLaunch(d.tape_exec[kind], s));
-    ctx->count(d.tape_launches[kind]);
+    if (!recompute && inverse_sample_step(b, step)) enqueue_inverse_sample(b, s, side);
+    FPG_CHECK_LAUNCH();
     return FPG_OK;
 }
 
@@ -790,15 +770,16 @@ static fpg_status rebuild_ring(fpg_inverse* v) {
 
 static cudaError_t enqueue_checkpoint(fpg_inverse* v, uint32_t c, bool restore) {
     fpg_batch* b = v->b;
+    const uint32_t side = (uint32_t)((uint64_t)c * v->d.window & 1u);
     CheckpointArgs a;
     for (int f = 0; f < kNumCkptFields; ++f) {
         a.field[f] = static_cast<uint4*>(b->pop->field[kCkptFields[f]]);
         a.saved[f] = reinterpret_cast<uint4*>(v->d.ckpt + ((size_t)c * kNumCkptFields + f) * b->capacity);
     }
     a.quads = b->capacity / 4;                       // the capacity is a multiple of a tile
-    a.st = b->st;
+    a.st = b->st + side;
     a.st_saved = v->d.ckpt_st + c;
-    a.sc = b->sc;
+    a.sc = b->scen_state(side);
     a.sc_saved = v->d.ckpt_sc + (size_t)c * b->scen.size();
     a.n_scen = (uint32_t)b->scen.size();
     a.restore = restore ? 1 : 0;
@@ -816,10 +797,6 @@ extern "C" fpg_status fpg_inverse_destroy(fpg_inverse* v) {
         v->b->inv = nullptr;
     }
     InverseData& d = v->d;
-    for (int k = 0; k < 3; ++k) {
-        if (d.tape_exec[k]) cudaGraphExecDestroy(d.tape_exec[k]);
-        if (d.tape_graph[k]) cudaGraphDestroy(d.tape_graph[k]);
-    }
     cudaFree(d.rmap); cudaFree(d.sim); cudaFree(d.last_hit); cudaFree(d.g); cudaFree(d.ring_raw); cudaFree(d.bias);
     cudaFree(d.ckpt); cudaFree(d.ckpt_st); cudaFree(d.ckpt_sc); cudaFree(d.st_all); cudaFree(d.sc_all);
     cudaFree(d.tape); cudaFree(d.lam); cudaFree(d.dbias); cudaFree(d.dbias_f); cudaFree(d.dsrc);
@@ -984,9 +961,10 @@ extern "C" fpg_status fpg_inverse_forward(fpg_inverse* v, double* simulated) {
     for (uint64_t k = 0; k < b->total_steps; ++k) {
         if (k < k_tail) {
             if (k % K == 0) FPG_CUDA(enqueue_checkpoint(v, (uint32_t)(k / K), false));
-            st = launch_step_graph(b, k, s);
+            enqueue_batched_step(b, s, k, output_step(b, k));
+            FPG_CHECK_LAUNCH();
         } else {
-            st = launch_taped_step(v, inverse_sample_step(b, k) ? TAPE_FORWARD_SAMPLE : TAPE_FORWARD, s);
+            st = enqueue_taped_step(v, k, false, s);
         }
         if (st != FPG_OK) return st;
     }
@@ -1034,7 +1012,7 @@ extern "C" fpg_status fpg_inverse_backward(fpg_inverse* v, const double* d_sim, 
             // bracket of its last step packed
             FPG_CUDA(enqueue_checkpoint(v, (uint32_t)w, true));
             for (uint64_t k = k0; k < k1; ++k) {
-                const fpg_status st = launch_taped_step(v, TAPE_RECOMPUTE, s);
+                const fpg_status st = enqueue_taped_step(v, k, true, s);
                 if (st != FPG_OK) return st;
             }
             d.packed_ta = step_bracket_start(b, k1 - 1);

@@ -12,16 +12,16 @@
 //
 // One step is a short kernel sequence that reads its per-step values
 // (clock, alpha, bracket, release ranges, counters) from device memory, so
-// it is captured into CUDA graphs (one for steps that end with grids or
-// receptor samples, one for the others) and replayed:
+// it is captured into CUDA graphs and replayed:
 //   batch_pre       bracket from the ring when it changed, PBL (and wet
 //                   forcing) per cell, new particles of every scenario
-//                   (lattice in f64), grids cleared before an output step
+//                   (lattice in f64), grids cleared before an output step,
+//                   and the next step's state: counters += capacity * blocks,
+//                   clock += dt, its bracket, alpha and release ranges
 //   batch_step      the fused per-particle step (step_core.cuh): one CTA per
 //                   work item, or persistent CTAs that pull items
 //   batch_grid      per-scenario grids at output steps
-//   batch_turn      counters += capacity * blocks; clock += dt; then the
-//                   bracket, alpha and release ranges of the next step
+// The state of a step and the next lie in two buffers that swap every step.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -63,29 +63,43 @@ __device__ __forceinline__ void advance_clock(BatchState* st, const BatchConst& 
     st->work = 0;
 }
 
-// Ends a step (`end`: counters and clock move on) and prepares the next one,
-// so that a step is one launch before its particle pass and one after it.
-// Runs once without `end` when the state is (re)set.
-__global__ void __launch_bounds__(256) batch_turn_kernel(BatchState* st, ScenDev* sc, BatchConst c, int end) {
+// The release range and Philox head of scenario d at time t; `lo` particles
+// are out already.
+__device__ __forceinline__ void advance_scenario(ScenDev& d, int64_t t, uint32_t lo) {
+    uint32_t hi = target_emitted(d.start, d.end, d.count, t, lo);
+    if (hi < lo) hi = lo;
+    d.rel_lo = lo;
+    d.rel_hi = hi;
+    d.released = hi;
+    d.head = philox_head(d.counter, d.key0, d.key1);
+    d.head_ok = (uint64_t)d.counter.x + 2u * (uint64_t)d.capacity <= (1ull << 32);
+}
+
+// The first step's state, when the batch is created or reset.
+__global__ void __launch_bounds__(256) batch_begin_kernel(BatchState* st, ScenDev* sc, BatchConst c) {
     chain_begin();
-    const int64_t t = st->t + (end ? c.dt : 0);
+    for (uint32_t s = threadIdx.x; s < c.n_scen; s += blockDim.x) advance_scenario(sc[s], st->t, sc[s].released);
+    if (threadIdx.x == 0) advance_clock(st, c);
+}
+
+// The next step's state from this one's (counters and clock moved on), by one
+// CTA.  The two steps' states lie in two buffers, so that this runs beside
+// the step that reads the first.
+__device__ __forceinline__ void turn(const BatchState* st, const ScenDev* sc, const BatchConst& c, BatchState* next_st,
+                                     ScenDev* next_sc) {
+    const int64_t t = st->t + c.dt;
     for (uint32_t s = threadIdx.x; s < c.n_scen; s += blockDim.x) {
-        ScenDev& d = sc[s];
-        if (end) d.counter = counter_add64(d.counter, (uint64_t)d.capacity * c.bpp);
-        const uint32_t lo = d.released;
-        uint32_t hi = target_emitted(d.start, d.end, d.count, t, lo);
-        if (hi < lo) hi = lo;
-        d.rel_lo = lo;
-        d.rel_hi = hi;
-        d.released = hi;
-        d.head = philox_head(d.counter, d.key0, d.key1);
-        d.head_ok = (uint64_t)d.counter.x + 2u * (uint64_t)d.capacity <= (1ull << 32);
+        ScenDev d = sc[s];
+        d.counter = counter_add64(d.counter, (uint64_t)d.capacity * c.bpp);
+        advance_scenario(d, t, d.released);
+        next_sc[s] = d;
     }
-    __syncthreads();                                    // every thread has read the old clock
     if (threadIdx.x == 0) {
-        st->t = t;
-        st->step += end ? 1u : 0u;
-        advance_clock(st, c);
+        BatchState n = *st;
+        n.t = t;
+        n.step += 1u;
+        advance_clock(&n, c);
+        *next_st = n;
     }
 }
 
@@ -93,8 +107,8 @@ __global__ void __launch_bounds__(256) batch_turn_kernel(BatchState* st, ScenDev
 // (release/mod.rs:103-146, coords/mod.rs:92-114,169-178) on the device, in
 // the same f64 arithmetic as the host release manager.  CTA `part` of `parts`
 // of one scenario.
-__device__ __forceinline__ void release_particles(BatchState* st, const ScenDev& d, const BatchConst& c,
-                                                  const PopFields& F, uint32_t part, uint32_t parts) {
+__device__ __forceinline__ void release_particles(const BatchState* st, const ScenDev& d, const BatchConst& c,
+                                                  const PopFields& F, uint32_t part, uint32_t parts, int32_t* error) {
     const int32_t now = (int32_t)st->t;
     for (uint32_t k = d.rel_lo + part * blockDim.x + threadIdx.x; k < d.rel_hi; k += parts * blockDim.x) {
         const uint64_t idx = k;
@@ -108,7 +122,7 @@ __device__ __forceinline__ void release_particles(BatchState* st, const ScenDev&
         const double x = (lon - c.xlon0) / c.dx;
         const double y = (lat - c.ylat0) / c.dy;
         if (!(x >= 0.0 && x < (double)(c.gnx - 1) && y >= 0.0 && y < (double)(c.gny - 1))) {
-            atomicOr(&st->error, 1);
+            atomicOr(error, 1);
             continue;
         }
         const double fxf = floor(x), fyf = floor(y);
@@ -126,8 +140,9 @@ __device__ __forceinline__ void release_particles(BatchState* st, const ScenDev&
     }
 }
 
-// Everything a step does before its particle pass, one launch: the CTAs are
-// shared out over independent parts that read the state the turn kernel left.
+// Everything a step does beside its particle pass, one launch before it: the
+// CTAs are shared out over independent parts that read the step's state, and
+// one CTA writes the next step's.
 // A step of a small ensemble is bound by its launches (separate advance,
 // pack, PBL, release and end kernels took 11 us of device time and five
 // launches a step beside an 11 us pass at 160 k particles).
@@ -150,16 +165,23 @@ struct PreArgs {
     BatchState* st_out;                  // inversion: the step's state kept per tape slice (NULL: not kept)
     ScenDev* sc_out;
     uint32_t slices;
+    BatchState* st_next;                 // the next step's state
+    ScenDev* sc_next;
+    int32_t* error;
     uint32_t* clear[2];                  // the output grids, cleared on output steps
     size_t clear_n;
     uint32_t clear_ctas;
 };
 constexpr uint32_t kPreThreads = 128;
 
-__global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, const ScenDev* sc, BatchConst c,
+__global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(const BatchState* st, const ScenDev* sc, BatchConst c,
                                                                 PreArgs a) {
     chain_begin();
-    uint32_t b = blockIdx.x;
+    if (blockIdx.x == 0) {
+        turn(st, sc, c, a.st_next, a.sc_next);
+        return;
+    }
+    uint32_t b = blockIdx.x - 1u;
     if (b < a.pbl_ctas) {
         const uint32_t i = b * kPreThreads + threadIdx.x;
         if (i >= a.ncell) return;
@@ -171,7 +193,7 @@ __global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, 
     }
     b -= a.pbl_ctas;
     if (b < c.n_scen * a.parts) {
-        release_particles(st, sc[b / a.parts], c, a.F, b % a.parts, a.parts);
+        release_particles(st, sc[b / a.parts], c, a.F, b % a.parts, a.parts, a.error);
         return;
     }
     b -= c.n_scen * a.parts;
@@ -191,7 +213,7 @@ __global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(BatchState* st, 
         }
         return;
     }
-    // the last CTA: the post-advance clock and scenario state of the step's tape slice
+    // the last CTA: the clock and scenario state of the step's tape slice
     const uint32_t j = st->step % a.slices;
     if (threadIdx.x == 0) a.st_out[j] = *st;
     for (uint32_t s = threadIdx.x; s < c.n_scen; s += kPreThreads) a.sc_out[(size_t)j * c.n_scen + s] = sc[s];
@@ -449,7 +471,8 @@ bool output_step(const fpg_batch* b, uint64_t step) { return grid_step(b, step) 
 
 // Everything before the particle pass; `output`: the step ends with grids.
 // st_out, sc_out: where an inversion keeps the step's state.
-void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, ScenDev* sc_out, uint32_t slices) {
+void enqueue_pre(fpg_batch* b, cudaStream_t s, uint32_t side, bool output, BatchState* st_out, ScenDev* sc_out,
+                 uint32_t slices) {
     const BatchConst c = make_const(b);
     PreArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -474,58 +497,64 @@ void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, 
     a.st_out = st_out;
     a.sc_out = sc_out;
     a.slices = std::max(slices, 1u);
+    a.st_next = b->st + (side ^ 1u);
+    a.sc_next = b->scen_state(side ^ 1u);
+    a.error = b->error;
     if (output && b->cfg.output_every_steps) {
         a.clear[0] = b->grid_counts;
         a.clear[1] = b->grid_mass;
         a.clear_n = (size_t)b->cfg.out_nx * b->cfg.out_ny * b->cfg.out_nz * b->scen.size();
         a.clear_ctas = (uint32_t)b->ctx->sm_count * 8u;
     }
-    const uint32_t ctas = a.pbl_ctas + c.n_scen * a.parts + a.pack_ctas + a.clear_ctas + (st_out ? 1u : 0u);
-    launch_chained(batch_pre_kernel, ctas, kPreThreads, 0, s, b->st, b->sc, c, a);
+    const uint32_t ctas = a.pbl_ctas + c.n_scen * a.parts + a.pack_ctas + a.clear_ctas + (st_out ? 2u : 1u);
+    launch_chained(batch_pre_kernel, ctas, kPreThreads, 0, s, b->st + side, b->scen_state(side), c, a);
     b->ctx->count(1);
 }
 
-// Everything after it; `output`: the step ends with grids or receptor samples.
-void enqueue_post(fpg_batch* b, cudaStream_t s, bool output) {
+// The grids or receptor samples of an output step.
+void enqueue_post(fpg_batch* b, cudaStream_t s, uint32_t side, bool output) {
     if (output && b->cfg.output_every_steps) {
         const GridConst g = make_grid_const(b);
         // 8 resident CTAs per SM, each over a contiguous range of tiles
         const uint32_t ctas = std::max<uint32_t>(1u, std::min<uint32_t>(b->n_tiles, (uint32_t)b->ctx->sm_count * 8u));
         const uint32_t per = (b->n_tiles + ctas - 1u) / ctas;
         const uint32_t blocks = std::max<uint32_t>(1u, (b->n_tiles + per - 1u) / per);
-        launch_chained(batch_grid_kernel, blocks, 256, 0, s, b->st, b->sc, b->tile_scen, pop_fields(b), g, b->n_tiles, per, b->grid_counts, b->grid_mass);
+        launch_chained(batch_grid_kernel, blocks, 256, 0, s, b->st + side, b->scen_state(side), b->tile_scen, pop_fields(b),
+                       g, b->n_tiles, per, b->grid_counts, b->grid_mass);
         b->ctx->count(1);
     }
-    if (output && b->inv) enqueue_inverse_sample(b, s);
-    enqueue_turn(b, s, true);
+    if (output && b->inv) enqueue_inverse_sample(b, s, side);
 }
 
-void enqueue_turn(fpg_batch* b, cudaStream_t s, bool end) {
-    launch_chained(batch_turn_kernel, 1, 256, 0, s, b->st, b->sc, make_const(b), end ? 1 : 0);
+static void enqueue_begin(fpg_batch* b, cudaStream_t s) {
+    launch_chained(batch_begin_kernel, 1, 256, 0, s, b->st, b->sc, make_const(b));
     b->ctx->count(1);
 }
 
-void enqueue_step_kernel(fpg_batch* b, cudaStream_t s) {
+void enqueue_step_kernel(fpg_batch* b, cudaStream_t s, uint32_t side) {
     const StepVariant& v = kVariants[b->variant];
     const StepArgs a = make_step_args(b);
     if (v.ppt == 0) {
         const StepKernel kernel = production_form(a) ? v.production[a.wet_mode == FPG_FORCING_PER_CELL] : v.kernel;
-        launch_chained(kernel, std::max(b->n_items, 1u), v.block, 0, s, a, b->st, b->sc, b->items, b->n_items);
+        launch_chained(kernel, std::max(b->n_items, 1u), v.block, 0, s, a, b->st + side,
+                       b->scen_state(side), b->items, b->n_items);
     } else {
         const uint32_t grid = (uint32_t)b->ctx->sm_count * std::max(b->resident[b->variant], 1u);
-        launch_chained(v.kernel, grid, v.block, level_smem_bytes(b->met), s, a, b->st, b->sc, b->items, b->n_items);
+        launch_chained(v.kernel, grid, v.block, level_smem_bytes(b->met), s, a, b->st + side, b->scen_state(side), b->items,
+                       b->n_items);
     }
     b->ctx->count(1);
 }
 
-void enqueue_batched_step(fpg_batch* b, cudaStream_t s, bool output) {
-    enqueue_pre(b, s, output, nullptr, nullptr, 0);
-    enqueue_step_kernel(b, s);
-    enqueue_post(b, s, output);
+void enqueue_batched_step(fpg_batch* b, cudaStream_t s, uint64_t step, bool output) {
+    const uint32_t side = (uint32_t)(step & 1u);
+    enqueue_pre(b, s, side, output, nullptr, nullptr, 0);
+    enqueue_step_kernel(b, s, side);
+    enqueue_post(b, s, side, output);
 }
 
 static void drop_graphs(fpg_batch* b) {
-    for (int o = 0; o < 2; ++o) {
+    for (int o = 0; o < 4; ++o) {
         if (b->exec[o]) cudaGraphExecDestroy(b->exec[o]);
         if (b->graph[o]) cudaGraphDestroy(b->graph[o]);
         b->exec[o] = nullptr;
@@ -578,7 +607,8 @@ fpg_status batch_reset(fpg_batch* b) {
     s0.t = b->cfg.start_seconds;
     FPG_CUDA(cudaMemcpyAsync(b->st, &s0, sizeof(s0), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(b->sc, b->scen.data(), b->scen.size() * sizeof(ScenDev), cudaMemcpyHostToDevice, s));
-    enqueue_turn(b, s, false);
+    FPG_CUDA(cudaMemsetAsync(b->error, 0, sizeof(int32_t), s));
+    enqueue_begin(b, s);
     FPG_CHECK_LAUNCH();
     FPG_CUDA(cudaStreamSynchronize(s));
     b->steps_done = 0;
@@ -590,30 +620,26 @@ fpg_status batch_reset(fpg_batch* b) {
     return FPG_OK;
 }
 
-// The graph of a step, without (0) and with (1) grids or receptor samples.
-fpg_status ensure_graph(fpg_batch* b, int output) {
-    if (b->exec[output]) return FPG_OK;
-    cudaStream_t s = b->ctx->stream;
-    FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const uint64_t before = b->ctx->launches.load();
-    enqueue_batched_step(b, s, output != 0);
-    // capture launches nothing: take the count back, keep it per replay
-    b->graph_launches[output] = b->ctx->launches.load() - before;
-    b->ctx->launches.fetch_sub(b->graph_launches[output]);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(s, &g);
-    if (e != cudaSuccess) return cuda_status(e);
-    b->graph[output] = g;
-    FPG_CUDA(cudaGraphInstantiate(&b->exec[output], g, 0));
-    return FPG_OK;
-}
-
-fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
-    const int output = output_step(b, step) ? 1 : 0;
-    const fpg_status st = ensure_graph(b, output);
-    if (st != FPG_OK) return st;
-    FPG_CUDA(cudaGraphLaunch(b->exec[output], s));
-    b->ctx->count(b->graph_launches[output]);
+// The graph of a step, by its side of the state (1) and whether it ends with
+// grids (2).
+static fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
+    const bool output = output_step(b, step);
+    const int which = (int)(step & 1u) + (output ? 2 : 0);
+    if (!b->exec[which]) {
+        FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        const uint64_t before = b->ctx->launches.load();
+        enqueue_batched_step(b, s, step, output);
+        // capture launches nothing: take the count back, keep it per replay
+        b->graph_launches[which] = b->ctx->launches.load() - before;
+        b->ctx->launches.fetch_sub(b->graph_launches[which]);
+        cudaGraph_t g = nullptr;
+        cudaError_t e = cudaStreamEndCapture(s, &g);
+        if (e != cudaSuccess) return cuda_status(e);
+        b->graph[which] = g;
+        FPG_CUDA(cudaGraphInstantiate(&b->exec[which], g, 0));
+    }
+    FPG_CUDA(cudaGraphLaunch(b->exec[which], s));
+    b->ctx->count(b->graph_launches[which]);
     return FPG_OK;
 }
 
@@ -647,7 +673,7 @@ extern "C" fpg_status fpg_batch_destroy(fpg_batch* b) {
     fpg_pbl_destroy(b->pbl);
     fpg_cellfield_destroy(b->wet);
     cudaFree(b->ring); cudaFree(b->sring); cudaFree(b->pring); cudaFree(b->staging);
-    cudaFree(b->st); cudaFree(b->sc); cudaFree(b->tile_scen); cudaFree(b->items); cudaFree(b->grid_counts); cudaFree(b->grid_mass);
+    cudaFree(b->st); cudaFree(b->sc); cudaFree(b->error); cudaFree(b->tile_scen); cudaFree(b->items); cudaFree(b->grid_counts); cudaFree(b->grid_mass);
     delete b;
     return FPG_OK;
 }
@@ -725,8 +751,10 @@ extern "C" fpg_status fpg_batch_create(fpg_ctx* ctx, const fpg_batch_config* cfg
     if (e == cudaSuccess) e = cudaMalloc(&b->sring, cells * cfg->n_frames * sizeof(fpg_surface_cell));
     if (e == cudaSuccess) e = cudaMalloc(&b->pring, cells * cfg->n_frames * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&b->staging, nodes * 3 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&b->st, sizeof(BatchState));
-    if (e == cudaSuccess) e = cudaMalloc(&b->sc, n_scen * sizeof(ScenDev));
+    if (e == cudaSuccess) e = cudaMalloc(&b->st, 2 * sizeof(BatchState));
+    if (e == cudaSuccess) e = cudaMalloc(&b->error, sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMemsetAsync(b->error, 0, sizeof(int32_t), ctx->stream);
+    if (e == cudaSuccess) e = cudaMalloc(&b->sc, 2 * n_scen * sizeof(ScenDev));
     if (e == cudaSuccess) e = cudaMalloc(&b->tile_scen, b->n_tiles * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->grid_counts, (grid_total ? grid_total : 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->grid_mass, (grid_total ? grid_total : 1) * sizeof(uint32_t));
@@ -743,7 +771,7 @@ extern "C" fpg_status fpg_batch_create(fpg_ctx* ctx, const fpg_batch_config* cfg
         e = cudaMemcpyAsync(b->tile_scen, b->tile_scen_h.data(), b->n_tiles * sizeof(uint32_t), cudaMemcpyHostToDevice,
                             ctx->stream);
     if (e == cudaSuccess) {
-        enqueue_turn(b, ctx->stream, false);
+        enqueue_begin(b, ctx->stream);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -799,7 +827,7 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
             const fpg_status st = launch_step_graph(b, step, s);
             if (st != FPG_OK) return st;
         } else {
-            enqueue_batched_step(b, s, output_step(b, step));
+            enqueue_batched_step(b, s, step, output_step(b, step));
             FPG_CHECK_LAUNCH();
         }
     }
@@ -828,7 +856,8 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
     // alpha of the step comes from the host clock (same formula as the device)
     for (uint64_t i = 0; i < n; ++i) {
         const bool output = output_step(b, b->steps_done + i);
-        enqueue_pre(b, s, output, nullptr, nullptr, 0);
+        const uint32_t side = (uint32_t)((b->steps_done + i) & 1u);
+        enqueue_pre(b, s, side, output, nullptr, nullptr, 0);
         int64_t k = (b->t_h - b->cfg.start_seconds) / b->cfg.frame_seconds;
         if (b->t_h - b->cfg.start_seconds == k * b->cfg.frame_seconds && k > 0) k -= 1;
         const int64_t ta = b->cfg.start_seconds + k * b->cfg.frame_seconds;
@@ -855,7 +884,7 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
             fused_step_kernel<<<(released + 255) / 256, 256, 0, s>>>(a);
             b->ctx->count();
         }
-        enqueue_post(b, s, output);
+        enqueue_post(b, s, side, output);
         FPG_CHECK_LAUNCH();
         b->t_h += b->cfg.timestep_seconds;
     }
@@ -886,10 +915,8 @@ extern "C" fpg_status fpg_batch_download_grids(fpg_batch* b, uint32_t* counts, u
 
 extern "C" fpg_status fpg_batch_errors(fpg_batch* b, int32_t* flags) {
     if (!b || !flags) return FPG_ERR_INVALID_ARGUMENT;
-    BatchState h;
-    FPG_CUDA(cudaMemcpyAsync(&h, b->st, sizeof(h), cudaMemcpyDeviceToHost, b->ctx->stream));
+    FPG_CUDA(cudaMemcpyAsync(flags, b->error, sizeof(int32_t), cudaMemcpyDeviceToHost, b->ctx->stream));
     FPG_CUDA(cudaStreamSynchronize(b->ctx->stream));
-    *flags = h.error;
     return FPG_OK;
 }
 
@@ -936,7 +963,8 @@ extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_
     if (reps == 0) reps = 1;
     cudaStream_t s = b->ctx->stream;
     const size_t pop_bytes = particles_block_bytes(b->capacity);
-    const size_t sc_bytes = b->scen.size() * sizeof(ScenDev);
+    const size_t sc_bytes = 2 * b->scen.size() * sizeof(ScenDev), st_bytes = 2 * sizeof(BatchState);
+    const uint32_t side = (uint32_t)(b->steps_done & 1u);
     void* snap = nullptr;
     BatchState* st_snap = nullptr;
     ScenDev* sc_snap = nullptr;
@@ -946,16 +974,16 @@ extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_
     float best_ms = 0.0f;
     cudaError_t e = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = cudaMalloc(&snap, pop_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&st_snap, sizeof(BatchState));
+    if (e == cudaSuccess) e = cudaMalloc(&st_snap, st_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&sc_snap, sc_bytes);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaMemcpyAsync(snap, b->pop->block, pop_bytes, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(st_snap, b->st, sizeof(BatchState), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(st_snap, b->st, st_bytes, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sc_snap, b->sc, sc_bytes, cudaMemcpyDeviceToDevice, s);
     auto restore = [&]() {
         cudaError_t r = cudaMemcpyAsync(b->pop->block, snap, pop_bytes, cudaMemcpyDeviceToDevice, s);
-        if (r == cudaSuccess) r = cudaMemcpyAsync(b->st, st_snap, sizeof(BatchState), cudaMemcpyDeviceToDevice, s);
+        if (r == cudaSuccess) r = cudaMemcpyAsync(b->st, st_snap, st_bytes, cudaMemcpyDeviceToDevice, s);
         if (r == cudaSuccess) r = cudaMemcpyAsync(b->sc, sc_snap, sc_bytes, cudaMemcpyDeviceToDevice, s);
         return r;
     };
@@ -965,10 +993,10 @@ extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_
         for (uint32_t r = 0; status == FPG_OK && e == cudaSuccess && r < reps; ++r) {
             e = restore();
             if (e != cudaSuccess) break;
-            enqueue_pre(b, s, false, nullptr, nullptr, 0);
+            enqueue_pre(b, s, side, false, nullptr, nullptr, 0);
             e = cudaEventRecord(e0, s);
             if (e != cudaSuccess) break;
-            enqueue_step_kernel(b, s);
+            enqueue_step_kernel(b, s, side);
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaEventRecord(e1, s);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

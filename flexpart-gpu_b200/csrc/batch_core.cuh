@@ -25,7 +25,6 @@ struct BatchState {
     int32_t have_bracket;
     int32_t changed;
     float alpha;
-    int32_t error;
     uint32_t work;
 };
 
@@ -35,7 +34,7 @@ struct ScenDev {
     uint32_t key0, key1;
     u32x4 counter;
     PhiloxHead head;                 // of the coming step's counter, and whether no block's counter
-    uint32_t head_ok;                // carries out of its first word (batch_turn_kernel)
+    uint32_t head_ok;                // carries out of its first word (advance_scenario)
     uint32_t released, rel_lo, rel_hi;
     float mass_per_particle;
     int64_t start, end;
@@ -104,8 +103,12 @@ struct fpg_batch {
     fpg_surface_cell* sring = nullptr;    // n_frames * cells
     float* pring = nullptr;               // n_frames * cells precipitation
     float* staging = nullptr;             // 3 * nodes
+    // the state of step k on side k & 1 and of the next step on the other:
+    // two BatchStates, and two times scen.size() ScenDevs
     fpg::BatchState* st = nullptr;
     fpg::ScenDev* sc = nullptr;
+    fpg::ScenDev* scen_state(uint32_t side) const { return sc + (size_t)side * scen.size(); }
+    int32_t* error = nullptr;             // bit 0: a release left the grid
     uint32_t* tile_scen = nullptr;
     uint2* items = nullptr;               // work items of the chosen launch shape
     uint32_t n_items = 0;
@@ -115,10 +118,10 @@ struct fpg_batch {
     float tuned_ms = 0.0f;
     uint32_t* grid_counts = nullptr;
     uint32_t* grid_mass = nullptr;
-    // the step's graphs: without (0) and with (1) grids or receptor samples at its end
-    cudaGraph_t graph[2] = {nullptr, nullptr};
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    uint64_t graph_launches[2] = {0, 0};  // kernels in one replay
+    // the step's graphs, by its side (1) and whether it ends with grids (2)
+    cudaGraph_t graph[4] = {};
+    cudaGraphExec_t exec[4] = {};
+    uint64_t graph_launches[4] = {};      // kernels in one replay
     std::vector<uint32_t> released_h;     // host mirror of the release counts (sequential path)
     std::vector<fpg::u32x4> counter_h;
     int64_t t_h = 0;
@@ -133,22 +136,19 @@ BatchConst make_const(const fpg_batch* b);
 PopFields pop_fields(fpg_batch* b);
 // Whether step `step` ends with grids or receptor samples.
 bool output_step(const fpg_batch* b, uint64_t step);
-// The launch before the particle pass (bracket, PBL, releases, cleared grids;
-// with st_out and sc_out the step's state kept in slice step % slices), the
-// particle pass in the chosen launch shape, and the launches after it (grids
-// or receptor samples, counter and clock advance).
-void enqueue_pre(fpg_batch* b, cudaStream_t s, bool output, BatchState* st_out, ScenDev* sc_out, uint32_t slices);
-void enqueue_step_kernel(fpg_batch* b, cudaStream_t s);
-void enqueue_post(fpg_batch* b, cudaStream_t s, bool output);
-// Counters and clock to the next step (`end`), and that step's bracket, alpha
-// and release ranges.
-void enqueue_turn(fpg_batch* b, cudaStream_t s, bool end);
+// The launch before the particle pass (bracket, PBL, releases, cleared grids,
+// the next step's state; with st_out and sc_out this step's state kept in
+// slice step % slices), the particle pass in the chosen launch shape, and the
+// launches after it (grids or receptor samples).  `side`: step & 1.
+void enqueue_pre(fpg_batch* b, cudaStream_t s, uint32_t side, bool output, BatchState* st_out, ScenDev* sc_out,
+                 uint32_t slices);
+void enqueue_step_kernel(fpg_batch* b, cudaStream_t s, uint32_t side);
+void enqueue_post(fpg_batch* b, cudaStream_t s, uint32_t side, bool output);
+// All of them for step `step`.
+void enqueue_batched_step(fpg_batch* b, cudaStream_t s, uint64_t step, bool output);
 // Repacks the bracket of state st's frames whether or not it changed.
 void enqueue_pack_forced(fpg_batch* b, const BatchState* st, cudaStream_t s);
 fpg_status build_items(fpg_batch* b, uint32_t variant);
-// Launches step `step` from its graph (pre, particle pass, post), captured
-// when none is held.
-fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s);
 // FPG_ERR_OUT_OF_GRID when the scenario's release lattice leaves the grid.
 fpg_status check_release_grid(const ScenDev& d, const fpg_grid_domain& g);
 size_t particles_block_bytes(size_t capacity);
@@ -157,6 +157,6 @@ size_t particles_block_bytes(size_t capacity);
 fpg_status batch_reset(fpg_batch* b);
 // Receptor sampling of a source inversion at output steps (adjoint.cu).
 bool inverse_sample_step(const fpg_batch* b, uint64_t step);
-void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s);
+void enqueue_inverse_sample(fpg_batch* b, cudaStream_t s, uint32_t side);
 
 }  // namespace fpg
