@@ -168,7 +168,11 @@ struct TapeRec {
 // kTapeParts CTAs per 256-slot work item, launched over all items; the level
 // arrays are read from global memory (no staging, no barrier).  Small CTAs
 // fill the last wave: 160 k particles are 625 items, one more than the 592
-// CTAs of 256 threads that are resident (13.6 us a step, @@ with 64 threads).
+// CTAs of 256 threads that are resident (13.6 us a step).  Small CTAs here and
+// a bracket's reverse in one launch (below) together took a 6 h inversion of
+// 160 k particles, forward and backward, from 1,903 to 1,765 us.  The stage
+// settings stay run-time values: set as constants in a copy of the arguments,
+// they put that copy on each thread's stack and the inversion took 180 us more.
 constexpr uint32_t kTapeThreads = 64, kTapeParts = TILE / kTapeThreads;
 
 __global__ void __launch_bounds__(kTapeThreads, 16) inverse_tape_kernel(StepArgs a, const BatchState* st,
@@ -281,31 +285,29 @@ __device__ __forceinline__ void bias_add(const BiasTable& t, uint32_t n, float g
     atomicAdd(dbias + 3u * n + 2u, (double)gw);
 }
 
-// Vector-Jacobian product of one dual-time trilinear sample: given lambda of
-// its (u, v, w), returns lambda . d(u, v, w)/d(x, y, z) and adds lambda x
-// corner weight to the bias gradient of each corner node (the bias enters
-// both frames, whose time weights sum to one).  Called by the whole warp;
-// lanes with valid == false contribute nothing.  The bias terms of lanes
-// whose samples share a corner set are summed across the warp first, and
-// eight lanes then add one corner each to the CTA's table.
-__device__ __forceinline__ float3 sample_vjp(const StepArgs& a, const Levels& lvl, bool valid, float x, float y,
-                                             float z, float alpha, float lu, float lv, float lw,
-                                             double* __restrict__ dbias, const BiasTable& table) {
+// One dual-time trilinear sample's cell: corners and weights.
+struct SampleCell {
     uint32_t x0, x1, y0, y1, z0, z1;
     float tx, ty, tz;
-    axis_bracket(x, a.nx, x0, x1, tx);
-    axis_bracket(y, a.ny, y0, y1, ty);
+};
+
+// Vector-Jacobian product of one dual-time trilinear sample: given lambda of
+// its (u, v, w), returns lambda . d(u, v, w)/d(x, y, z) and the sample's cell
+// for the bias scatter.  A lane whose lambda is zero (a particle that reaches
+// no receptor after this step) loads no corners.
+__device__ __forceinline__ float3 sample_vjp(const StepArgs& a, const Levels& lvl, bool valid, float x, float y,
+                                             float z, float alpha, float lu, float lv, float lw, SampleCell& s) {
+    axis_bracket(x, a.nx, s.x0, s.x1, s.tx);
+    axis_bracket(y, a.ny, s.y0, s.y1, s.ty);
     const float lev = meters_to_level(lvl, z);
-    axis_bracket(lev, a.nz, z0, z1, tz);
+    axis_bracket(lev, a.nz, s.z0, s.z1, s.tz);
     const float ix = (x > 0.0f && x < (float)(a.nx - 1u)) ? 1.0f : 0.0f;
     const float iy = (y > 0.0f && y < (float)(a.ny - 1u)) ? 1.0f : 0.0f;
     const float iz = (lev > 0.0f && lev < (float)(a.nz - 1u))
                          ? level_slope(lvl, z) : 0.0f;
-    const uint32_t xs[2] = {x0, x1}, ys[2] = {y0, y1}, zs[2] = {z0, z1};
-    const float wx[2] = {1.0f - tx, tx}, wy[2] = {1.0f - ty, ty}, wz[2] = {1.0f - tz, tz};
+    const uint32_t xs[2] = {s.x0, s.x1}, ys[2] = {s.y0, s.y1}, zs[2] = {s.z0, s.z1};
+    const float wx[2] = {1.0f - s.tx, s.tx}, wy[2] = {1.0f - s.ty, s.ty}, wz[2] = {1.0f - s.tz, s.tz};
     const float ta = 1.0f - alpha;
-    // a lane whose lambda is zero (a particle that reaches no receptor after
-    // this step) adds nothing: it loads no corners and joins no group
     const bool act = valid && (lu != 0.0f || lv != 0.0f || lw != 0.0f);
     float f[2][2][2];
 #pragma unroll
@@ -322,37 +324,6 @@ __device__ __forceinline__ float3 sample_vjp(const StepArgs& a, const Levels& lv
                 }
                 f[i][j][k] = fv;
             }
-    if (dbias) {
-        const uint32_t key = act ? (x0 * a.ny + y0) * a.nz + z0 : 0xffffffffu;
-        const unsigned lane = threadIdx.x & 31u;
-        unsigned pending = __ballot_sync(0xffffffffu, act);
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            const uint32_t k0 = __shfl_sync(0xffffffffu, key, src);
-            const bool mine = act && key == k0;
-            const unsigned grp = __ballot_sync(0xffffffffu, mine);
-            float v[24];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float w = mine ? wx[c >> 2] * wy[(c >> 1) & 1] * wz[c & 1] : 0.0f;
-                v[3 * c] = w * lu; v[3 * c + 1] = w * lv; v[3 * c + 2] = w * lw;
-            }
-            warp_sum24(v, lane);
-            // the group's corner set is the source lane's (two integer divisions a
-            // corner took more instructions than these exchanges); lane 4c
-            // issues corner c
-            const uint32_t bx = __shfl_sync(0xffffffffu, x0, src), cx = __shfl_sync(0xffffffffu, x1, src);
-            const uint32_t by = __shfl_sync(0xffffffffu, y0, src), cy = __shfl_sync(0xffffffffu, y1, src);
-            const uint32_t bz = __shfl_sync(0xffffffffu, z0, src), cz = __shfl_sync(0xffffffffu, z1, src);
-            if ((lane & 3u) == 0u && (v[0] != 0.0f || v[1] != 0.0f || v[2] != 0.0f)) {
-                const uint32_t c = lane >> 2;
-                const uint32_t n = (((c >> 2) ? cx : bx) * a.ny + (((c >> 1) & 1u) ? cy : by)) * a.nz +
-                                   ((c & 1u) ? cz : bz);
-                bias_add(table, n, v[0], v[1], v[2], dbias);
-            }
-            pending &= ~grp;
-        }
-    }
     float gx = 0.0f, gy = 0.0f, gz = 0.0f;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -367,6 +338,53 @@ __device__ __forceinline__ float3 sample_vjp(const StepArgs& a, const Levels& lv
 #pragma unroll
         for (int j = 0; j < 2; ++j) gz += wx[i] * wy[j] * (f[i][j][1] - f[i][j][0]);
     return make_float3(gx * ix, gy * iy, gz * iz);
+}
+
+// Adds lambda x corner weight of every lane's sample to the bias gradient of
+// its corner nodes (the bias enters both frames, whose time weights sum to
+// one).  Called by the whole warp; `act` lanes take part.  The terms of lanes
+// whose samples share a corner set are summed across the warp first, and
+// eight lanes then add one corner each to the CTA's table.  A step's two
+// samples mostly lie in one cell: with `both` the second sample's terms
+// (`t`, mu, mv, mw) join the first's, one exchange for the two (6 h inversion
+// of 160 k / 1 M particles 1,468 -> 1,441 us / 3,228 -> 3,167 us).
+__device__ __forceinline__ void scatter_bias(const StepArgs& a, bool act, const SampleCell& s, float lu, float lv,
+                                             float lw, bool both, const SampleCell& t, float mu, float mv, float mw,
+                                             double* __restrict__ dbias, const BiasTable& table) {
+    const uint32_t key = act ? (s.x0 * a.ny + s.y0) * a.nz + s.z0 : 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned pending = __ballot_sync(0xffffffffu, act);
+    while (pending) {
+        const int src = __ffs(pending) - 1;
+        const uint32_t k0 = __shfl_sync(0xffffffffu, key, src);
+        const bool mine = act && key == k0;
+        const unsigned grp = __ballot_sync(0xffffffffu, mine);
+        const float s_on = mine ? 1.0f : 0.0f, t_on = mine && both ? 1.0f : 0.0f;
+        const float sx[2] = {s_on * (1.0f - s.tx), s_on * s.tx}, tx[2] = {t_on * (1.0f - t.tx), t_on * t.tx};
+        float v[24];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float ws = sx[c >> 2] * (((c >> 1) & 1) ? s.ty : 1.0f - s.ty) * ((c & 1) ? s.tz : 1.0f - s.tz);
+            const float wt = tx[c >> 2] * (((c >> 1) & 1) ? t.ty : 1.0f - t.ty) * ((c & 1) ? t.tz : 1.0f - t.tz);
+            v[3 * c] = ws * lu + wt * mu;
+            v[3 * c + 1] = ws * lv + wt * mv;
+            v[3 * c + 2] = ws * lw + wt * mw;
+        }
+        warp_sum24(v, lane);
+        // the group's corner set is the source lane's (two integer divisions a
+        // corner took more instructions than these exchanges); lane 4c
+        // issues corner c
+        const uint32_t bx = __shfl_sync(0xffffffffu, s.x0, src), cx = __shfl_sync(0xffffffffu, s.x1, src);
+        const uint32_t by = __shfl_sync(0xffffffffu, s.y0, src), cy = __shfl_sync(0xffffffffu, s.y1, src);
+        const uint32_t bz = __shfl_sync(0xffffffffu, s.z0, src), cz = __shfl_sync(0xffffffffu, s.z1, src);
+        if ((lane & 3u) == 0u && (v[0] != 0.0f || v[1] != 0.0f || v[2] != 0.0f)) {
+            const uint32_t c = lane >> 2;
+            const uint32_t n = (((c >> 2) ? cx : bx) * a.ny + (((c >> 1) & 1u) ? cy : by)) * a.nz +
+                               ((c & 1u) ? cz : bz);
+            bias_add(table, n, v[0], v[1], v[2], dbias);
+        }
+        pending &= ~grp;
+    }
 }
 
 // dL/d(output state) of the receptor term of a sampling step.
@@ -448,7 +466,8 @@ __device__ __forceinline__ void reverse_step(const StepArgs& a, const Levels& lv
     const float lu1 = lu0, lv1 = lv0, lw1 = lw0;
     ltu0 += lu1;
     ltv0 += lv1;
-    const float3 g1 = sample_vjp(a, lvl, valid, px, py, pz, alpha, lu1, lv1, lw1, dbias, table);
+    SampleCell c1, c0;
+    const float3 g1 = sample_vjp(a, lvl, valid, px, py, pz, alpha, lu1, lv1, lw1, c1);
     const float gpx = (fl & ADV_PX) ? g1.x : 0.0f;
     const float gpy = (fl & ADV_PY) ? g1.y : 0.0f;
     const float gpz = (fl & ADV_PZ) ? g1.z : 0.0f;
@@ -457,8 +476,16 @@ __device__ __forceinline__ void reverse_step(const StepArgs& a, const Levels& lv
     lz0 += gpz; lw0 += gpz * kz;
     ltu0 += lu0;
     ltv0 += lv0;
-    const float3 g0 = sample_vjp(a, lvl, valid, x0, y0, z0, alpha, lu0, lv0, lw0, dbias, table);
+    const float3 g0 = sample_vjp(a, lvl, valid, x0, y0, z0, alpha, lu0, lv0, lw0, c0);
     lx0 += g0.x; ly0 += g0.y; lz0 += g0.z;
+    if (dbias) {
+        const bool act1 = valid && (lu1 != 0.0f || lv1 != 0.0f || lw1 != 0.0f);
+        const bool act0 = valid && (lu0 != 0.0f || lv0 != 0.0f || lw0 != 0.0f);
+        const bool both = act0 && act1 && c0.x0 == c1.x0 && c0.y0 == c1.y0 && c0.z0 == c1.z0;
+        scatter_bias(a, act0, c0, lu0, lv0, lw0, both, c1, lu1, lv1, lw1, dbias, table);
+        if (__ballot_sync(0xffffffffu, act1 && !both))
+            scatter_bias(a, act1 && !both, c1, lu1, lv1, lw1, false, c1, 0.0f, 0.0f, 0.0f, dbias, table);
+    }
     if (valid) lam = Lam{lx0, ly0, lz0, ltu0, ltv0, ltw0, lm};
     // released this step: the adjoint is the gradient of the release state
     const bool rel = valid && local >= d.rel_lo && local < d.rel_hi;
@@ -547,7 +574,7 @@ __global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, con
 // step to step, and the level arrays and the bias table are set up once (the
 // table goes to the gradient after every step, as above, so its float sums
 // are no longer).  One launch per bracket and window instead of one per step:
-// at 160 k particles @@ us for 25 steps, 455 us one by one.  Above
+// at 160 k particles 353 us for 25 steps, 455 us one by one.  Above
 // kReverseItems items the persistent kernel is the better one: it merges the
 // bias terms of many items before the f64 atomics.
 constexpr uint32_t kReverseItems = 4096;
@@ -1043,13 +1070,13 @@ extern "C" fpg_status fpg_inverse_backward(fpg_inverse* v, const double* d_sim, 
             FPG_CHECK_LAUNCH();
         }
     }
-    std::vector<double> src(n_src * 4);
-    FPG_CUDA(cudaMemcpyAsync(src.data(), d.dsrc, n_src * 4 * 8, cudaMemcpyDeviceToHost, s));
     if (d_bias) {
         to_float_kernel<<<b->ctx->sm_count * 4, 256, 0, s>>>(d.dbias, d.nodes * 3, d.dbias_f);
         b->ctx->count(1);
-        FPG_CUDA(cudaMemcpyAsync(d_bias, d.dbias_f, d.nodes * 3 * 4, cudaMemcpyDeviceToHost, s));
     }
+    std::vector<double> src(n_src * 4);
+    FPG_CUDA(cudaMemcpyAsync(src.data(), d.dsrc, n_src * 4 * 8, cudaMemcpyDeviceToHost, s));
+    if (d_bias) FPG_CUDA(cudaMemcpyAsync(d_bias, d.dbias_f, d.nodes * 3 * 4, cudaMemcpyDeviceToHost, s));
     FPG_CUDA(cudaStreamSynchronize(s));
     const fpg_grid_domain& gd = b->cfg.release_grid;
     for (size_t k = 0; k < n_src; ++k) {
