@@ -103,7 +103,7 @@ class SourceInversion:
         dm = np.zeros(self.n_sources, np.float64)
         dp = np.zeros((self.n_sources, 3), np.float64)
         nx, ny, nz = self.shape
-        db = np.zeros((nx, ny, nz, 3), np.float32) if want_bias else None
+        db = np.empty((nx, ny, nz, 3), np.float32) if want_bias else None   # the call fills it
         check(lib.fpg_inverse_backward(self.h, _p(g), _p(dm), _p(dp), _p(db)), "fpg_inverse_backward")
         if db is not None and group is not None:
             from .distributed import allreduce_gradient_fixed_point
