@@ -177,9 +177,12 @@ __global__ void conv_heights_kernel(uint32_t L, const float* __restrict__ m, con
 // edge of bucket b - 1, so rounding of the bucket index cannot pass it) and
 // the search scans up, one comparison or two where a bisection of 60 levels
 // takes six dependent loads.  A column whose bucket width is not a normal
-// float is bisected; otherwise the scan itself runs.
+// float, or with more than kMixScan levels in three adjacent buckets (the
+// longest scan: about as many loads as a bisection of those columns, which
+// have 1000s of levels or crowd them), is bisected; without sorted interfaces
+// the scan over all levels runs.
 enum { MIX_SCAN = 0, MIX_BISECT = 1, MIX_TABLE = 2 };
-constexpr uint32_t kMixBuckets = 1024;
+constexpr uint32_t kMixBuckets = 1024, kMixScan = 8;
 
 struct MixColumn {
     const float* iface;                  // L + 1
@@ -267,14 +270,17 @@ struct fpg_convection {
     fpg_ctx* ctx = nullptr;
     size_t levels = 0;
     float* matrix = nullptr;        // levels^2, column-major (source * levels + destination)
-    float* iface = nullptr;         // levels + 1
+    float* iface = nullptr;         // levels + 1, and in the same block:
     float* centers = nullptr;       // levels
-    float* heights = nullptr;       // levels: expected destination height per source level
     uint16_t* table = nullptr;      // kMixBuckets: the level search (MIX_TABLE)
+    float* heights = nullptr;       // levels: expected destination height per source level
     float inv_w = 0.0f;
     int search = MIX_SCAN;
     bool ready = false;
 };
+
+// Bytes of a column of L levels: interfaces, centres, bucket table.
+static size_t column_bytes(size_t L) { return (2 * L + 1) * sizeof(float) + kMixBuckets * sizeof(uint16_t); }
 
 extern "C" fpg_status fpg_cbl_sample(fpg_ctx* ctx, const fpg_particles* P, const fpg_hanna_params* hanna_dev,
                                      size_t n_hanna, const fpg_cbl_sampling_input* inputs_dev, size_t n_inputs,
@@ -324,14 +330,14 @@ extern "C" fpg_status fpg_convection_create(fpg_ctx* ctx, size_t level_count, fp
     c->levels = level_count;
     const size_t L = level_count;
     cudaError_t e = cudaMalloc(&c->matrix, L * L * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&c->iface, (L + 1) * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&c->centers, L * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&c->iface, column_bytes(L));
     if (e == cudaSuccess) e = cudaMalloc(&c->heights, L * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&c->table, kMixBuckets * sizeof(uint16_t));
     if (e != cudaSuccess) {
         fpg_convection_destroy(c);
         return cuda_status(e);
     }
+    c->centers = c->iface + L + 1;
+    c->table = reinterpret_cast<uint16_t*>(c->centers + L);
     *out = c;
     return FPG_OK;
 }
@@ -340,9 +346,7 @@ extern "C" fpg_status fpg_convection_destroy(fpg_convection* c) {
     if (!c) return FPG_ERR_INVALID_ARGUMENT;
     cudaFree(c->matrix);
     cudaFree(c->iface);
-    cudaFree(c->centers);
     cudaFree(c->heights);
-    cudaFree(c->table);
     delete c;
     return FPG_OK;
 }
@@ -371,28 +375,30 @@ extern "C" fpg_status fpg_convection_set_matrix(fpg_convection* c, const float* 
         if (!std::isfinite(level_interfaces_m[l]) || (l > 0 && !(level_interfaces_m[l] > level_interfaces_m[l - 1])))
             sorted = false;
     }
-    // level_centers_from_interfaces (src/gpu/convection.rs:63-69)
-    std::vector<float> centers(L);
+    // interfaces, centres (level_centers_from_interfaces, src/gpu/convection.rs:63-69)
+    // and the bucket table (in double), one copy
+    std::vector<float> column(column_bytes(L) / sizeof(float));
+    float* centers = column.data() + L + 1;
+    uint16_t* table = reinterpret_cast<uint16_t*>(centers + L);
+    std::memcpy(column.data(), level_interfaces_m, (L + 1) * sizeof(float));
     for (size_t l = 0; l < L; ++l) centers[l] = 0.5f * (level_interfaces_m[l] + level_interfaces_m[l + 1]);
-    // the bucket table, in double
-    std::vector<uint16_t> table(kMixBuckets);
     int search = sorted ? MIX_BISECT : MIX_SCAN;
     const double span = (double)level_interfaces_m[L] - (double)level_interfaces_m[0];
     const float inv_w = sorted ? (float)(kMixBuckets / span) : 0.0f;
     if (sorted && std::isnormal(inv_w) && std::isfinite((float)span)) {
         search = MIX_TABLE;
-        size_t l = 0;
-        for (uint32_t b = 0; b < kMixBuckets; ++b) {
+        uint32_t last[3] = {}, l = 0;                   // the levels at the three buckets' edges below
+        for (uint32_t b = 0; b < kMixBuckets + 3u; ++b) {
             const double edge = (double)level_interfaces_m[0] + ((double)b - 1.0) * (span / kMixBuckets);
-            while (l + 1 < L && (double)level_interfaces_m[l + 1] <= edge) ++l;
-            table[b] = (uint16_t)l;
+            while (l + 1u < L && (double)level_interfaces_m[l + 1u] <= edge) ++l;
+            if (b < kMixBuckets) table[b] = (uint16_t)l;
+            if (l - last[b % 3u] > kMixScan) search = MIX_BISECT;
+            last[b % 3u] = l;
         }
     }
     cudaStream_t s = c->ctx->pick(stream);
-    FPG_CUDA(cudaMemcpyAsync(c->table, table.data(), kMixBuckets * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
     FPG_CUDA(cudaMemcpyAsync(c->matrix, matrix_column_major, L * L * sizeof(float), cudaMemcpyHostToDevice, s));
-    FPG_CUDA(cudaMemcpyAsync(c->iface, level_interfaces_m, (L + 1) * sizeof(float), cudaMemcpyHostToDevice, s));
-    FPG_CUDA(cudaMemcpyAsync(c->centers, centers.data(), L * sizeof(float), cudaMemcpyHostToDevice, s));
+    FPG_CUDA(cudaMemcpyAsync(c->iface, column.data(), column_bytes(L), cudaMemcpyHostToDevice, s));
     conv_heights_kernel<<<(unsigned)((L + 127) / 128), 128, 0, s>>>((uint32_t)L, c->matrix, c->centers,
                                                                    level_interfaces_m[0], level_interfaces_m[L],
                                                                    c->heights);

@@ -178,7 +178,6 @@ extern "C" fpg_status fpg_compaction_destroy(fpg_compaction* c) {
     if (!c) return FPG_OK;
     cudaFree(c->block);
     cudaFree(c->tile_counts);
-   
     cudaFree(c->active_count_dev);
     cudaFreeHost(c->active_count_host);
     delete c;
