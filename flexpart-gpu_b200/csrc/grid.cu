@@ -136,10 +136,14 @@ __global__ void __launch_bounds__(256) grid_kernel(GridArgs a, LevelTable lt, ui
 // predicated additions per height and no level index.  A warp takes four
 // adjacent slots per lane (16-byte loads, the next four in flight) as long as
 // they lie in its current column; when the column changes, its sums go to the
-// CTA's table, one reduction per value.  A few slots of another column are
-// added to the table one by one.  All sums are u32 modulo 2^32, as the
+// CTA's table, one reduction per value.  A few slots of another column, and
+// slots scattered over many, are added to the table one by one: a change of
+// column pays only when more than half of the lanes go to the new one
+// (10 M particles with 30 % of their slots one cell off: 67 us by run sums,
+// 67 us with a change whenever half of the lanes lie elsewhere, 55 us so; all
+// slots in random order 90, 83, 76 us).  All sums are u32 modulo 2^32, as the
 // grid's, so the differences are exact.  10 M particles of the global run:
-// 57.8 -> 40.0 us, 78 % of the measured HBM bandwidth for 20 B a slot (64
+// 57.8 -> 40 us, 78 % of the measured HBM bandwidth for 20 B a slot (64
 // registers and 4 CTAs per SM; 5 or 6 of them spill or thrash: 42-53 us; the
 // loads of a quad not issued ahead: 42-45 us).
 constexpr uint32_t kQuad = 4;
@@ -270,8 +274,16 @@ __global__ void __launch_bounds__(256, 4) grid_columns_kernel(GridArgs a, LevelT
                 }
             const unsigned left = __ballot_sync(0xffffffffu, pending != 0u);
             if (left == 0u) break;
-            if (column != kNoColumn && (!first || __popc(left) <= kFew)) {
-                // few, or as many again after a change of column: one by one
+            // the first pending slot's column takes over if it is that of many lanes
+            uint32_t next = 0u;
+            bool take = column == kNoColumn;
+            if (first && (take || __popc(left) > kFew)) {
+                const uint32_t mine_col = pending & 1u ? col[0] : pending & 2u ? col[1] : pending & 4u ? col[2] : col[3];
+                next = __shfl_sync(0xffffffffu, mine_col, __ffs(left) - 1);
+                take |= __popc(__ballot_sync(0xffffffffu, pending != 0u && mine_col == next)) > kFew;
+            }
+            if (!take) {
+                // few, scattered, or as many again after a change: one by one
 #pragma unroll
                 for (uint32_t k = 0; k < kQuad; ++k)
                     if (pending >> k & 1u)
@@ -279,9 +291,8 @@ __global__ void __launch_bounds__(256, 4) grid_columns_kernel(GridArgs a, LevelT
                 break;
             }
             flush_column(sums, column, lane, t_key, t_cnt, t_mass, counts, mass);
-            const uint32_t mine_col = pending & 1u ? col[0] : pending & 2u ? col[1] : pending & 4u ? col[2] : col[3];
             first = column == kNoColumn;
-            column = __shfl_sync(0xffffffffu, mine_col, __ffs(left) - 1);
+            column = next;
         }
     }
     flush_column(sums, column, lane, t_key, t_cnt, t_mass, counts, mass);
