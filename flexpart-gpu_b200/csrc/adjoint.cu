@@ -165,26 +165,23 @@ struct TapeRec {
 // whose last receptor hit came before this step has a zero adjoint from this
 // step on, so its tape is never read -- it is marked inactive for the
 // reverse and not stepped.
-// kTapeParts CTAs per 256-slot work item, launched over all items; the level
-// arrays are read from global memory (no staging, no barrier).  Small CTAs
-// fill the last wave: 160 k particles are 625 items, one more than the 592
-// CTAs of 256 threads that are resident (13.6 us a step).  Small CTAs here and
-// a bracket's reverse in one launch (below) together took a 6 h inversion of
-// 160 k particles, forward and backward, from 1,903 to 1,765 us.  The stage
-// settings stay run-time values: set as constants in a copy of the arguments,
-// they put that copy on each thread's stack and the inversion took 180 us more.
-constexpr uint32_t kTapeThreads = 64, kTapeParts = TILE / kTapeThreads;
-
-__global__ void __launch_bounds__(kTapeThreads, 16) inverse_tape_kernel(StepArgs a, const BatchState* st,
+// One CTA per 256-slot work item, launched over all items; the level arrays
+// are read from global memory (no staging, no barrier).  CTAs of 64 threads
+// fill a small run's last wave (160 k particles are 625 items, one more than
+// the 592 CTAs resident), which gives 0.5 % there, but cost a quarter of the
+// pass at 12 M (430 against 361 us).  The stage settings stay run-time values:
+// set as constants in a copy of the arguments, they put that copy on each
+// thread's stack and a 6 h inversion of 160 k particles took 180 us more.
+__global__ void __launch_bounds__(TILE, 4) inverse_tape_kernel(StepArgs a, const BatchState* st,
                                                               const ScenDev* sc,
                                                               const uint2* __restrict__ items, uint32_t n_items,
                                                               TapeBase tb, uint32_t every,
                                                               const uint32_t* live) {
     chain_begin();
-    if (blockIdx.x / kTapeParts >= n_items) return;
-    const uint2 w = items[blockIdx.x / kTapeParts];
+    if (blockIdx.x >= n_items) return;
+    const uint2 w = items[blockIdx.x];
     const ScenDev& d = sc[w.x];
-    const uint32_t local = w.y + blockIdx.x % kTapeParts * kTapeThreads + threadIdx.x;
+    const uint32_t local = w.y + threadIdx.x;
     if (local >= d.released) return;
     const uint32_t slice = st->step % tb.slices;
     TapeRec rec;
@@ -775,7 +772,7 @@ static fpg_status enqueue_taped_step(fpg_inverse* v, uint64_t step, bool recompu
     InverseData& d = v->d;
     const uint32_t side = (uint32_t)(step & 1u);
     enqueue_pre(b, s, side, false, d.st_all, d.sc_all, d.slices);
-    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u) * kTapeParts, kTapeThreads, 0, s, make_step_args(b),
+    launch_chained(inverse_tape_kernel, std::max(d.n_items, 1u), TILE, 0, s, make_step_args(b),
                    b->st + side, b->scen_state(side), d.items, d.n_items, tape_base(v), d.cfg.sample_every_steps,
                    recompute ? d.last_hit : nullptr);
     b->ctx->count(1);
