@@ -59,22 +59,22 @@ ADJOINT_HBM_BUDGET = 140e9  # device bytes the batched adjoint may hold (the 150
 # steps between spatial reorders of the population (one per simulated day at
 # dt 900 s): measured at 10 M particles over 96 steps, a reorder every
 # 24 / 32 / 48 / 96 steps gives 1.297 / 1.318 / 1.324 / 1.335e10
-# particle-steps/s.  A reorder costs about 0.94 ms and the step kernel gains
-# little from it beyond the first step after it (the turbulence mixes the
-# heights within each column at once: 0.582 ms right after a reorder, 0.618
-# ms from the second step on).  The default window of timed steps is one
+# particle-steps/s (of an earlier step kernel, 0.62 ms).  A reorder costs
+# about 0.86 ms and the step kernel gains little from it beyond the first step
+# after it (the turbulence mixes the heights within each column at once:
+# 0.463 ms right after a reorder, 0.500 ms over the 96 steps).  The default window of timed steps is one
 # reorder period, and its first step reorders.
 SORT_EVERY = 96
 # DRAM bytes (read + write) per particle of one fused-step launch, from an
 # ncu capture of a 10 M-particle launch of the global run's population
 # (bench.py --quick: particles around the 8 sources, reordered by met cell
-# before the timed steps): 443.2 MB read + 421.9 MB written = 86.5 B per
+# before the timed steps): 443.2 MB read + 432.0 MB written = 87.5 B per
 # particle against the algorithmic 96 B (44 B read, 52 B written); the last
 # ~100 MB of writes are still in the 126 MB L2 when the kernel ends.
-DRAM_BYTES_PER_PARTICLE_NCU = (443.2e6 + 421.9e6) / 10.0e6
+DRAM_BYTES_PER_PARTICLE_NCU = (443.2e6 + 432.0e6) / 10.0e6
 # Warp instructions per 32 particle-steps (smsp__inst_executed.sum of the
-# same capture: 553.5 M for 10 M particles).
-WARP_INSTRUCTIONS_PER_32_PARTICLES_NCU = 553.5e6 / (10.0e6 / 32)
+# same capture: 451.4 M for 10 M particles).
+WARP_INSTRUCTIONS_PER_32_PARTICLES_NCU = 451.4e6 / (10.0e6 / 32)
 
 
 def issue_roofline(n_particles, kernel_ms, clk):
@@ -369,7 +369,7 @@ def parity_sample(ctx, scn, frames, rec, t, counter):
     within = {k: float((v <= 1e-5).mean()) for k, v in err.items()}
     return {"particles": int(act.sum()), "max_rel_err": out, "share_within_1e-5": within,
             "integers_bit_exact": bool(np.array_equal(g["flags"], o["flags"]) and np.array_equal(g["cbt"], o["cbt"])),
-            "step": "one production step (dry + per-cell wet) of the sample, device fused_step_kernel vs FP32 oracle"}
+            "step": "one production step (dry + per-cell wet) of the sample, device production_step_kernel vs FP32 oracle"}
 
 
 def cpu_sample(scn, args, n):
@@ -1134,7 +1134,7 @@ def main():
                          "traffic_source": "ncu dram__bytes_read+write of a 10M-particle launch (bench.py --quick), "
                                            "scaled by particles",
                          "peak_kind": peak_kind,
-                         "kernel": "fused_step_kernel", "kernel_ms": avg_kernel_ms,
+                         "kernel": "production_step_kernel", "kernel_ms": avg_kernel_ms,
                          "bytes_per_launch": BYTES_PER_PARTICLE_STEP * n_active,
                          # the bound that binds: warp-instruction issue (148 SMs x 4 per clock)
                          "issue": issue_roofline(n_active, avg_kernel_ms, clk)},

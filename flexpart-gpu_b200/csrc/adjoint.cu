@@ -960,7 +960,7 @@ extern "C" fpg_status fpg_inverse_set_sources(fpg_inverse* v, const double* mass
     return FPG_OK;
 }
 
-// Start of the met bracket that step k runs in: batch_advance_kernel's
+// Start of the met bracket that step k runs in: the batch's state kernels'
 // formula at t = start + k dt (at a frame time the bracket ending there).
 static int64_t step_bracket_start(const fpg_batch* b, uint64_t k) {
     const int64_t start = b->cfg.start_seconds, fs = b->cfg.frame_seconds;

@@ -21,7 +21,8 @@
 //   PBL: float4 (u*, w*, hmix, 1/L) per met cell, one 16-byte gather per
 //     particle;
 //   wet forcing per cell: float2 (lambda, fraction).
-// Level heights sit in shared memory beside a 1024-bucket table of level
+// Level heights are read through L1 (the shapes with several particles per
+// thread stage them in shared memory) beside a 1024-bucket table of level
 // indices; for non-decreasing heights the metres->level search reads the
 // bucket's entry and scans up from it (same first index as the reference's
 // linear scan, advection_dual_wind.wgsl:94-117), else it runs the scan.
@@ -50,10 +51,10 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
 }
 
 // The production form of the pass (production_form in step_core.cuh), what
-// the forward loop launches.  Instruction issue binds it: 1,480 warp
-// instructions per 32 particles against 1,771 of the general body, 0.77-0.79
-// of the issue slots used.  At 10 M particles of the global run 609 -> 532 us
-// in a mixed population and 577 -> 479 us right after a reorder.
+// the forward loop launches.  Instruction issue binds it: 1,444 warp
+// instructions per 32 particles against 1,771 of the general body, 0.78-0.84
+// of the issue slots used.  At 10 M particles of the global run 616 -> 501 us
+// over the 96 steps from one reorder to the next, 581 -> 463 us right after it.
 template <bool kWet, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) production_step_kernel(StepArgs a) {
     chain_begin();

@@ -366,7 +366,10 @@ fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* particles, const fpg_met* met,
  * times each candidate workgroup size of the key kernels and keeps the
  * fastest), over CUDA block size, resident blocks per SM and particles per
  * thread.  Every shape gives the same results bit for bit.  The shape is a
- * setting of the context (shape 0, <256, 5, 1>, until changed).
+ * setting of the context (shape 0, <256, 5, 1>, until changed).  Shape 0 also
+ * stands for the forms of the step compiled for common settings (the forward
+ * loop's step, one seam function at a time), whose shapes follow the slot
+ * count; any other shape runs the general kernel.
  * fpg_step_tuning_candidates writes up to `max` compiled shapes and returns
  * their count.  fpg_step_autotune times one fpg_step of `params` under every
  * shape (best of `reps`), each from the same snapshot of the particle state,
