@@ -587,15 +587,6 @@ __device__ __forceinline__ T langevin_v_t(T prev, T sigma_w, T tlw, T dsigwdz, f
     return finitef(val(next)) ? next : T(0.0f);
 }
 
-__device__ __forceinline__ float langevin_h(float prev, float sigma, float tl, float dt, float eta) {
-    return langevin_h_t<float>(prev, sigma, tl, dt, eta);
-}
-
-__device__ __forceinline__ float langevin_v(float prev, float sigma_w, float tlw, float dsigwdz, float dt,
-                                            float rho, float eta) {
-    return langevin_v_t<float>(prev, sigma_w, tlw, dsigwdz, dt, rho, eta);
-}
-
 // ---- the same without the checks that cannot fire ---------------------------
 // For a cell inside plain_cell's bounds and a finite height, sigma and every
 // time scale come out finite and positive, so the reference's sanitising of
