@@ -157,6 +157,10 @@ extern "C" fpg_status fpg_ctx_synchronize(fpg_ctx* c, void* stream) {
 
 extern "C" uint64_t fpg_ctx_kernel_launches(fpg_ctx* c) { return c ? c->launches.load() : 0; }
 
+extern "C" uint64_t fpg_ctx_form_launches(const fpg_ctx* c, int32_t form) {
+    return c && form >= 0 && form < FPG_FORM_COUNT ? c->form_launches[form].load() : 0;
+}
+
 extern "C" fpg_status fpg_device_alloc(fpg_ctx* c, size_t bytes, void** out) {
     if (!c || !out) return FPG_ERR_INVALID_ARGUMENT;
     *out = nullptr;

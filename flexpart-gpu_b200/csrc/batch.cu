@@ -821,6 +821,7 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
     if (b->steps_done >= b->total_steps) return FPG_ERR_SIMULATION_COMPLETE;
     const uint64_t n = std::min<uint64_t>(n_steps, b->total_steps - b->steps_done);
     cudaStream_t s = b->ctx->stream;
+    const bool form = kVariants[b->variant].ppt == 0 && production_form(make_step_args(b));
     for (uint64_t i = 0; i < n; ++i) {
         const uint64_t step = b->steps_done + i;
         if (use_graph) {
@@ -830,6 +831,7 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
             enqueue_batched_step(b, s, step, output_step(b, step));
             FPG_CHECK_LAUNCH();
         }
+        if (form) b->ctx->count_form(FPG_FORM_STEP);
     }
     // keep the host mirror (used by the sequential path) in step
     const uint32_t bpp = b->cfg.n_substeps <= 2u ? 1u : 2u;

@@ -653,14 +653,17 @@ static bool launch_form(fpg_ctx* ctx, StepArgs& a, bool no_carry, cudaStream_t s
     if (production_form(a)) {
         const ProductionShape ps = production_shape_for(a.n, ctx->sm_count);
         launch_chained(a.stages & FPG_STAGE_WET ? ps.wet : ps.dry, blocks_for(a.n, ps.block), ps.block, 0, s, a);
+        ctx->count_form(FPG_FORM_STEP);
         return true;
     }
     if (a.stages == FPG_STAGE_ADVECT && advection_form(a)) {
         launch_chained(advection_kernel, blocks_for(a.n, kStageThreads), kStageThreads, 0, s, a);
+        ctx->count_form(FPG_FORM_ADVECTION);
         return true;
     }
     if (a.stages == FPG_STAGE_TURBULENCE && turbulence_form(a)) {
         launch_chained(turbulence_kernel, blocks_for(a.n, kStageThreads), kStageThreads, 0, s, a);
+        ctx->count_form(FPG_FORM_TURBULENCE);
         return true;
     }
     const bool dry = a.stages == FPG_STAGE_DRY && a.dry_mode == FPG_FORCING_PER_PARTICLE;
@@ -678,6 +681,7 @@ static bool launch_form(fpg_ctx* ctx, StepArgs& a, bool no_carry, cudaStream_t s
         d.dt = a.tdt;
         d.href = a.href;
         launch_chained(dry ? deposition_kernel<false> : deposition_kernel<true>, blocks_for(a.n, 1024), 256, 0, s, d);
+        ctx->count_form(FPG_FORM_DEPOSITION);
         return true;
     }
     return false;
@@ -1113,6 +1117,7 @@ extern "C" fpg_status fpg_langevin_with_hanna(fpg_ctx* ctx, fpg_particles* P, co
         a.keys = philox_keys(a.head);
         launch_chained(blocks > 1u ? langevin_record_plain_kernel<true> : langevin_record_plain_kernel<false>,
                        (unsigned)((n + 63) / 64), 64, 0, ctx->pick(stream), a);
+        ctx->count_form(FPG_FORM_RECORD);
     } else {
         launch_chained(langevin_record_kernel, (unsigned)((n + 255) / 256), 256, 0, ctx->pick(stream), a);
     }

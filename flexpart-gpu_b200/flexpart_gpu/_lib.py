@@ -57,6 +57,7 @@ _sig("fpg_ctx_destroy", _i32, _vp)
 _sig("fpg_ctx_stream", _vp, _vp)
 _sig("fpg_ctx_synchronize", _i32, _vp, _vp)
 _sig("fpg_ctx_kernel_launches", ctypes.c_uint64, _vp)
+_sig("fpg_ctx_form_launches", ctypes.c_uint64, _vp, _i32)
 _sig("fpg_device_alloc", _i32, _vp, _sz, ctypes.POINTER(_vp))
 _sig("fpg_device_free", _i32, _vp, _vp)
 _sig("fpg_memcpy", _i32, _vp, _vp, _vp, _sz, _i32, _vp)
@@ -187,6 +188,7 @@ def check(status: int, what: str) -> None:
 EXPORTED = [
     "fpg_status_string", "fpg_last_cuda_error", "fpg_abi_version",
     "fpg_ctx_create", "fpg_ctx_destroy", "fpg_ctx_stream", "fpg_ctx_synchronize", "fpg_ctx_kernel_launches",
+    "fpg_ctx_form_launches",
     "fpg_device_alloc", "fpg_device_free", "fpg_memcpy", "fpg_memset", "fpg_host_alloc", "fpg_host_free",
     "fpg_particles_create", "fpg_particles_destroy", "fpg_particles_capacity", "fpg_particles_dispatch_count",
     "fpg_particles_set_dispatch_count", "fpg_particles_upload", "fpg_particles_upload_slots",

@@ -61,6 +61,13 @@ class Context:
         return int(lib.fpg_ctx_kernel_launches(self.h))
 
     @property
+    def form_launches(self) -> dict:
+        """Particle passes that ran a kernel compiled for common settings, by
+        kind (fpg_ctx_form_launches)."""
+        names = ("step", "advection", "turbulence", "deposition", "record")
+        return {name: int(lib.fpg_ctx_form_launches(self.h, k)) for k, name in enumerate(names)}
+
+    @property
     def stream(self):
         return lib.fpg_ctx_stream(self.h)
 

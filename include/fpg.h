@@ -143,6 +143,15 @@ fpg_status fpg_ctx_synchronize(fpg_ctx* ctx, void* stream);
 /* Number of kernels this context has launched since creation (all entry
  * points, graph replays counted per kernel node). */
 uint64_t fpg_ctx_kernel_launches(fpg_ctx* ctx);
+/* Of those, the particle passes that ran a kernel compiled for common
+ * settings instead of the general one, by kind: the whole step (fpg_step and
+ * fpg_batch_run), the advection and turbulence seam calls alone, a deposition
+ * seam call, fpg_langevin_with_hanna.  0 for another kind. */
+enum {
+    FPG_FORM_STEP = 0, FPG_FORM_ADVECTION = 1, FPG_FORM_TURBULENCE = 2, FPG_FORM_DEPOSITION = 3, FPG_FORM_RECORD = 4,
+    FPG_FORM_COUNT = 5
+};
+uint64_t fpg_ctx_form_launches(const fpg_ctx* ctx, int32_t form);
 
 /* Plain device buffers for callers without a CUDA allocator of their own
  * (the role wgpu::Buffer plays for the reference's per-slot forcing and
