@@ -174,7 +174,7 @@ __device__ __forceinline__ float2 box_muller(float u0, float u1) {
 // residual x - g^2 from a fused multiply-add (P. Markstein, Computation of
 // elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34,
 // 1990).  No range test and no branch: five instructions.  Equal to sqrtf for
-// every float of that range (checked exhaustively on a B200).
+// every float of that range (tests/native/math_check.cu, on the device).
 __device__ __forceinline__ float rsqrt_of(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -192,6 +192,7 @@ __device__ __forceinline__ float plain_sqrt(float x) {
 // lower one is kept; -2 ln u lies in [1.1e-7, 175]; 2 pi 2^-24 is formed
 // before its product with the integer, which scales exactly; and rintf of the
 // quadrant is an addition of 1.5 2^23, whose low bits are the quadrant.
+// Both forms give box_muller's bits for every word (math_check.cu).
 __device__ __forceinline__ float2 box_muller_plain(uint32_t va, uint32_t vb) {
     const float ru = fmaxf(u32_to_uniform01(va), 1.17549435e-38f);
     const float radius = plain_sqrt(-2.0f * bm_log(ru));
@@ -593,7 +594,8 @@ __device__ __forceinline__ T langevin_v_t(T prev, T sigma_w, T tlw, T dsigwdz, f
 // them (hanna.rs:113-141) and of the updated velocity (langevin.rs:128,168)
 // returns its argument: the functions below leave it out and take the
 // approximate reciprocals once.  sdiv(a, b) is a times rcp(b) in the step's
-// units (the same bits over 3e9 random pairs with |b| in [1e-4, 1e6]), so
+// units (the same bits for every significand of a with 64 b each in [1e-4,
+// 1e6], math_check.cu), so
 // z / h with a kept 1 / h, or two quotients over one sigma_w, round as
 // written there.  d(sigma_w)/dz can still be zero (a neutral cell far above
 // its scale height, or an exact cancellation) and keeps its test.
