@@ -579,14 +579,15 @@ def run_batched(ctx, stream, args, rank, world):
         "gpu_launches": int(launches), "errors": errors,
         "tuning": best, "tuning_candidates": cands,
         "sequential_interleaved": {"value": ps * world / (ms_seq / 1e3), "ms_per_run": ms_seq,
-                                   "path": "fpg_batch_run_sequential: one fused_step_kernel launch per scenario "
-                                           "per step, shared per-step kernels, no graph"},
+                                   "path": "fpg_batch_run_sequential: one launch per scenario per step, "
+                                           "the one fpg_step makes (same form of the step as the batched "
+                                           "pass), shared per-step kernels, no graph"},
         "per_scenario_driver": {"value": ps_sub / t_drv, "scenarios_timed": sub, "seconds": t_drv,
                                 "path": "fpg_forward_run_timestep per scenario, one plain run after another, "
                                         "every met frame resident in the driver's device frame ring"},
         "speedup": ms_seq / ms,
-        "speedup_baseline": "sequential_interleaved: the same run as one plain fused-step launch per scenario "
-                            "per step (per-step kernels shared)",
+        "speedup_baseline": "sequential_interleaved: the same run as one fpg_step launch per scenario per step "
+                            "(the same form of the step, per-step kernels shared)",
         "speedup_vs_interleaved": ms_seq / ms,
         "speedup_vs_per_scenario_driver": value / world / (ps_sub / t_drv),
         "e2e": {"value": ps * world / (ms_e2e / 1e3), "unit": UNIT, "h2d_bytes_per_run": h2d,

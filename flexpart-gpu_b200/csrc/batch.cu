@@ -38,9 +38,6 @@ namespace fpg {
 
 size_t particles_block_bytes(size_t capacity);
 
-// the plain fused step (step.cu), launched once per scenario by the sequential path
-__global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a);
-
 namespace {
 
 
@@ -873,7 +870,7 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
             // the counter advances every step, released particles or not (as the driver's)
             b->counter_h[sidx] = counter_add64(counter, (uint64_t)d.capacity * bpp);
             if (released == 0) continue;
-            // one plain launch of the fused step over this scenario's segment
+            // one launch of the step over this scenario's segment, as fpg_step makes it
             StepArgs a = base;
             const uint32_t o = d.offset;
             a.cell_x += o; a.cell_y += o; a.pos_x += o; a.pos_y += o; a.pos_z += o; a.flags += o;
@@ -883,8 +880,8 @@ extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
             a.alpha = alpha;
             a.key0 = d.key0; a.key1 = d.key1;
             a.counter = counter;
-            fused_step_kernel<<<(released + 255) / 256, 256, 0, s>>>(a);
-            b->ctx->count();
+            const fpg_status st = launch_step(b->ctx, a, s);
+            if (st != FPG_OK) return st;
         }
         enqueue_post(b, s, side, output);
         FPG_CHECK_LAUNCH();

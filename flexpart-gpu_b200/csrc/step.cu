@@ -644,9 +644,10 @@ namespace fpg {
 
 // The kernels for the arguments that have a form of their own; false when
 // they have none and the general body runs.
-static bool launch_form(fpg_ctx* ctx, StepArgs& a, bool no_carry, cudaStream_t s) {
+static bool launch_form(fpg_ctx* ctx, StepArgs& a, cudaStream_t s) {
     if (a.stages & FPG_STAGE_TURBULENCE) {
-        if (!no_carry) return false;
+        // a block's counter carries out of its first word
+        if ((uint64_t)a.counter.x + 2u * (uint64_t)a.n > (1ull << 32)) return false;
         a.head = philox_head(a.counter, a.key0, a.key1);
         a.keys = philox_keys(a.head);
     }
@@ -685,6 +686,17 @@ static bool launch_form(fpg_ctx* ctx, StepArgs& a, bool no_carry, cudaStream_t s
         return true;
     }
     return false;
+}
+
+fpg_status launch_step(fpg_ctx* ctx, StepArgs& a, cudaStream_t s) {
+    if (ctx->step_shape != 0 || !launch_form(ctx, a, s)) {
+        const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
+        const size_t smem = sh.ppt > 1 && (a.stages & FPG_STAGE_ADVECT) ? a.nz * sizeof(float) + FPG_LEVEL_BUCKETS : 0;
+        launch_chained(sh.kernel, blocks_for(a.n, sh.block * sh.ppt), sh.block, smem, s, a);
+    }
+    ctx->count();
+    FPG_CHECK_LAUNCH();
+    return FPG_OK;
 }
 
 }  // namespace fpg
@@ -749,7 +761,6 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     a.n_species = P->n_species;
     a.stages = (adv ? FPG_STAGE_ADVECT : 0u) | (turb ? FPG_STAGE_TURBULENCE : 0u) | (dry ? FPG_STAGE_DRY : 0u) |
                (wet ? FPG_STAGE_WET : 0u);
-    size_t smem = 0;
     if (adv) {
         a.bracket = met->bracket;
         a.nx = (uint32_t)met->nx; a.ny = (uint32_t)met->ny; a.nz = (uint32_t)met->nz;
@@ -761,7 +772,6 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
         a.alpha = fminf(fmaxf(prm->alpha, 0.0f), 1.0f);
         a.dt = prm->dt_seconds;
         a.xs = prm->x_grid_per_meter; a.ys = prm->y_grid_per_meter; a.zs = prm->z_grid_per_meter;
-        smem = level_smem_bytes(met);
         a.heights = met->heights_dev;
     }
     if (turb) {
@@ -792,15 +802,8 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     }
     a.wet_prob = prm->wet_probability_dev;
 
-    cudaStream_t s = ctx->pick(stream);
-    // no block's counter carries out of its first word
-    const bool no_carry = (uint64_t)prm->counter[0] + 2u * (uint64_t)n <= (1ull << 32);
-    if (ctx->step_shape != 0 || !launch_form(ctx, a, no_carry, s)) {
-        const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
-        launch_chained(sh.kernel, blocks_for(n, sh.block * sh.ppt), sh.block, sh.ppt > 1 ? smem : 0, s, a);
-    }
-    ctx->count();
-    FPG_CHECK_LAUNCH();
+    const fpg_status launched = launch_step(ctx, a, ctx->pick(stream));
+    if (launched != FPG_OK) return launched;
     if (turb && next_counter) {
         // gpu/langevin_fused.rs:229-233
         const uint64_t bpp = prm->n_substeps <= 2u ? 1u : 2u;

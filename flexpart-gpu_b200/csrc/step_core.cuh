@@ -88,6 +88,11 @@ inline bool production_form(const StepArgs& a) {
     return a.pnx == a.nx && a.pny == a.ny && advection_form(a) && turbulence_form(a);
 }
 
+// One launch of the pass for slots [0, a.n), as fpg_step makes it: the form
+// the arguments have, under its own launch shape, or the general body under
+// the context's (step.cu).
+fpg_status launch_step(fpg_ctx* ctx, StepArgs& a, cudaStream_t s);
+
 // The search a met's heights allow (host side).
 inline int level_mode(const fpg_met* m) {
     return m->level_table ? LEVELS_TABLE : m->monotonic ? LEVELS_BISECT : LEVELS_SCAN;

@@ -333,9 +333,9 @@ fpg_status fpg_batch_upload_frame(fpg_batch* b, uint32_t k, const float* u, cons
  * captured on the first call), else the same kernels launched one by one.
  * Returns FPG_ERR_SIMULATION_COMPLETE when no step is left. */
 fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_graph);
-/* The same steps with one plain fused-step launch per scenario per step
- * (sequential launches, no graph): the comparison the batching is measured
- * against.  Bit-identical results. */
+/* The same steps with one launch per scenario per step, the one fpg_step
+ * makes for that scenario alone (its form and launch shape; no graph): the
+ * comparison the batching is measured against.  Bit-identical results. */
 fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps);
 /* Steps taken so far; slot range of scenario s; the whole population. */
 uint64_t fpg_batch_steps_done(const fpg_batch* b);

@@ -130,3 +130,19 @@ def test_batched_pass(graph):
     b.tuning = {"block_threads": 256, "min_blocks_per_sm": 4, "particles_per_thread": 1}
     assert _took(ctx, lambda: b.run(2, graph=graph)) == {}
     assert _took(ctx, lambda: batch(0.0).run(3, graph=graph)) == {}
+
+
+def test_sequential_path_launches_what_a_step_of_the_scenario_alone_would():
+    ctx = api.Context(0)
+    met = synthetic.MetSpec(nx=40, ny=30, nz=16, dx_deg=1.0, dy_deg=1.0, xlon0=-20.0, ylat0=30.0, n_frames=3,
+                            frame_seconds=3600, seed=5, wet=True)
+    ens = synthetic.config2(n_scenarios=3, lo=200, hi=2000, hours=2, met=met, seed=11)
+    for src in ens.sources:
+        src.start = src.end = ens.start                      # all released at once
+    scenarios = bt.ensemble_scenarios(ens)
+    scenarios[2].counter[0] = 2**32 - 1                     # carries in the first step
+    b = bt.Batch(ctx, bt.ensemble_config(ens), scenarios, (met.nx, met.ny, met.nz),
+                 synthetic.level_heights(met.nz, met.top_m))
+    bt.upload_ensemble_met(b, ens)
+    assert _took(ctx, lambda: b.run_sequential(1)) == {"step": 2}
+    assert _took(ctx, lambda: b.run_sequential(2)) == {"step": 6}
