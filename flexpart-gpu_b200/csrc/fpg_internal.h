@@ -66,7 +66,10 @@ struct fpg_ctx {
     int sm_count = 0;
     std::atomic<uint64_t> launches{0};
     std::atomic<uint64_t> form_launches[FPG_FORM_COUNT] = {};
-    uint32_t step_shape = 0;                // launch shape of fpg_step (index into its compiled shapes)
+    // fpg_step: the general body's launch shape (index into its compiled
+    // shapes), and whether the forms compiled for common settings run
+    uint32_t step_shape = 0;
+    bool step_forms = true;
     cudaStream_t pick(void* s) const { return s ? static_cast<cudaStream_t>(s) : stream; }
     void count(uint64_t n = 1) { launches.fetch_add(n, std::memory_order_relaxed); }
     void count_form(int form, uint64_t n = 1) { form_launches[form].fetch_add(n, std::memory_order_relaxed); }

@@ -224,7 +224,7 @@ struct StepShape {
 
 // Shape 0 (the default) is the general body for everything outside the
 // production form, which has its own launch shapes; the others run the
-// general body always.
+// general body always (`forms` off).
 const StepShape kStepShapes[] = {
     {256, 5, 1, fused_step_kernel},
     {256, 4, 1, fused_step_shape_kernel<256, 4, 1>},
@@ -688,21 +688,30 @@ static bool launch_form(fpg_ctx* ctx, StepArgs& a, cudaStream_t s) {
     return false;
 }
 
-fpg_status launch_step(fpg_ctx* ctx, StepArgs& a, cudaStream_t s) {
-    if (ctx->step_shape != 0 || !launch_form(ctx, a, s)) {
-        const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
+// With `forms`, the form the arguments have; else, or without one, the
+// general body under `shape`.  *in_form (may be NULL): whether a form ran.
+static fpg_status launch_pass(fpg_ctx* ctx, StepArgs& a, uint32_t shape, bool forms, bool* in_form, cudaStream_t s) {
+    const bool form = forms && launch_form(ctx, a, s);
+    if (!form) {
+        const StepShape& sh = kStepShapes[shape];
         const size_t smem = sh.ppt > 1 && (a.stages & FPG_STAGE_ADVECT) ? a.nz * sizeof(float) + FPG_LEVEL_BUCKETS : 0;
         launch_chained(sh.kernel, blocks_for(a.n, sh.block * sh.ppt), sh.block, smem, s, a);
     }
     ctx->count();
     FPG_CHECK_LAUNCH();
+    if (in_form) *in_form = form;
     return FPG_OK;
+}
+
+fpg_status launch_step(fpg_ctx* ctx, StepArgs& a, cudaStream_t s) {
+    return launch_pass(ctx, a, ctx->step_shape, ctx->step_forms, nullptr, s);
 }
 
 }  // namespace fpg
 
-extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* met, const fpg_pbl* pbl,
-                               const fpg_step_params* prm, uint32_t next_counter[4], void* stream) {
+static fpg_status step_pass(fpg_ctx* ctx, fpg_particles* P, const fpg_met* met, const fpg_pbl* pbl,
+                            const fpg_step_params* prm, uint32_t next_counter[4], uint32_t shape, bool forms,
+                            bool* in_form, void* stream) {
     if (!ctx || !P || !prm) return FPG_ERR_INVALID_ARGUMENT;
     if (next_counter) std::memcpy(next_counter, prm->counter, sizeof(uint32_t) * 4);
     const size_t n = P->dispatch;
@@ -802,7 +811,7 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
     }
     a.wet_prob = prm->wet_probability_dev;
 
-    const fpg_status launched = launch_step(ctx, a, ctx->pick(stream));
+    const fpg_status launched = launch_pass(ctx, a, shape, forms, in_form, ctx->pick(stream));
     if (launched != FPG_OK) return launched;
     if (turb && next_counter) {
         // gpu/langevin_fused.rs:229-233
@@ -810,6 +819,12 @@ extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* me
         counter_add64(prm->counter, (uint64_t)n * bpp, next_counter);
     }
     return FPG_OK;
+}
+
+extern "C" fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* P, const fpg_met* met, const fpg_pbl* pbl,
+                               const fpg_step_params* prm, uint32_t next_counter[4], void* stream) {
+    if (!ctx) return FPG_ERR_INVALID_ARGUMENT;
+    return step_pass(ctx, P, met, pbl, prm, next_counter, ctx->step_shape, ctx->step_forms, nullptr, stream);
 }
 
 namespace fpg {
@@ -828,6 +843,7 @@ extern "C" fpg_status fpg_step_set_tuning(fpg_ctx* ctx, const fpg_batch_tuning* 
         if (kStepShapes[v].block == t->block_threads && kStepShapes[v].minb == t->min_blocks_per_sm &&
             kStepShapes[v].ppt == t->particles_per_thread) {
             ctx->step_shape = v;
+            ctx->step_forms = v == 0;
             return FPG_OK;
         }
     return FPG_ERR_INVALID_ARGUMENT;
@@ -835,14 +851,17 @@ extern "C" fpg_status fpg_step_set_tuning(fpg_ctx* ctx, const fpg_batch_tuning* 
 
 extern "C" fpg_status fpg_step_get_tuning(const fpg_ctx* ctx, fpg_batch_tuning* t) {
     if (!ctx || !t) return FPG_ERR_INVALID_ARGUMENT;
-    const StepShape& sh = kStepShapes[ctx->step_shape < kNumStepShapes ? ctx->step_shape : 0];
+    const StepShape& sh = kStepShapes[ctx->step_shape];
     *t = fpg_batch_tuning{sh.block, sh.minb, sh.ppt, 0.0f};
     return FPG_OK;
 }
 
 // auto_tune_key_kernels (src/gpu/workgroup.rs:377-440) for the fused step:
 // every compiled shape timed from one snapshot of the particle arrays (the
-// restore copy also evicts them from L2), fastest kept.
+// restore copy also evicts them from L2), fastest kept.  Shape 0 is timed as
+// the form the call has, if it has one.  The forms are left off only when a
+// general shape was faster than this call's own form: a tuning of settings
+// without a form says nothing about the calls that have one.
 extern "C" fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* P, const fpg_met* met, const fpg_pbl* pbl,
                                         const fpg_step_params* prm, uint32_t reps, fpg_batch_tuning* results,
                                         uint32_t max_results, fpg_batch_tuning* best, void* stream) {
@@ -850,11 +869,11 @@ extern "C" fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* P, const fp
     if (reps == 0) reps = 1;
     cudaStream_t s = ctx->pick(stream);
     const size_t bytes = particles_block_bytes(P->capacity);
-    const uint32_t keep = ctx->step_shape;
     void* snap = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     fpg_status status = FPG_OK;
-    uint32_t best_v = keep < kNumStepShapes ? keep : 0;
+    uint32_t best_v = 0;
+    bool has_form = false;
     float best_ms = 0.0f;
     cudaError_t e = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = cudaMalloc(&snap, bytes);
@@ -862,13 +881,13 @@ extern "C" fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* P, const fp
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaMemcpyAsync(snap, P->block, bytes, cudaMemcpyDeviceToDevice, s);
     for (uint32_t v = 0; e == cudaSuccess && status == FPG_OK && v < kNumStepShapes; ++v) {
-        ctx->step_shape = v;
         float tmin = 0.0f;
+        bool form = false;
         for (uint32_t r = 0; r < reps; ++r) {
             e = cudaMemcpyAsync(P->block, snap, bytes, cudaMemcpyDeviceToDevice, s);
             if (e == cudaSuccess) e = cudaEventRecord(e0, s);
             if (e != cudaSuccess) break;
-            status = fpg_step(ctx, P, met, pbl, prm, nullptr, s);
+            status = step_pass(ctx, P, met, pbl, prm, nullptr, v, v == 0, &form, s);
             if (status != FPG_OK) break;
             e = cudaEventRecord(e1, s);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -880,6 +899,7 @@ extern "C" fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* P, const fp
         if (e != cudaSuccess || status != FPG_OK) break;
         if (results && v < max_results)
             results[v] = fpg_batch_tuning{kStepShapes[v].block, kStepShapes[v].minb, kStepShapes[v].ppt, tmin};
+        has_form |= form;
         if (v == 0 || tmin < best_ms) { best_ms = tmin; best_v = v; }
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(P->block, snap, bytes, cudaMemcpyDeviceToDevice, s);
@@ -887,11 +907,9 @@ extern "C" fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* P, const fp
     cudaFree(snap);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    if (e != cudaSuccess || status != FPG_OK) {
-        ctx->step_shape = keep;
-        return e != cudaSuccess ? cuda_status(e) : status;
-    }
+    if (e != cudaSuccess || status != FPG_OK) return e != cudaSuccess ? cuda_status(e) : status;
     ctx->step_shape = best_v;
+    ctx->step_forms = !has_form || best_v == 0;
     if (best) *best = fpg_batch_tuning{kStepShapes[best_v].block, kStepShapes[best_v].minb, kStepShapes[best_v].ppt,
                                        best_ms};
     return FPG_OK;

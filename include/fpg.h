@@ -375,18 +375,20 @@ fpg_status fpg_step(fpg_ctx* ctx, fpg_particles* particles, const fpg_met* met,
  * times each candidate workgroup size of the key kernels and keeps the
  * fastest), over CUDA block size, resident blocks per SM and particles per
  * thread.  Every shape gives the same results bit for bit.  The shape is a
- * setting of the context (shape 0, <256, 5, 1>, until changed).  Shape 0 also
- * stands for the forms of the step compiled for common settings (the forward
- * loop's step, one seam function at a time), whose shapes follow the slot
- * count; any other shape runs the general kernel.
+ * setting of the context (shape 0, <256, 5, 1>, until changed) and that of
+ * the general kernel: the kernels compiled for common settings
+ * (fpg_ctx_form_launches) have shapes of their own, by the slot count, and
+ * run wherever their settings hold, unless another shape than 0 is selected
+ * by hand or a tuning found one faster than the compiled kernel of its call.
  * fpg_step_tuning_candidates writes up to `max` compiled shapes and returns
  * their count.  fpg_step_autotune times one fpg_step of `params` under every
- * shape (best of `reps`), each from the same snapshot of the particle state,
- * restores the state, keeps the fastest shape in the context and returns it
+ * shape (best of `reps`; shape 0 as the compiled kernel if `params` have one),
+ * each from the same snapshot of the particle state, restores the state, keeps the fastest shape in the context and returns it
  * in `best`; it needs device memory for one copy of the particle arrays, and
  * the Philox counter is not advanced.  `results` (candidate order) and `best`
  * may be NULL.  fpg_step_set_tuning selects a compiled shape
- * (FPG_ERR_INVALID_ARGUMENT if none matches). */
+ * (FPG_ERR_INVALID_ARGUMENT if none matches); any but shape 0 runs the general
+ * kernel for every call. */
 uint32_t fpg_step_tuning_candidates(fpg_batch_tuning* out, uint32_t max);
 fpg_status fpg_step_autotune(fpg_ctx* ctx, fpg_particles* particles, const fpg_met* met, const fpg_pbl* pbl,
                              const fpg_step_params* params, uint32_t reps, fpg_batch_tuning* results,

@@ -80,6 +80,28 @@ def test_species_and_a_shape_selected_by_hand_run_the_general_body(world):
     assert _took(ctx, lambda: api.step(ctx, p, m, pbl, production_params())) == {"step": 1}
 
 
+@pytest.mark.parametrize("n", [97, 1003, 40_001, 300_007])
+def test_tuning_settings_without_a_form_leaves_the_forms_on(world, n):
+    """Whatever shape wins for two species, calls with a form still run it;
+    a tuning of those keeps a shape it measured, and selecting shape 0 by hand
+    brings the forms back."""
+    ctx, _, m, pbl, _ = world
+    p2, p = _particles(world, n, species=2), _particles(world, n)
+    best, cands = api.step_autotune(ctx, p2, m, pbl, production_params(), reps=3)
+    assert best["step_ms"] == min(c["step_ms"] for c in cands)
+    got = api.get_step_tuning(ctx)
+    assert all(got[k] == best[k] for k in ("block_threads", "min_blocks_per_sm", "particles_per_thread"))
+    assert _took(ctx, lambda: api.step(ctx, p2, m, pbl, production_params())) == {}
+    assert _took(ctx, lambda: api.step(ctx, p, m, pbl, production_params())) == {"step": 1}
+    assert _took(ctx, lambda: api.advect_dual_wind(ctx, p, m, 0.3, 900.0, 2.5e-5, 1.8e-5)) == {"advection": 1}
+    first = api.step_tuning_candidates()[0]
+    best, _ = api.step_autotune(ctx, p, m, pbl, production_params(), reps=3)
+    in_form = all(best[k] == first[k] for k in ("block_threads", "min_blocks_per_sm", "particles_per_thread"))
+    assert _took(ctx, lambda: api.step(ctx, p, m, pbl, production_params())) == ({"step": 1} if in_form else {})
+    api.set_step_tuning(ctx, first)
+    assert _took(ctx, lambda: api.step(ctx, p, m, pbl, production_params())) == {"step": 1}
+
+
 @pytest.mark.parametrize("species,shift", [(1, 0), (4, 0), (1, 1)])
 def test_seam_calls(world, species, shift):
     ctx, _, m, pbl, _ = world
