@@ -311,6 +311,12 @@ const StepVariant kVariants[] = {
 };
 static_assert(sizeof(kVariants) / sizeof(kVariants[0]) == kNumVariants, "launch shape table");
 
+// What shape v runs for these arguments.  In the production form the two flat
+// shapes of 128 threads are one kernel.
+StepKernel pass_kernel(const StepVariant& v, const StepArgs& a) {
+    return v.ppt == 0 && production_form(a) ? v.production[a.wet_mode == FPG_FORCING_PER_CELL] : v.kernel;
+}
+
 struct GridConst {
     uint32_t nx, ny, nz, cells;
     int meters, sorted;
@@ -532,8 +538,7 @@ void enqueue_step_kernel(fpg_batch* b, cudaStream_t s, uint32_t side) {
     const StepVariant& v = kVariants[b->variant];
     const StepArgs a = make_step_args(b);
     if (v.ppt == 0) {
-        const StepKernel kernel = production_form(a) ? v.production[a.wet_mode == FPG_FORCING_PER_CELL] : v.kernel;
-        launch_chained(kernel, std::max(b->n_items, 1u), v.block, 0, s, a, b->st + side,
+        launch_chained(pass_kernel(v, a), std::max(b->n_items, 1u), v.block, 0, s, a, b->st + side,
                        b->scen_state(side), b->items, b->n_items);
     } else {
         const uint32_t grid = (uint32_t)b->ctx->sm_count * std::max(b->resident[b->variant], 1u);
@@ -818,7 +823,7 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
     if (b->steps_done >= b->total_steps) return FPG_ERR_SIMULATION_COMPLETE;
     const uint64_t n = std::min<uint64_t>(n_steps, b->total_steps - b->steps_done);
     cudaStream_t s = b->ctx->stream;
-    const bool form = kVariants[b->variant].ppt == 0 && production_form(make_step_args(b));
+    const bool form = pass_kernel(kVariants[b->variant], make_step_args(b)) != kVariants[b->variant].kernel;
     for (uint64_t i = 0; i < n; ++i) {
         const uint64_t step = b->steps_done + i;
         if (use_graph) {
@@ -953,8 +958,9 @@ extern "C" fpg_status fpg_batch_get_tuning(const fpg_batch* b, fpg_batch_tuning*
 // Times the particle pass of the next step under every compiled launch
 // shape, each from the same snapshot of the live state (population, clock,
 // release and counter state), restores the snapshot and keeps the fastest
-// shape.  Each particle's arithmetic does not depend on the launch shape, so
-// the choice changes speed only, never results.
+// shape; two shapes that run one kernel are timed once.  Each particle's
+// arithmetic does not depend on the launch shape, so the choice changes speed
+// only, never results.
 extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_tuning* results, uint32_t max_results,
                                          fpg_batch_tuning* best) {
     if (!b) return FPG_ERR_INVALID_ARGUMENT;
@@ -986,10 +992,14 @@ extern "C" fpg_status fpg_batch_autotune(fpg_batch* b, uint32_t reps, fpg_batch_
         if (r == cudaSuccess) r = cudaMemcpyAsync(b->sc, sc_snap, sc_bytes, cudaMemcpyDeviceToDevice, s);
         return r;
     };
+    const StepArgs args = make_step_args(b);
+    float time_of[kNumVariants] = {};
     for (uint32_t v = 0; e == cudaSuccess && status == FPG_OK && v < kNumVariants; ++v) {
-        status = build_items(b, v);
-        float tmin = 0.0f;
-        for (uint32_t r = 0; status == FPG_OK && e == cudaSuccess && r < reps; ++r) {
+        uint32_t same = 0;                               // the first shape that runs this kernel
+        while (pass_kernel(kVariants[same], args) != pass_kernel(kVariants[v], args)) ++same;
+        float& tmin = time_of[v];
+        if (same < v) tmin = time_of[same]; else status = build_items(b, v);
+        for (uint32_t r = 0; same == v && status == FPG_OK && e == cudaSuccess && r < reps; ++r) {
             e = restore();
             if (e != cudaSuccess) break;
             enqueue_pre(b, s, side, false, nullptr, nullptr, 0);

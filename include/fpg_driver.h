@@ -353,7 +353,10 @@ fpg_status fpg_batch_errors(fpg_batch* b, int32_t* flags);
  * block_threads * particles_per_thread consecutive slots of one scenario),
  * which persistent CTAs pull from a counter.  particles_per_thread 0 is the
  * non-persistent pass: one CTA per item of block_threads slots, one slot per
- * thread, launched over all items.  step_ms is the particle pass's time
+ * thread, launched over all items.  With the settings of the compiled step
+ * (fpg_ctx_form_launches) a non-persistent pass is compiled for 1280 threads
+ * per SM whatever min_blocks_per_sm says, so the two of 128 threads are one
+ * kernel there, timed once.  step_ms is the particle pass's time
  * measured by the tuner (0 when set by hand).
  * The compiled launch shapes: writes up to max of them, returns their count. */
 uint32_t fpg_batch_tuning_candidates(fpg_batch_tuning* out, uint32_t max);

@@ -154,6 +154,29 @@ def test_batched_pass(graph):
     assert _took(ctx, lambda: batch(0.0).run(3, graph=graph)) == {}
 
 
+def test_tuner_times_one_kernel_once():
+    """In the production form the flat shapes of 128 threads run one kernel and
+    report one time; in the general body they are two."""
+    ctx = api.Context(0)
+    met = synthetic.MetSpec(nx=40, ny=30, nz=16, dx_deg=1.0, dy_deg=1.0, xlon0=-20.0, ylat0=30.0, n_frames=3,
+                            frame_seconds=3600, seed=5, wet=True)
+    ens = synthetic.config2(n_scenarios=3, lo=200, hi=2000, hours=2, met=met, seed=11)
+    times = {}
+    for dry in (0.002, 0.0):
+        ens.dry_velocity = dry
+        b = bt.Batch(ctx, bt.ensemble_config(ens), bt.ensemble_scenarios(ens), (met.nx, met.ny, met.nz),
+                     synthetic.level_heights(met.nz, met.top_m))
+        bt.upload_ensemble_met(b, ens)
+        launches = ctx.kernel_launches
+        best, cands = b.autotune(reps=1)
+        assert best["step_ms"] == min(c["step_ms"] for c in cands) > 0.0
+        flat = [c["step_ms"] for c in cands if c["particles_per_thread"] == 0 and c["block_threads"] == 128]
+        times[dry] = (len(cands), ctx.kernel_launches - launches, flat)
+    (n, launches, flat), (n_general, launches_general, _) = times[0.002], times[0.0]
+    assert len(flat) == 2 and flat[0] == flat[1]
+    assert n == n_general and launches_general == 2 * n and launches == 2 * (n - 1)
+
+
 def test_sequential_path_launches_what_a_step_of_the_scenario_alone_would():
     ctx = api.Context(0)
     met = synthetic.MetSpec(nx=40, ny=30, nz=16, dx_deg=1.0, dy_deg=1.0, xlon0=-20.0, ylat0=30.0, n_frames=3,
