@@ -104,7 +104,7 @@ __device__ __forceinline__ int receptor_at(const Receptors& r, uint32_t inst, in
 // ---- forward sampling ---------------------------------------------------------
 
 __global__ void __launch_bounds__(256) inverse_sample_kernel(const BatchState* st, const ScenDev* sc,
-                                                             const uint2* __restrict__ items, uint32_t n_items,
+                                                             const uint2* items, uint32_t n_items,
                                                              PopFields F, Receptors r) {
     chain_begin();
     if (r.every == 0 || (st->step + 1u) % r.every != 0u) return;
@@ -174,7 +174,7 @@ struct TapeRec {
 // thread's stack and a 6 h inversion of 160 k particles took 180 us more.
 __global__ void __launch_bounds__(TILE, 4) inverse_tape_kernel(StepArgs a, const BatchState* st,
                                                               const ScenDev* sc,
-                                                              const uint2* __restrict__ items, uint32_t n_items,
+                                                              const uint2* items, uint32_t n_items,
                                                               TapeBase tb, uint32_t every,
                                                               const uint32_t* live) {
     chain_begin();
@@ -526,7 +526,7 @@ __device__ __forceinline__ void flush_bias_table(uint32_t* key, float* g, double
 // The reverse of step `slice`'s tape over all items: persistent CTAs, one
 // bias table per CTA for all of its items.
 __global__ void __launch_bounds__(256, 4) inverse_adjoint_kernel(StepArgs a, const BatchState* st, const ScenDev* sc,
-                                                                 const uint2* __restrict__ items, uint32_t n_items,
+                                                                 const uint2* items, uint32_t n_items,
                                                                  uint32_t* work, TapeBase tb, uint32_t slice,
                                                                  LamArrays lam, Receptors r, double* dbias,
                                                                  double* dsrc) {
@@ -578,7 +578,7 @@ constexpr uint32_t kReverseItems = 4096;
 
 __global__ void __launch_bounds__(256, 4) inverse_reverse_kernel(StepArgs a, const BatchState* st_all,
                                                                  const ScenDev* sc_all, uint32_t n_scen,
-                                                                 const uint2* __restrict__ items, TapeBase tb,
+                                                                 const uint2* items, TapeBase tb,
                                                                  uint32_t last, uint32_t count, LamArrays lam,
                                                                  Receptors r, double* dbias, double* dsrc) {
     chain_begin();

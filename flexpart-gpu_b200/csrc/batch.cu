@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kPreThreads) batch_pre_kernel(const BatchState
 template <int BLOCK, int MINB, int PPT>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_step_kernel(StepArgs a, BatchState* st,
                                                                  const ScenDev* sc,
-                                                                 const uint2* __restrict__ items, uint32_t n_items) {
+                                                                 const uint2* items, uint32_t n_items) {
     chain_begin();
     extern __shared__ float s_levels[];
     __shared__ uint32_t s_item;
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step_kernel(StepArgs a, Bat
 template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_step_flat_kernel(StepArgs a, BatchState* st,
                                                                       const ScenDev* sc,
-                                                                      const uint2* __restrict__ items,
+                                                                      const uint2* items,
                                                                       uint32_t n_items) {
     chain_begin();
     if (blockIdx.x >= n_items) return;
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_step_flat_kernel(StepArgs a
 template <bool kWet, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) batch_production_kernel(StepArgs a, BatchState* st,
                                                                        const ScenDev* sc,
-                                                                       const uint2* __restrict__ items,
+                                                                       const uint2* items,
                                                                        uint32_t n_items) {
     chain_begin();
     if (blockIdx.x >= n_items) return;
@@ -333,7 +333,7 @@ struct GridConst {
 // are summed by the segmented scan, the run ends add to the table, and the
 // table goes to the grids once per cell per CTA (grid_core.cuh).
 __global__ void __launch_bounds__(256) batch_grid_kernel(const BatchState* st, const ScenDev* sc,
-                                                         const uint32_t* __restrict__ tile_scen, PopFields F,
+                                                         const uint32_t* tile_scen, PopFields F,
                                                          GridConst g, uint32_t n_tiles, uint32_t tiles_per_cta,
                                                          uint32_t* counts, uint32_t* mass) {
     chain_begin();

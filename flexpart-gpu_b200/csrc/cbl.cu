@@ -196,19 +196,19 @@ template <int kSearch>
 __device__ __forceinline__ uint32_t source_level(float z, float z_min, const MixColumn& c) {
     if constexpr (kSearch == MIX_TABLE) {
         const uint32_t b = min(__float2uint_rz((z - z_min) * c.inv_w), kMixBuckets - 1u);
-        uint32_t lo = __ldg(c.table + b);
-        while (lo + 1u < c.L && __ldg(c.iface + lo + 1u) <= z) ++lo;
+        uint32_t lo = c.table[b];
+        while (lo + 1u < c.L && c.iface[lo + 1u] <= z) ++lo;
         return lo;
     } else if constexpr (kSearch == MIX_BISECT) {
         uint32_t lo = 0u, hi = c.L;               // count of iface[0..L) <= z lies in [1, L]
         while (hi - lo > 1u) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(c.iface + mid) <= z) lo = mid; else hi = mid;
+            if (c.iface[mid] <= z) lo = mid; else hi = mid;
         }
         return lo;
     } else {
         for (uint32_t l = 0; l < c.L; ++l)
-            if (z >= __ldg(c.iface + l) && z < __ldg(c.iface + l + 1u)) return l;
+            if (z >= c.iface[l] && z < c.iface[l + 1u]) return l;
         return c.L - 1u;
     }
 }
@@ -219,7 +219,7 @@ template <int kSearch>
 __device__ __forceinline__ float mix_height(float z_in, float z_min, float z_max, const MixColumn& c, int32_t& level_out) {
     const uint32_t level = source_level<kSearch>(clampf(z_in, z_min, z_max), z_min, c);
     level_out = (int32_t)level;
-    return __ldg(c.heights + level);
+    return c.heights[level];
 }
 
 // Four slots per thread: the flags and heights of a quad arrive in one
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) conv_apply_kernel(size_t n, const uint32_
     chain_begin();
     const size_t p0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4u;
     if (p0 >= n) return;
-    const float z_min = __ldg(c.iface), z_max = __ldg(c.iface + c.L);
+    const float z_min = c.iface[0], z_max = c.iface[c.L];
     if (p0 + 4u <= n) {
         const uint4 f = *reinterpret_cast<const uint4*>(flags + p0);
         const float4 z = *reinterpret_cast<const float4*>(pos_z + p0);

@@ -240,8 +240,7 @@ constexpr uint32_t kNumStepShapes = sizeof(kStepShapes) / sizeof(kStepShapes[0])
 
 // ---- per-cell kernels --------------------------------------------------------
 
-__global__ void __launch_bounds__(256) pbl_diag_kernel(const fpg_surface_cell* __restrict__ s0,
-                                                       const fpg_surface_cell* __restrict__ s1, float alpha,
+__global__ void __launch_bounds__(256) pbl_diag_kernel(const fpg_surface_cell* s0, const fpg_surface_cell* s1, float alpha,
                                                        fpg_pbl_options o, uint32_t ncell, float* ustar_o,
                                                        float* wstar_o, float* hmix_o, float* oli_o, float* sshf_o,
                                                        float* ssr_o, float* surfstr_o, float4* packed,

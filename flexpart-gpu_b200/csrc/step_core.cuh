@@ -122,7 +122,7 @@ __device__ __forceinline__ Levels stage_levels(const StepArgs& a, float* smem) {
     uint32_t* tab = reinterpret_cast<uint32_t*>(smem + a.nz);
     if (a.level_mode == LEVELS_TABLE)
         for (uint32_t i = threadIdx.x; i < FPG_LEVEL_BUCKETS / 4u; i += blockDim.x)
-            tab[i] = __ldg(reinterpret_cast<const uint32_t*>(a.level_table) + i);
+            tab[i] = reinterpret_cast<const uint32_t*>(a.level_table)[i];
     return Levels{smem, reinterpret_cast<const uint8_t*>(tab), a.level_inv_w, a.nz, a.has_heights, a.level_mode};
 }
 
