@@ -624,22 +624,33 @@ fpg_status batch_reset(fpg_batch* b) {
 
 // The graph of a step, by its side of the state (1) and whether it ends with
 // grids (2).
-static fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
-    const bool output = output_step(b, step);
-    const int which = (int)(step & 1u) + (output ? 2 : 0);
-    if (!b->exec[which]) {
-        FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        const uint64_t before = b->ctx->launches.load();
-        enqueue_batched_step(b, s, step, output);
-        // capture launches nothing: take the count back, keep it per replay
-        b->graph_launches[which] = b->ctx->launches.load() - before;
-        b->ctx->launches.fetch_sub(b->graph_launches[which]);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(s, &g);
-        if (e != cudaSuccess) return cuda_status(e);
-        b->graph[which] = g;
-        FPG_CUDA(cudaGraphInstantiate(&b->exec[which], g, 0));
+static int graph_of(const fpg_batch* b, uint64_t step) { return (int)(step & 1u) + (output_step(b, step) ? 2 : 0); }
+
+// Captures the graph of `step` if it is not held yet.
+static fpg_status ensure_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
+    const int which = graph_of(b, step);
+    if (b->exec[which]) return FPG_OK;
+    FPG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    const uint64_t before = b->ctx->launches.load();
+    enqueue_batched_step(b, s, step, output_step(b, step));
+    // capture launches nothing: take the count back, keep it per replay
+    b->graph_launches[which] = b->ctx->launches.load() - before;
+    b->ctx->launches.fetch_sub(b->graph_launches[which]);
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(s, &g);
+    if (e != cudaSuccess) return cuda_status(e);
+    e = cudaGraphInstantiate(&b->exec[which], g, 0);
+    if (e != cudaSuccess) {
+        b->exec[which] = nullptr;
+        cudaGraphDestroy(g);
+        return cuda_status(e);
     }
+    b->graph[which] = g;
+    return FPG_OK;
+}
+
+static fpg_status launch_step_graph(fpg_batch* b, uint64_t step, cudaStream_t s) {
+    const int which = graph_of(b, step);
     FPG_CUDA(cudaGraphLaunch(b->exec[which], s));
     b->ctx->count(b->graph_launches[which]);
     return FPG_OK;
@@ -824,20 +835,30 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
     const uint64_t n = std::min<uint64_t>(n_steps, b->total_steps - b->steps_done);
     cudaStream_t s = b->ctx->stream;
     const bool form = pass_kernel(kVariants[b->variant], make_step_args(b)) != kVariants[b->variant].kernel;
-    for (uint64_t i = 0; i < n; ++i) {
-        const uint64_t step = b->steps_done + i;
+    // every graph of the run before its first step: a capture that fails
+    // leaves the batch as it was
+    for (uint64_t i = 0; use_graph && i < n; ++i) {
+        const fpg_status st = ensure_graph(b, b->steps_done + i, s);
+        if (st != FPG_OK) return st;
+    }
+    fpg_status st = FPG_OK;
+    uint64_t done = 0;
+    for (; done < n; ++done) {
+        const uint64_t step = b->steps_done + done;
         if (use_graph) {
-            const fpg_status st = launch_step_graph(b, step, s);
-            if (st != FPG_OK) return st;
+            st = launch_step_graph(b, step, s);
         } else {
             enqueue_batched_step(b, s, step, output_step(b, step));
-            FPG_CHECK_LAUNCH();
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) st = cuda_status(e);
         }
+        if (st != FPG_OK) break;
         if (form) b->ctx->count_form(FPG_FORM_STEP);
     }
-    // keep the host mirror (used by the sequential path) in step
+    // keep the host mirror (used by the sequential path) and the state's side
+    // with the steps launched
     const uint32_t bpp = b->cfg.n_substeps <= 2u ? 1u : 2u;
-    for (uint64_t i = 0; i < n; ++i) {
+    for (uint64_t i = 0; i < done; ++i) {
         for (size_t k = 0; k < b->scen.size(); ++k) {
             const ScenDev& d = b->scen[k];
             uint32_t hi = target_emitted(d.start, d.end, d.count, b->t_h, b->released_h[k]);
@@ -846,8 +867,8 @@ extern "C" fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_
         }
         b->t_h += b->cfg.timestep_seconds;
     }
-    b->steps_done += n;
-    return FPG_OK;
+    b->steps_done += done;
+    return st;
 }
 
 extern "C" fpg_status fpg_batch_run_sequential(fpg_batch* b, uint32_t n_steps) {
