@@ -595,7 +595,7 @@ def run_batched(ctx, stream, args, rank, world):
                 "path": "fpg_batch_upload_frame x9 + fpg_batch_run + fpg_batch_download_grids "
                         "(page-locked host buffers)"},
         "roofline": {"bound": "hbm",
-                     "kernel": "batch_step_flat_kernel" if best["particles_per_thread"] == 0 else "batch_step_kernel",
+                     "kernel": "batch_production_kernel" if best["particles_per_thread"] == 0 else "batch_step_kernel",
                      "particles_per_launch": pass_particles,
                      "kernel_ms": best["step_ms"], "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind},

@@ -23,8 +23,8 @@
 // The tape is recorded either during the forward itself (checkpoint_every
 // == 0: one tape slice per step, no recompute) or, to bound memory, per
 // K-step window from checkpoints during the backward.  Tape slices are
-// indexed on the device by step % slices, so one captured graph serves
-// every step of either mode.
+// indexed by step % slices.  The steps of either mode are launched one by
+// one, each kernel chained to the one before it (launch_chained).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -35,7 +35,8 @@ fpg_status cuda_status(cudaError_t e);
 // to memory, in every CTA, and reads what earlier kernels of the stream write
 // through plain pointers: a load marked read-only for the kernel's life
 // (__restrict__ const, __ldg) whose address does not come from memory could
-// be moved above the wait.
+// be moved above the wait.  That holds for buffers that only copies write
+// today, too: a kernel that fills them later would break it silently.
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchAttribute attr{};

@@ -595,10 +595,10 @@ __device__ __forceinline__ T langevin_v_t(T prev, T sigma_w, T tlw, T dsigwdz, f
 // returns its argument: the functions below leave it out and take the
 // approximate reciprocals once.  sdiv(a, b) is a times rcp(b) in the step's
 // units (the same bits for every significand of a with 64 b each in [1e-4,
-// 1e6], math_check.cu), so
-// z / h with a kept 1 / h, or two quotients over one sigma_w, round as
-// written there.  d(sigma_w)/dz can still be zero (a neutral cell far above
-// its scale height, or an exact cancellation) and keeps its test.
+// 1e6], math_check.cu), so z / h with a kept 1 / h, or two quotients over one
+// sigma_w, round as written there.  d(sigma_w)/dz can still be zero (a neutral
+// cell far above its scale height, or an exact cancellation) and keeps its
+// test.
 __device__ __forceinline__ float rcp_of(float b) {
 #ifdef FPG_RECIPROCAL_DIVISION
     float r;

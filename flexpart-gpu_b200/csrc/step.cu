@@ -50,8 +50,9 @@ __global__ void __launch_bounds__(256, 5) fused_step_kernel(StepArgs a) {
     particle_step(a, lv, p, p, a.alpha, a.counter, a.key0, a.key1);
 }
 
-// The production form of the pass (production_form in step_core.cuh), what
-// the forward loop launches.  Instruction issue binds it: 1,444 warp
+// The production form of the pass (production_form in step_core.cuh): what a
+// run with one species, a dry deposition velocity and per-cell wet forcing or
+// none launches.  Instruction issue binds it: 1,444 warp
 // instructions per 32 particles against 1,771 of the general body, 0.78-0.84
 // of the issue slots used.  At 10 M particles of the global run 616 -> 501 us
 // over the 96 steps from one reorder to the next, 581 -> 463 us right after it.

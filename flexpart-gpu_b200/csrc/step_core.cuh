@@ -57,10 +57,14 @@ struct StepArgs {
     PhiloxKeys keys;                     // for the production form
 };
 
-// The production form of the step (production_step below): the forward
-// loop's own settings.  It is taken when every one of these holds, which the
-// host sees from the arguments; anything else runs the general body, and
-// both give the same bits.
+// The production form of the step (production_step below): the settings of
+// the global forward run, and of the ensemble's and the inversion's steps.  It
+// is taken when every one of these holds, which the host sees from the
+// arguments; anything else runs the general body, and both give the same
+// bits.  Outside it: no dry deposition (the driver passes a zero velocity as
+// none, so its default forcing is one of these), a uniform or per-slot wet
+// coefficient, two to four species, and the driver's separated passes where
+// a call holds more than one stage.
 //   * all of advection, turbulence with four sub-steps and uniform dry
 //     deposition, with per-cell wet deposition or none, no probability
 //     outputs and one species;

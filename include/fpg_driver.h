@@ -283,11 +283,11 @@ fpg_status fpg_backward_set_validation_mode(fpg_backward* d, int32_t on);
  * come out bit for bit as in a plain run of it alone.  All scenarios share
  * one met frame ring and one global clock; their particles sit in one
  * structure-of-arrays population, each scenario in a 256-slot-aligned
- * segment.  One step is a CUDA graph of device-side kernels (clock and
- * release bookkeeping, bracket repack when it changes, per-cell PBL and wet
- * forcing, release of new particles, one persistent launch over all
- * scenarios' tiles from a work queue, per-scenario grids at output steps,
- * counter advance), so the host only launches the graph.
+ * segment.  One step is a CUDA graph of two device-side kernels, three at
+ * output steps (clock, counter and release bookkeeping, bracket repack when it
+ * changes, per-cell PBL and wet forcing and release of new particles in one;
+ * one launch over all scenarios' work items; per-scenario grids), so the host
+ * only launches the graph.
  * ---------------------------------------------------------------------- */
 typedef struct fpg_batch_scenario {
     fpg_release release;
@@ -329,8 +329,8 @@ fpg_status fpg_batch_destroy(fpg_batch* b);
 fpg_status fpg_batch_upload_frame(fpg_batch* b, uint32_t k, const float* u, const float* v, const float* w,
                                   const fpg_surface_cell* surface, const float* precipitation_mm_h);
 /* Runs n_steps steps (fewer if the end time comes first): each step is one
- * replay of the captured graph when use_graph is non-zero (the graph is
- * captured on the first call), else the same kernels launched one by one.
+ * replay of a captured graph when use_graph is non-zero (the first call that
+ * needs a graph captures it, before its first step), else the same kernels launched one by one.
  * Returns FPG_ERR_SIMULATION_COMPLETE when no step is left. */
 fpg_status fpg_batch_run(fpg_batch* b, uint32_t n_steps, int32_t use_graph);
 /* The same steps with one launch per scenario per step, the one fpg_step
